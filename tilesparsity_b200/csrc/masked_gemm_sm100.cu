@@ -36,6 +36,8 @@
 // Warp roles (448 threads): warp 0 = weight TMA, warp 1 = TMEM allocation + MMA issue,
 // warps 2-5 = activation gather, warps 6-13 = epilogue.  (Eight gather warps were measured: 18 warps
 // leave 96 registers per thread, the kernel spills, and every workload got slower.)
+#include <cstddef>
+
 #include "ts_common.cuh"
 #include "ts_kernels.h"
 
@@ -46,55 +48,44 @@ namespace {
 constexpr int kNT = 128;                 // columns per tile (MMA M, TMEM lanes)
 constexpr int kKB = 64;                  // kept rows per pipeline stage
 constexpr int kWBytes = kNT * kKB * 2;   // 16 KiB of packed weights per stage
-constexpr int kEpiThreads = 256;
+constexpr int kEpiWarps = 8;
 constexpr uint32_t kASbo = 1024;         // bytes between 8-row K groups of the gathered operand
 constexpr uint32_t kALbo = kKB * 128;    // bytes between its 64-column batch groups
 constexpr uint32_t kWSbo = 1024;         // bytes between 8-row groups of the weight operand
 constexpr int kMaxStages = 6;
-#ifndef TS_GATHER_WARPS
-#define TS_GATHER_WARPS 4
-#endif
-constexpr int kGW = TS_GATHER_WARPS;     // gather warps
+// Gather warps.  Four keep the L2-to-SM path full: 470 cycles per 32 KiB block on B200 with every SM
+// copying, the same with 8 and 16 warps; all four fill every block together, 16 rows each, which is
+// one K step of the MMA.
+constexpr int kGW = 4;
+constexpr int kRowsPerWarp = kKB / kGW;
 constexpr int kEpiWarp0 = 2 + kGW;       // first epilogue warp
-constexpr int kThreads = 32 * kEpiWarp0 + kEpiThreads;
-// Gather warps that share one K block.  Measured on B200 with 1, 2 and 4: 4 is best or within 3 % of
-// the best on every workload tried (1 loses up to 30 % where the activations stream from DRAM,
-// because the blocks of different warps then land out of order and the MMA warp consumes them in
-// order).  With fewer than 4 the per-warp record slices grow and the ring below must shrink to fit.
-#ifndef TS_WARPS_PER_BLOCK
-#define TS_WARPS_PER_BLOCK 4
-#endif
-constexpr int kWarpsPerBlock = TS_WARPS_PER_BLOCK;
-constexpr int kWarpGroups = kGW / kWarpsPerBlock;    // group p of warps takes blocks p, p+kWarpGroups, ...
-constexpr int kRowsPerWarp = kKB / kWarpsPerBlock;
+constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
 constexpr int kMetaInts = kBlockMetaInts;  // one block record: {m0, meta, 0, 0} + 64 row numbers
-constexpr int kAhead = 4;                // a warp requests its part of a record this many of its blocks ahead
-constexpr int kMetaSlots = 6;            // ring slots per warp (> kAhead)
+constexpr int kAhead = 4;                // records are requested this many blocks ahead of the weights
+constexpr int kMaxRecs = kMaxStages + kAhead;
+constexpr int kEpiWarpBytes = 4096;      // staging of one epilogue warp: two 32-row x 32-column chunks of 2 KiB
 
 struct Barriers {
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
+  uint64_t rec_full[kMaxRecs];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  // Per gather warp: ring of the parts of the coming blocks' records that the warp needs: the
-  // descriptor words and the row numbers of its slice.
-  alignas(16) int meta_ring[kGW][kMetaSlots][4 + kRowsPerWarp];
+  alignas(16) int rec[kMaxRecs][kMetaInts];   // ring of block records, slot = block % Cfg::kRecs
 };
 
 // Compile-time shape of one kernel variant: MT batch rows per work unit.
 template <int MT>
 struct Cfg {
-  // As many stages as fit beside the staging groups in 227 KiB.  A warp group must never run two
-  // phases of one stage ahead of the MMA warp (the parity wait could not tell them apart), which
-  // holds as long as there are at least as many stages as warp groups.
+  // as many stages as fit beside the staging buffers in 227 KiB
   static constexpr int kStages = MT == 256 ? 4 : 6;
-  static_assert(kStages <= kMaxStages && kStages >= kWarpGroups, "stage count");
+  static constexpr int kRecs = kStages + kAhead;
+  static_assert(kStages <= kMaxStages && kRecs <= kMaxRecs, "stage count");
   static constexpr int kABytes = kKB * MT * 2;
   static constexpr int kStageBytes = kWBytes + kABytes;
-  static constexpr int kEpiGroupBytes = kNT * 128;   // staging: one 128-row x 64-column swizzled group
-  static constexpr int kEpiBytes = 2 * kEpiGroupBytes;  // one group per half of the epilogue warps
+  static constexpr int kEpiBytes = kEpiWarps * kEpiWarpBytes;
   static constexpr int kTmemCols = 2 * MT;          // two accumulators of MT fp32 columns
   // stages + staging + barriers/records + what the 1024-byte alignment of the first stage may skip
   static constexpr int kUsedBytes = kStages * kStageBytes + kEpiBytes + static_cast<int>(sizeof(Barriers));
@@ -103,6 +94,7 @@ struct Cfg {
   static_assert(kUsedBytes <= kSmemBytes, "stages, staging and barriers exceed the shared memory of one CTA");
   static constexpr int kLanesPerRow = MT / 8;       // 16-byte chunks in one gathered row
   static constexpr int kRowsPerInstr = 32 / kLanesPerRow;
+  static constexpr int kChunks = MT / 64;           // 32-column chunks per epilogue warp
 };
 
 __device__ __forceinline__ WorkItem load_item(const WorkItem* p) {
@@ -117,10 +109,6 @@ __device__ __forceinline__ WorkItem load_item(const WorkItem* p) {
   return u.w;
 }
 
-__device__ __forceinline__ void named_barrier_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // Work item of CTA `cta` in round r, or an empty item past the end of the schedule.
 __device__ __forceinline__ WorkItem fetch_item(const WorkItem* sched, int rounds, int grid, int cta,
                                                int r) {
@@ -133,19 +121,48 @@ __device__ __forceinline__ WorkItem fetch_item(const WorkItem* sched, int rounds
   return w;
 }
 
+// What the epilogue reads of a work item that the warp holds one word per lane.
+constexpr int kItemWords = sizeof(WorkItem) / 4;
+constexpr int kItemWordTile = 11;
+static_assert(offsetof(WorkItem, n_list) == 8 && offsetof(WorkItem, k_count) == 16 && offsetof(WorkItem, n_count) == 20 &&
+                  offsetof(WorkItem, c_row0) == 28 && offsetof(WorkItem, flags) == 32 && offsetof(WorkItem, m_begin) == 36 &&
+                  offsetof(WorkItem, m_len) == 40 && offsetof(WorkItem, tile) == 44,
+              "word numbers below");
+struct EpiItem {
+  const int* n_list;
+  int n_count, c_row0, flags, m_begin, m_len;
+  bool has_rows;
+};
+__device__ __forceinline__ EpiItem epi_item(int word) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  EpiItem w;
+  const uint32_t lo = __shfl_sync(kAll, word, 2), hi = __shfl_sync(kAll, word, 3);
+  w.n_list = reinterpret_cast<const int*>((static_cast<uint64_t>(hi) << 32) | lo);
+  w.has_rows = __shfl_sync(kAll, word, 4) > 0;
+  w.n_count = __shfl_sync(kAll, word, 5);
+  w.c_row0 = __shfl_sync(kAll, word, 7);
+  w.flags = __shfl_sync(kAll, word, 8);
+  w.m_begin = __shfl_sync(kAll, word, 9);
+  w.m_len = __shfl_sync(kAll, word, 10);
+  return w;
+}
+
 __device__ __forceinline__ int k_blocks(const WorkItem& w) { return (w.k_count + kKB - 1) / kKB; }
 
 // Ct row (global column of W) of tile column j of a work item.
-__device__ __forceinline__ long long c_row_of(const WorkItem& w, int j) {
+__device__ __forceinline__ long long c_row_of(const EpiItem& w, int j) {
   return w.c_row0 + (w.n_list ? __ldg(w.n_list + j) + ((w.flags & kItemRelative) ? j : 0) : j);
 }
 
 __device__ __forceinline__ float apply_act(float x, int act) {
   if (act == kActRelu) return fmaxf(x, 0.0f);
   if (act == kActGelu) {
-    // x * 0.5 * (1 + tanh(sqrt(2/pi) * (x + 0.044715 x^3)))   (Pruning/BERT/utils/modeling.py:264-277)
-    const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-    return 0.5f * x * (1.0f + tanhf(u));
+    // x * 0.5 * (1 + tanh(u)), u = sqrt(2/pi) * (x + 0.044715 x^3)  (Pruning/BERT/utils/modeling.py:264-277),
+    // written as x / (1 + exp(-2u)), which is the same function without the cancellation of 1 + tanh for
+    // negative u; two special-function instructions instead of tanhf's branches (the epilogue of a
+    // 256 x 128 unit spent 17000 cycles on tanhf).
+    const float u2 = 1.5957691216057308f * (x + 0.044715f * x * x * x);
+    return __fdividef(x, 1.0f + __expf(-u2));
   }
   return x;
 }
@@ -168,6 +185,7 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                    uint16_t* __restrict__ Ct, long long ldc, int M, const __grid_constant__ EpilogueArgs ep,
                    int* __restrict__ status) {
   const float alpha = ep.alpha, beta = ep.beta;
+  const int act = ep.act;
   constexpr bool SPLIT = MODE == kModeSplit, PEERS = MODE == kModePeers, LEAN = MODE == kModeLean;
   using C = Cfg<MT>;
   constexpr int kStages = C::kStages;
@@ -189,37 +207,31 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   const int grid = gridDim.x;
   const int cta = blockIdx.x;
 
-  // First work item, and for the gather warps the record of their first block: requested before
-  // the set-up below so their latency overlaps it.  The schedule is static data.
+  // First work item: requested before the set-up below so its latency overlaps it.  The schedule is
+  // static data.
   WorkItem w = fetch_item(sched, rounds, grid, cta, 0);
-  const int gw = warp - 2;                                  // gather warp number (warps 2..5)
   const int* recs = block_meta + static_cast<size_t>(cta) * blk_stride * kMetaInts;
-  // lanes 0..: one 16-byte piece each: the descriptor, then the warp's slice of the row numbers
-  const int meta_piece = lane == 0 ? 0 : 4 + (gw % kWarpsPerBlock) * kRowsPerWarp + (lane - 1) * 4;
-  constexpr int kMetaLanes = 1 + kRowsPerWarp / 4;
-  if (warp >= 2 && warp < kEpiWarp0) {
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i) {
-      if (lane < kMetaLanes) {
-        cp_async_16_ca(smem_u32(&bars->meta_ring[gw][i][lane * 4]),
-                       recs + static_cast<size_t>(gw / kWarpsPerBlock + i * kWarpGroups) * kMetaInts + meta_piece);
-      }
-      cp_async_commit();
-    }
-  }
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < kStages; ++s) {
-      // weight TMA thread + the cp.async lanes of the warps that fill the stage
-      mbar_init(smem_u32(&bars->full[s]), 1 + 32 * kWarpsPerBlock);
+      // weight TMA thread + the cp.async lanes of the gather warps
+      mbar_init(smem_u32(&bars->full[s]), 1 + 32 * kGW);
       mbar_init(smem_u32(&bars->empty[s]), 1);       // one tcgen05.commit
     }
+    for (int s = 0; s < C::kRecs; ++s) mbar_init(smem_u32(&bars->rec_full[s]), 1);
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&bars->acc_full[a]), 1);
-      mbar_init(smem_u32(&bars->acc_empty[a]), kEpiThreads);
+      mbar_init(smem_u32(&bars->acc_empty[a]), kEpiWarps);
     }
     bars->abort_flag = 0;
     mbar_fence_init();
+    fence_proxy_async_smem();
+    // The records of the first blocks: their latency is the head of the chain record -> rows -> MMA.
+    for (int i = 0; i < kAhead; ++i) {
+      const uint32_t bar = smem_u32(&bars->rec_full[i]);
+      mbar_arrive_expect_tx(bar, kMetaInts * 4);
+      bulk_load(smem_u32(bars->rec[i]), recs + static_cast<size_t>(i) * kMetaInts, kMetaInts * 4, bar);
+    }
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&bars->tmem_base), C::kTmemCols);
@@ -234,149 +246,146 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   grid_launch_dependents();
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ weight TMA producer
-    if (lane == 0) tma_prefetch_desc(&tmap_w);
-    uint32_t it = 0;
-    bool ok = true;
-    for (int r = 0; ok && w.tile >= 0; ++r) {
-      const WorkItem wn = fetch_item(sched, rounds, grid, cta, r + 1);
-      const int nkb = (w.k_count + kKB - 1) / kKB;
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
-        const uint32_t s = it % kStages;
-        const uint32_t ph = (it / kStages) & 1u;
-        ok = mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1u, abort_flag);
-        if (!ok) break;
-        if (lane == 0) {
+    // ------------------------------------------------------------------ weights and block records
+    // Block `it`: its weights once its stage is free, and the record of block it + kAhead, whose ring slot
+    // was last used by block it + kAhead - kRecs = it - kStages, consumed when that stage became free.
+    if (elect_one()) {
+      tma_prefetch_desc(&tmap_w);
+      uint32_t it = 0;
+      bool ok = true;
+      for (int r = 0; ok && w.tile >= 0; ++r) {
+        const WorkItem wn = fetch_item(sched, rounds, grid, cta, r + 1);
+        const int nkb = k_blocks(w);
+        // (a split-K part starts at K block flags >> 8 of its tile's packed weights)
+        const int kb_first = SPLIT ? static_cast<int>(static_cast<uint32_t>(w.flags) >> kItemKb0Shift) : 0;
+        for (int kb = 0; kb < nkb; ++kb, ++it) {
+          const uint32_t s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1u;
+          ok = mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1u, abort_flag);
+          if (!ok) break;
           const uint32_t bar = smem_u32(&bars->full[s]);
           mbar_arrive_expect_tx(bar, kWBytes);
-          // (a split-K part starts at K block flags >> 8 of its tile's packed weights)
-          const int kb_first = SPLIT ? static_cast<int>(static_cast<uint32_t>(w.flags) >> kItemKb0Shift) : 0;
           tma_load_2d(smem_u32(smem + s * C::kStageBytes), &tmap_w, (kb + kb_first) * kKB, w.w_row0, bar);
+          const uint32_t slot = (it + kAhead) % C::kRecs;
+          const uint32_t rbar = smem_u32(&bars->rec_full[slot]);
+          mbar_arrive_expect_tx(rbar, kMetaInts * 4);
+          bulk_load(smem_u32(bars->rec[slot]), recs + static_cast<size_t>(it + kAhead) * kMetaInts, kMetaInts * 4, rbar);
         }
-        __syncwarp();
+        w = wn;
       }
-      w = wn;
+      // the records past the end marker (never read) must have landed before the CTA retires
+      for (uint32_t i = it; i < it + kAhead; ++i) {
+        mbar_wait(smem_u32(&bars->rec_full[i % C::kRecs]), (i / C::kRecs) & 1u, abort_flag);
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    // the MMA's N dimension is the unit's batch-row count (a multiple of 64, at most MT)
+    // One elected thread runs the whole loop (see elect_one).  The MMA's N dimension is the unit's
+    // batch-row count (at most MT).
     constexpr uint32_t idesc0 = umma_idesc_f16(DT == kBF16 ? 1 : 0, /*a_mn=*/0, /*b_mn=*/1, kNT, 0);
-    uint32_t it = 0, acc_it = 0;
-    bool ok = true;
-    for (int r = 0; ok && w.tile >= 0; ++r) {
-      const WorkItem wn = fetch_item(sched, rounds, grid, cta, r + 1);
-      const int nkb = (w.k_count + kKB - 1) / kKB;
-      const uint32_t a = acc_it & 1u;
-      const uint32_t aph = (acc_it >> 1) & 1u;
-      ok = mbar_wait(smem_u32(&bars->acc_empty[a]), aph ^ 1u, abort_flag);
-      if (!ok) break;
-      tc_fence_after_sync();
-      const uint32_t tmem_d = tmem_base + a * MT;
-      const uint32_t idesc = idesc0 | (static_cast<uint32_t>(w.m_len >> 3) << 17);
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
-        const uint32_t s = it % kStages;
-        const uint32_t ph = (it / kStages) & 1u;
-        ok = mbar_wait(smem_u32(&bars->full[s]), ph, abort_flag);
+    if (elect_one()) {
+      uint32_t it = 0, acc_it = 0;
+      bool ok = true;
+      for (int r = 0; ok && w.tile >= 0; ++r) {
+        const WorkItem wn = fetch_item(sched, rounds, grid, cta, r + 1);
+        const int nkb = (w.k_count + kKB - 1) / kKB;
+        const uint32_t a = acc_it & 1u;
+        const uint32_t aph = (acc_it >> 1) & 1u;
+        ok = mbar_wait(smem_u32(&bars->acc_empty[a]), aph ^ 1u, abort_flag);
         if (!ok) break;
-        // The gathered rows were written through the generic proxy; the MMA reads them through
-        // the async proxy.
-        fence_proxy_async_smem();
         tc_fence_after_sync();
-        if (lane == 0) {
+        const uint32_t tmem_d = tmem_base + a * MT;
+        // batch rows past the end of the matrix are neither gathered nor multiplied (N in steps of 16)
+        const int n_cols = min(w.m_len, (M - w.m_begin + 15) & ~15);
+        const uint32_t idesc = idesc0 | (static_cast<uint32_t>(n_cols >> 3) << 17);
+        for (int kb = 0; kb < nkb; ++kb, ++it) {
+          const uint32_t s = it % kStages;
+          const uint32_t ph = (it / kStages) & 1u;
+          ok = mbar_wait(smem_u32(&bars->full[s]), ph, abort_flag);
+          if (!ok) break;
+          // The gathered rows were written through the generic proxy; the MMA reads them through
+          // the async proxy.
+          fence_proxy_async_smem();
+          tc_fence_after_sync();
           const int krem = w.k_count - kb * kKB;
           const int nk16 = krem >= kKB ? kKB / 16 : (krem + 15) / 16;
           const uint32_t w_addr = smem_u32(smem + s * C::kStageBytes);
           const uint32_t a_addr = w_addr + kWBytes;
-          for (int k = 0; k < nk16; ++k) {
-            // weights: K-major, 16 K elements = 32 bytes inside the 128-byte swizzled row
-            const uint64_t dw = umma_smem_desc_sw128(w_addr + k * 32, 16, kWSbo);
-            // activations: MN-major, 16 K rows = two 8-row groups
-            const uint64_t da = umma_smem_desc_sw128(a_addr + k * 2 * kASbo, kALbo, kASbo);
-            umma_f16(tmem_d, dw, da, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          // weights: K-major, 16 K elements = 32 bytes inside the 128-byte swizzled row; activations:
+          // MN-major, 16 K rows = two 8-row groups
+          const uint64_t dw = umma_smem_desc_sw128(w_addr, 16, kWSbo);
+          const uint64_t da = umma_smem_desc_sw128(a_addr, kALbo, kASbo);
+#pragma unroll
+          for (int k = 0; k < kKB / 16; ++k) {
+            if (k < nk16) {
+              umma_f16(tmem_d, dw + static_cast<uint64_t>(k * 32 >> 4), da + static_cast<uint64_t>(k * 2 * kASbo >> 4), idesc,
+                       (kb > 0 || k > 0) ? 1u : 0u);
+            }
           }
           umma_commit(smem_u32(&bars->empty[s]));
         }
-        __syncwarp();
-      }
-      if (!ok) break;
-      if (lane == 0) {
+        if (!ok) break;
         if (nkb > 0) {
           umma_commit(smem_u32(&bars->acc_full[a]));
         } else {
           mbar_arrive(smem_u32(&bars->acc_full[a]));  // tile with no kept rows: nothing to wait for
         }
+        ++acc_it;
+        w = wn;
       }
-      __syncwarp();
-      ++acc_it;
-      w = wn;
     }
   } else if (warp < kEpiWarp0) {
     // ------------------------------------------------------------------ activation gather
-    // kWarpsPerBlock warps share one block (a slice of its rows each); group p of warps takes the
-    // blocks p, p+kWarpGroups, ... of the CTA's stream, block j lives in stage j % kStages.  Per block: wait
-    // for its record (requested kAhead blocks earlier), wait for the stage, issue the
-    // warp's rows in one burst (row numbers read from the record into registers first: a
-    // shared-memory read between two copies stalls the warp until the load/store unit has taken the
-    // copies before it), hand the copies to the stage's barrier.  One cp.async group is committed
-    // per block, made of the block's row copies and the request for the record kAhead blocks on;
-    // "all but the latest kAhead - 1 groups have completed" therefore says that this block's
-    // record has landed while the rows of the kAhead - 1 blocks before it may still be in flight.
+    // The four warps fill every block together, 16 rows each (one K step of the MMA).  Per block: wait for
+    // the stage, issue the warp's rows in one burst of 16-byte copies, hand them to the stage's barrier.
+    // The row numbers of the next block go from the record ring to registers before that wait, so neither
+    // the record nor a shared-memory read sits between a free stage and its copies (a read between two
+    // copies would also stall the warp until the load/store unit has taken the copies before it).
     constexpr int kLpr = C::kLanesPerRow, kRpi = C::kRowsPerInstr;
     const int chunk = lane % kLpr, sub = lane / kLpr;
     const int g = chunk >> 3, c = chunk & 7;
-    const int grp = gw / kWarpsPerBlock;                    // group of warps this warp belongs to
-    const int row_base = (gw % kWarpsPerBlock) * kRowsPerWarp;   // first row of the warp's slice
+    const int row_base = (warp - 2) * kRowsPerWarp;         // first row of the warp's slice
+    int rr[kRowsPerWarp], rn[kRowsPerWarp];
+    int m0 = 0, m0_next;
+    uint32_t meta = kBlockEnd, meta_next;
+    auto read_record = [&](uint32_t j, int& m0_out, uint32_t& meta_out, int (&rows)[kRowsPerWarp]) -> bool {
+      const uint32_t slot = j % C::kRecs;
+      if (!mbar_wait(smem_u32(&bars->rec_full[slot]), (j / C::kRecs) & 1u, abort_flag)) return false;
+      const int* rec = bars->rec[slot];
+      const int2 head = *reinterpret_cast<const int2*>(rec);
+      m0_out = head.x;
+      meta_out = static_cast<uint32_t>(head.y);
+#pragma unroll
+      for (int q4 = 0; q4 < kRowsPerWarp / 4; ++q4) {
+        const int4 v = *reinterpret_cast<const int4*>(rec + 4 + row_base + q4 * 4);
+        rows[q4 * 4] = v.x;
+        rows[q4 * 4 + 1] = v.y;
+        rows[q4 * 4 + 2] = v.z;
+        rows[q4 * 4 + 3] = v.w;
+      }
+      return true;
+    };
+    bool ok = read_record(0, m0, meta, rr);
     // The schedule is static; the activations may be the previous kernel's output: wait for it
     // before the first row is copied.
     grid_dependency_wait();
 
-    for (uint32_t it = 0;; ++it) {
-      const int j = grp + static_cast<int>(it) * kWarpGroups;
-      cp_async_wait_group<kAhead - 1>();
-      __syncwarp();
-      const int* rec = bars->meta_ring[gw][it % kMetaSlots];
-      const int m0 = rec[0];
-      const uint32_t meta = static_cast<uint32_t>(rec[1]);
-      if (meta == kBlockEnd) break;
-      const int nv = static_cast<int>(meta & 0x7fu);
+    for (uint32_t j = 0; ok && meta != kBlockEnd; ++j) {
+      if (!read_record(j + 1, m0_next, meta_next, rn)) break;
+      const int nv = static_cast<int>(meta & 0x7fu) - row_base;                 // valid rows of the slice
       const int m_len = (static_cast<int>((meta >> 8) & 3u) + 1) * 64;          // batch rows of the unit
       const int m = m0 + chunk * 8;
-      const bool m_ok = m < M;
-      const uint16_t* src_col = At + (m_ok ? m : 0);
-      const bool lane_live = chunk * 8 < m_len;             // columns past the unit are never read
-      const bool full_block = nv == kKB && m0 + m_len <= M;
-      const uint32_t s = static_cast<uint32_t>(j) % kStages;
-      const uint32_t ph = (static_cast<uint32_t>(j) / kStages) & 1u;
+      // lanes past the unit or past the batch: their columns are never multiplied into a stored result
+      const bool live = chunk * 8 < m_len && m < M;
+      const uint16_t* src_col = At + m;
+      const uint32_t s = j % kStages;
+      const uint32_t ph = (j / kStages) & 1u;
       const uint32_t dst0 = smem_u32(smem + s * C::kStageBytes + kWBytes) + g * kALbo;
       const uint32_t bar = smem_u32(&bars->full[s]);
       if (!mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1u, abort_flag)) break;
-      int rr[kRowsPerWarp];
-#pragma unroll
-      for (int q4 = 0; q4 < kRowsPerWarp / 4; ++q4) {
-        const int4 v = reinterpret_cast<const int4*>(rec + 4)[q4];
-        rr[q4 * 4] = v.x;
-        rr[q4 * 4 + 1] = v.y;
-        rr[q4 * 4 + 2] = v.z;
-        rr[q4 * 4 + 3] = v.w;
-      }
       // Two separate bursts: mixing the zero-fill form into the loop of plain copies makes every
-      // copy as slow as the zero-fill form.
-      if (full_block) {
-        if (lane_live) {
-#pragma unroll
-          for (int e = 0; e < kRowsPerWarp / kRpi; ++e) {
-            const int row = row_base + e * kRpi + sub;
-            int kr;
-            if constexpr (kRpi == 1) {
-              kr = rr[e];
-            } else {
-              kr = sub ? rr[e * 2 + 1] : rr[e * 2];
-            }
-            cp_async_16_full(dst0 + (row >> 3) * kASbo + (row & 7) * 128 + ((c ^ (row & 7)) << 4),
-                             src_col + (static_cast<long long>(kr) << 3));
-          }
-        }
-      } else if (lane_live) {
+      // copy as slow as the zero-fill form.  A slice without valid rows is not multiplied at all.
+      if (live && nv >= kRowsPerWarp) {
 #pragma unroll
         for (int e = 0; e < kRowsPerWarp / kRpi; ++e) {
           const int row = row_base + e * kRpi + sub;
@@ -386,37 +395,60 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
           } else {
             kr = sub ? rr[e * 2 + 1] : rr[e * 2];
           }
-          const bool valid = (row < nv) && m_ok;
+          cp_async_16_full(dst0 + (row >> 3) * kASbo + (row & 7) * 128 + ((c ^ (row & 7)) << 4),
+                           src_col + (static_cast<long long>(kr) << 3));
+        }
+      } else if (live && nv > 0) {
+#pragma unroll
+        for (int e = 0; e < kRowsPerWarp / kRpi; ++e) {
+          const int row = row_base + e * kRpi + sub;
+          int kr;
+          if constexpr (kRpi == 1) {
+            kr = rr[e];
+          } else {
+            kr = sub ? rr[e * 2 + 1] : rr[e * 2];
+          }
+          const bool valid = row - row_base < nv;
           cp_async_16(dst0 + (row >> 3) * kASbo + (row & 7) * 128 + ((c ^ (row & 7)) << 4),
                       valid ? src_col + (static_cast<long long>(kr) << 3) : At, valid ? 16u : 0u);
         }
       }
       cp_async_arrive_noinc(bar);
-      // request the warp's part of the record kAhead of its blocks ahead; one group per block
-      if (lane < kMetaLanes) {
-        cp_async_16_ca(smem_u32(&bars->meta_ring[gw][(it + kAhead) % kMetaSlots][lane * 4]),
-                       recs + static_cast<size_t>(j + kAhead * kWarpGroups) * kMetaInts + meta_piece);
-      }
-      cp_async_commit();
+      m0 = m0_next;
+      meta = meta_next;
+#pragma unroll
+      for (int e = 0; e < kRowsPerWarp; ++e) rr[e] = rn[e];
     }
     cp_async_wait_all();  // nothing of this thread is in flight when the CTA retires
   } else if (warp >= kEpiWarp0) {
     // ------------------------------------------------------------------ epilogue
-    constexpr int kGroups = MT / 128;            // 64-column groups per epilogue thread
+    // Every warp works alone: it owns 32 tile columns (its TMEM lane quarter) and every other 32-column
+    // chunk of the unit's batch, stages a chunk (32 rows x 64 bytes, 64-byte swizzle) in one of two
+    // buffers of its own and sends it off, as one TMA tile store where its 32 rows are consecutive rows of
+    // Ct, else with 16-byte stores through the kept-column list.  No barrier between warps: with staging
+    // groups shared by four warps a 256 x 128 unit took 3500-5000 cycles here, most of them waiting.
     const int ew = warp - kEpiWarp0;             // 0..7
-    const int half = ew >> 2;                    // takes the 64-column groups half, half+2, ...
+    const int half = ew >> 2;                    // takes the 32-column chunks half, half+2, ...
     const int q = warp & 3;                      // TMEM lane quarter this warp may read
     const int j = q * 32 + lane;                 // tile column owned by this thread
-    const bool leader = ((ew & 3) == 0 && lane == 0);   // one per half
-    const int half_bar = 1 + half;               // named barrier of this half (128 threads)
     const int peer_rot = (PEERS && ep.n_peers > 0) ? cta % ep.n_peers : 0;   // the peer this CTA writes first
-    uint32_t acc_it = 0;
-    bool ok = true;
+    uint8_t* const own_stage = epi + ew * kEpiWarpBytes;
+    // this lane's row of a staging chunk, and the 16-byte pieces of it in swizzled order
+    const int row_off = lane * 64, row_swz = (lane >> 1) & 3;
+    uint32_t n_staged = 0;
+    // Work items are held one word per lane, the next one in flight while this one is worked on: whole
+    // copies in every lane cost the registers that two TMEM chunks need.
+    const int* const items = reinterpret_cast<const int*>(sched + cta) + lane;
+    auto item_word = [&](int r) -> int {
+      return r < rounds && lane < kItemWords ? __ldg(items + static_cast<size_t>(r) * grid * kItemWords) : -1;
+    };
+    int word = item_word(0);
     grid_dependency_wait();   // Ct may still be read or written by the previous kernel
-    for (int r = 0; ok && w.tile >= 0; ++r) {
-      const WorkItem wn = fetch_item(sched, rounds, grid, cta, r + 1);
-      const uint32_t a = acc_it & 1u;
-      const uint32_t aph = (acc_it >> 1) & 1u;
+    for (uint32_t r = 0; __shfl_sync(0xffffffffu, word, kItemWordTile) >= 0; ++r) {
+      const int word_next = item_word(r + 1);
+      const EpiItem w = epi_item(word);
+      const uint32_t a = r & 1u;
+      const uint32_t aph = (r >> 1) & 1u;
       const int m0 = w.m_begin;
       const int m_cnt = min(w.m_len, M - m0);
       const bool active = j < w.n_count;
@@ -425,190 +457,160 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                       (!PEERS || ep.multicast == nullptr));
       const bool tma_peers = PEERS && tma_store && ep.peer_maps != nullptr;   // the peers' copies leave by TMA too
       // The CTA's last unit: every K block has been consumed, so the pipeline stages are free and
-      // each 64-column group gets a staging group of its own there; no group waits for the store
-      // of the one before it.
-      const bool last_unit = wn.tile < 0;
-      const bool plain = LEAN || (beta == 0.0f && ep.bias == nullptr && ep.act == kActNone);
+      // each chunk gets a staging buffer of its own there; none waits for a store before it.
+      const bool last_unit = __shfl_sync(0xffffffffu, word_next, kItemWordTile) < 0;
       const long long c_row = active ? c_row_of(w, j) : 0;
       const int c_row_or_none = active ? static_cast<int>(c_row) : -1;
       const float bias_j = (ep.bias != nullptr && active) ? __ldg(ep.bias + c_row) : 0.0f;
-      uint16_t* gdst = Ct + c_row * ldc + m0;
       const int tile_row0 = w.c_row0 + ((tma_store && w.n_list) ? __ldg(w.n_list) : 0);
-      ok = mbar_wait(smem_u32(&bars->acc_full[a]), aph, abort_flag);
-      if (!ok) break;
+      if (!mbar_wait(smem_u32(&bars->acc_full[a]), aph, abort_flag)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + a * MT + (static_cast<uint32_t>(q * 32) << 16);
-      const bool has_acc = w.k_count > 0;
-      // TMEM is read one 64-column group (two 32-column reads, one wait) at a time: a read's latency
-      // is far longer than the conversion of one chunk, so the two must overlap each other.
-      constexpr int kBatch = 2;
-      // Not unrolled: the epilogue's hot code stays small enough for the instruction cache it
-      // shares with the other roles (-3 % on the BERT layer).
+      const bool has_acc = w.has_rows;
+      // Not unrolled: the hot code stays small enough for the instruction cache it shares with the other
+      // roles, and one chunk's registers leave room for everything else (with two the kernel spilled, and
+      // a spilled register waits behind the gather's copies in the load/store queue).
 #pragma unroll 1
-      for (int gi = 0; gi < kGroups; ++gi) {
-        const int grp_col = (gi * 2 + half) * 64;        // first batch column of this thread's group
-        const bool grp_live = grp_col < m_cnt;           // uniform over the half
-        uint32_t v[kBatch][32];
-        if (grp_live) {
-          if (has_acc) {
+      for (int ci = 0; ci < C::kChunks; ++ci) {
+        const int col0 = (ci * 2 + half) * 32;              // first batch column of the chunk
+        const bool live = col0 < m_cnt;                     // uniform over the warp
+        uint32_t cur[32];
+        if (has_acc && live) {
+          tmem_ld_32x32(taddr + col0, cur);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-            for (int b = 0; b < kBatch; ++b) tmem_ld_32x32(taddr + grp_col + b * 32, v[b]);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int b = 0; b < kBatch; ++b)
-#pragma unroll
-              for (int e = 0; e < 32; ++e) v[b][e] = 0u;
-          }
+          for (int e = 0; e < 32; ++e) cur[e] = 0u;
         }
-        if (gi == kGroups - 1) {
-          // every TMEM read of this accumulator has completed: hand it back to the MMA warp
+        if (ci + 1 == C::kChunks) {
+          // every TMEM read of this accumulator by this warp has completed: hand it back to the MMA warp
           tc_fence_before_sync();
-          mbar_arrive(smem_u32(&bars->acc_empty[a]));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[a]));
         }
-        if (!grp_live) continue;
-        if constexpr (SPLIT) if (w.flags & kItemScratch) {
-          // split-K part: alpha * acc leaves as fp32 for the part's 128 scratch rows.  32 fp32 columns
-          // fill one 128-row x 128-byte staging group, which goes out as one TMA tile store; bias, beta
-          // and the activation are applied by the kernel that adds the parts up.  (Tile columns past
-          // n_count carry zero weights, so their rows receive zeros.)
-          uint8_t* stage = epi + half * C::kEpiGroupBytes;
-#pragma unroll
-          for (int b = 0; b < kBatch; ++b) {
-            if (grp_col + b * 32 >= m_cnt) break;              // uniform over the half
-            if (leader) bulk_wait_read_all();
-            named_barrier_sync(half_bar, 128);
-            uint8_t* row_ptr = stage + j * 128;
+        if (!live) continue;
+        {
+          if constexpr (SPLIT) if (w.flags & kItemScratch) {
+            // split-K part: alpha * acc leaves as fp32 for the part's scratch rows (32 rows x 128 bytes,
+            // 128-byte swizzle, both staging buffers); bias, beta and the activation are applied by the
+            // kernel that adds the parts up.  (Tile columns past n_count carry zero weights, so their rows
+            // receive zeros.)
+            if (lane == 0) bulk_wait_read_all();
+            __syncwarp();
+            uint8_t* row_ptr = own_stage + lane * 128;
 #pragma unroll
             for (int cc = 0; cc < 8; ++cc) {
-              *reinterpret_cast<float4*>(row_ptr + ((cc ^ (j & 7)) << 4)) =
-                  make_float4(alpha * __uint_as_float(v[b][cc * 4]), alpha * __uint_as_float(v[b][cc * 4 + 1]),
-                              alpha * __uint_as_float(v[b][cc * 4 + 2]), alpha * __uint_as_float(v[b][cc * 4 + 3]));
+              *reinterpret_cast<float4*>(row_ptr + ((cc ^ (lane & 7)) << 4)) =
+                  make_float4(alpha * __uint_as_float(cur[cc * 4]), alpha * __uint_as_float(cur[cc * 4 + 1]),
+                              alpha * __uint_as_float(cur[cc * 4 + 2]), alpha * __uint_as_float(cur[cc * 4 + 3]));
             }
             fence_proxy_async_smem();
-            named_barrier_sync(half_bar, 128);
-            if (leader) {
-              tma_store_2d(ep.scratch_map, smem_u32(stage), m0 + grp_col + b * 32, w.c_row0);
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(ep.scratch_map, smem_u32(own_stage), m0 + col0, w.c_row0 + q * 32);
+              bulk_commit();
+            }
+            continue;
+          }
+          uint8_t* stage = last_unit ? smem + (ew * C::kChunks + ci) * 2048 : own_stage + (n_staged & 1u) * 2048;
+          if (!last_unit) {
+            // the store before the latest one has read this buffer
+            if (lane == 0) bulk_wait_read_but_one();
+            __syncwarp();
+            ++n_staged;
+          }
+#pragma unroll
+          for (int e4 = 0; e4 < 4; ++e4) {                  // eight batch columns, one 16-byte piece
+            float y[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = fmaf(alpha, __uint_as_float(cur[e4 * 8 + e]), bias_j);
+            if constexpr (!LEAN) {
+              if (beta != 0.0f && active && col0 + e4 * 8 < m_cnt) {
+                const uint4 old = *reinterpret_cast<const uint4*>(Ct + c_row * ldc + m0 + col0 + e4 * 8);
+                const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  y[e * 2] = fmaf(beta, unpack1<DT>(static_cast<uint16_t>(ow[e] & 0xffffu)), y[e * 2]);
+                  y[e * 2 + 1] = fmaf(beta, unpack1<DT>(static_cast<uint16_t>(ow[e] >> 16)), y[e * 2 + 1]);
+                }
+              }
+            }
+            if (act == kActRelu) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) y[e] = fmaxf(y[e], 0.0f);
+            } else if (act == kActGelu) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) y[e] = apply_act(y[e], kActGelu);
+            }
+            *reinterpret_cast<uint4*>(stage + row_off + ((e4 ^ row_swz) << 4)) =
+                make_uint4(pack2<DT>(y[0], y[1]), pack2<DT>(y[2], y[3]), pack2<DT>(y[4], y[5]), pack2<DT>(y[6], y[7]));
+          }
+          if (tma_store) {
+            fence_proxy_async_smem();
+            __syncwarp();                          // the whole chunk is staged
+            if (lane == 0) {
+              tma_store_2d(&tmap_c, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
+              if constexpr (PEERS) if (tma_peers) {
+                for (int p = 0; p < ep.n_peers; ++p) {
+                  int pp = p + peer_rot;
+                  if (pp >= ep.n_peers) pp -= ep.n_peers;
+                  tma_store_2d(ep.peer_maps + pp, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
+                }
+              }
               bulk_commit();
             }
           }
-          continue;
-        }
-        uint8_t* stage_grp = last_unit ? smem + (half * kGroups + gi) * C::kEpiGroupBytes
-                                       : epi + half * C::kEpiGroupBytes;
-        if (!last_unit) {
-          // The half's staging group is free once its previous TMA store has read it (the leader
-          // waits for that) and every warp of the half has finished its previous copy-out.
-          if (leader) bulk_wait_read_all();
-          named_barrier_sync(half_bar, 128);
-        }
-#pragma unroll
-        for (int b = 0; b < kBatch; ++b) {
-          const int col0 = grp_col + b * 32;             // first batch column of the chunk
-          uint32_t(&cur)[32] = v[b];
-          uint32_t o[16];
-          if (plain) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              o[e] = pack2<DT>(alpha * __uint_as_float(cur[2 * e]),
-                               alpha * __uint_as_float(cur[2 * e + 1]));
-            }
-          } else {
-            // general form: alpha * x + beta * Ct_old + bias, then the activation
-            const bool read_old = beta != 0.0f && active && (col0 < m_cnt);
-            const uint4* cs = reinterpret_cast<const uint4*>(gdst + col0);
-#pragma unroll
-            for (int e4 = 0; e4 < 4; ++e4) {
-              uint4 old = make_uint4(0, 0, 0, 0);
-              if (read_old && col0 + e4 * 8 < m_cnt) old = cs[e4];
-              const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
+          if constexpr (!LEAN) {
+            if (!tma_store || (PEERS && ep.n_peers > 0 && !tma_peers)) {
+              // copy-out through the kept-column list: this warp's own 32 rows, eight rows per
+              // instruction, 16 bytes per lane; to Ct unless the TMA store took it, and to every peer.
+              // Tile-sharded layers: the peers are the other GPUs' copies of Ct, written over NVLink;
+              // CTAs start at different peers so that the GPUs' stores do not converge on one
+              // destination at a time.
+              __syncwarp();
+              const int piece = lane & 3, rsub = lane >> 2;
+              const bool m_ok = col0 + piece * 8 < m_cnt;
+              int cr[4];
+              uint4 val[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const float c0f = unpack1<DT>(static_cast<uint16_t>(ow[e] & 0xffffu));
-                const float c1f = unpack1<DT>(static_cast<uint16_t>(ow[e] >> 16));
-                const int idx = e4 * 8 + e * 2;
-                const float y0 = alpha * __uint_as_float(cur[idx]) + beta * c0f + bias_j;
-                const float y1 = alpha * __uint_as_float(cur[idx + 1]) + beta * c1f + bias_j;
-                o[e4 * 4 + e] = pack2<DT>(apply_act(y0, ep.act), apply_act(y1, ep.act));
+                const int row = e * 8 + rsub;                   // row inside the warp's quarter
+                cr[e] = __shfl_sync(0xffffffffu, c_row_or_none, row);
+                val[e] = *reinterpret_cast<const uint4*>(stage + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
               }
-            }
-          }
-          // staging: [tile column j][128 bytes], 16-byte chunks swizzled by j & 7
-          uint8_t* row_ptr = stage_grp + j * 128;
 #pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {
-            const int cc = b * 4 + e4;
-            *reinterpret_cast<uint4*>(row_ptr + ((cc ^ (j & 7)) << 4)) =
-                make_uint4(o[e4 * 4], o[e4 * 4 + 1], o[e4 * 4 + 2], o[e4 * 4 + 3]);
-          }
-        }
-        if (tma_store) {
-          fence_proxy_async_smem();
-          named_barrier_sync(half_bar, 128);     // the whole group is staged
-          if (leader) {
-            tma_store_2d(&tmap_c, smem_u32(stage_grp), m0 + grp_col, tile_row0);
-            if constexpr (PEERS) if (tma_peers) {
-              for (int p = 0; p < ep.n_peers; ++p) {
-                int pp = p + peer_rot;
-                if (pp >= ep.n_peers) pp -= ep.n_peers;
-                tma_store_2d(ep.peer_maps + pp, smem_u32(stage_grp), m0 + grp_col, tile_row0);
-              }
-            }
-            bulk_commit();
-          }
-        }
-        if (!tma_store || (PEERS && ep.n_peers > 0 && !tma_peers)) {
-          // copy-out through the kept-column list: this warp's own 32 rows, four rows per
-          // instruction, 16 bytes per lane; to Ct unless the TMA store took it, and to every peer.
-          // Tile-sharded layers: the peers are the other GPUs' copies of Ct, written over NVLink;
-          // CTAs start at different peers so that the GPUs' stores do not converge on one
-          // destination at a time.
-          __syncwarp();
-          const int cchunk = lane & 7, rsub = lane >> 3;
-          const bool m_ok = grp_col + cchunk * 8 < m_cnt;
-#pragma unroll
-          for (int r4 = 0; r4 < 32; r4 += 16) {
-            int cr[4];
-            uint4 val[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int lrow = r4 + e * 4 + rsub;           // row inside the warp's quarter
-              const int row = q * 32 + lrow;
-              cr[e] = __shfl_sync(0xffffffffu, c_row_or_none, lrow);
-              val[e] = *reinterpret_cast<const uint4*>(stage_grp + row * 128 + ((cchunk ^ (row & 7)) << 4));
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if (cr[e] >= 0 && m_ok) {
-                const long long off = static_cast<long long>(cr[e]) * ldc + m0 + grp_col + cchunk * 8;
-                if constexpr (PEERS) {
-                  if (ep.multicast != nullptr) {
-                    multimem_st_16(ep.multicast + off, val[e]);     // every GPU's copy, this one included
-                    continue;
+              for (int e = 0; e < 4; ++e) {
+                if (cr[e] >= 0 && m_ok) {
+                  const long long off = static_cast<long long>(cr[e]) * ldc + m0 + col0 + piece * 8;
+                  if constexpr (PEERS) {
+                    if (ep.multicast != nullptr) {
+                      multimem_st_16(ep.multicast + off, val[e]);     // every GPU's copy, this one included
+                      continue;
+                    }
                   }
-                }
-                if (!tma_store) *reinterpret_cast<uint4*>(Ct + off) = val[e];
-                if constexpr (PEERS) {
-                  for (int p = 0; p < ep.n_peers; ++p) {
-                    int pp = p + peer_rot;
-                    if (pp >= ep.n_peers) pp -= ep.n_peers;
-                    *reinterpret_cast<uint4*>(ep.peers[pp] + off) = val[e];
+                  if (!tma_store) *reinterpret_cast<uint4*>(Ct + off) = val[e];
+                  if constexpr (PEERS) {
+                    for (int p = 0; p < ep.n_peers; ++p) {
+                      int pp = p + peer_rot;
+                      if (pp >= ep.n_peers) pp -= ep.n_peers;
+                      *reinterpret_cast<uint4*>(ep.peers[pp] + off) = val[e];
+                    }
                   }
                 }
               }
+              __syncwarp();
             }
           }
-          __syncwarp();
         }
       }
-      ++acc_it;
-      w = wn;
+      word = word_next;
     }
-    // The CTA may retire once its last TMA stores have read the staging groups; the stores
+    // The CTA may retire once its last TMA stores have read the staging buffers; the stores
     // themselves complete before the grid does.
-    if (leader) bulk_wait_read_all();
+    if (lane == 0) bulk_wait_read_all();
   }
 
+  __syncwarp();   // warps 0 and 1 ran their roles on one elected thread
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

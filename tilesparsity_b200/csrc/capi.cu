@@ -85,19 +85,19 @@ int make_weight_tmap(CUtensorMap* map, int dtype, const void* base, long long ro
   return TS_OK;
 }
 
-// Tensor map over the output Ct [n_rows][ldc] for the epilogue's TMA stores: box 32 batch columns x 32
-// rows (one staging chunk of an epilogue warp), 64-byte swizzle.
+// Tensor map over the output Ct [n_rows][ldc] for the epilogue's TMA stores: box 64 batch columns x 32
+// rows (the staging buffer of an epilogue warp), 128-byte swizzle.
 int make_out_tmap(CUtensorMap* map, int dtype, const void* Ct, long long n_rows, long long M, long long ldc) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(TS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(n_rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldc) * 2};
-  cuuint32_t box[2] = {32, 32};
+  cuuint32_t box[2] = {64, 32};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, dtype == TS_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                   2, const_cast<void*>(Ct), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TS_ERR_CUDA, "cuTensorMapEncodeTiled (output) failed (%d)", (int)r);
   return TS_OK;

@@ -37,6 +37,7 @@
 // warps 2-5 = activation gather, warps 6-13 = epilogue.  (Eight gather warps were measured: 18 warps
 // leave 96 registers per thread, the kernel spills, and every workload got slower.)
 #include <cstddef>
+#include <type_traits>
 
 #include "ts_common.cuh"
 #include "ts_kernels.h"
@@ -58,12 +59,13 @@ constexpr int kMaxStages = 6;
 // one K step of the MMA.
 constexpr int kGW = 4;
 constexpr int kRowsPerWarp = kKB / kGW;
-constexpr int kEpiWarp0 = 2 + kGW;       // first epilogue warp
+constexpr int kGatherWarp0 = 2;          // warps 0 and 1: weights, MMA
+constexpr int kEpiWarp0 = kGatherWarp0 + kGW;       // first epilogue warp
 constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
 constexpr int kMetaInts = kBlockMetaInts;  // one block record: {m0, meta, 0, 0} + 64 row numbers
 constexpr int kAhead = 4;                // records are requested this many blocks ahead of the weights
 constexpr int kMaxRecs = kMaxStages + kAhead;
-constexpr int kEpiWarpBytes = 4096;      // staging of one epilogue warp: two 32-row x 32-column chunks of 2 KiB
+constexpr int kEpiWarpBytes = 4096;      // staging of one epilogue warp: 32 rows x 64 batch columns
 
 struct Barriers {
   uint64_t full[kMaxStages];
@@ -94,7 +96,7 @@ struct Cfg {
   static_assert(kUsedBytes <= kSmemBytes, "stages, staging and barriers exceed the shared memory of one CTA");
   static constexpr int kLanesPerRow = MT / 8;       // 16-byte chunks in one gathered row
   static constexpr int kRowsPerInstr = 32 / kLanesPerRow;
-  static constexpr int kChunks = MT / 64;           // 32-column chunks per epilogue warp
+  static constexpr int kGroups = MT / 128;          // 64-column groups of a unit per epilogue warp
 };
 
 __device__ __forceinline__ WorkItem load_item(const WorkItem* p) {
@@ -154,26 +156,44 @@ __device__ __forceinline__ long long c_row_of(const EpiItem& w, int j) {
   return w.c_row0 + (w.n_list ? __ldg(w.n_list + j) + ((w.flags & kItemRelative) ? j : 0) : j);
 }
 
+// gelu(x) = x * 0.5 * (1 + tanh(u)), u = sqrt(2/pi) * (x + 0.044715 x^3)  (Pruning/BERT/utils/modeling.py:264-277),
+// for two values, written as x / (1 + exp(-2u)): the same function without the cancellation of 1 + tanh for
+// negative u.  The special-function unit bounds it (16 results per cycle and SM), so the two share one
+// reciprocal, 1 / (a b): three special-function instructions a pair.  exp's argument is cut at 2^60, so that
+// the product stays finite; beyond that the result is below 1e-17 |x| anyway.
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float gelu_denominator(float x) {
+  // -2u * log2(e) = x * (-2 sqrt(2/pi) log2(e)) * (1 + 0.044715 x^2)
+  const float p = fmaf(x * x, -0.10294324f, -2.3022082f);
+  return 1.0f + ex2_approx(fminf(x * p, 60.0f));
+}
+__device__ __forceinline__ void gelu2(float& x0, float& x1) {
+  const float a = gelu_denominator(x0), b = gelu_denominator(x1);
+  const float r = rcp_approx(a * b);
+  x0 *= r * b;
+  x1 *= r * a;
+}
+
 __device__ __forceinline__ float apply_act(float x, int act) {
   if (act == kActRelu) return fmaxf(x, 0.0f);
-  if (act == kActGelu) {
-    // x * 0.5 * (1 + tanh(u)), u = sqrt(2/pi) * (x + 0.044715 x^3)  (Pruning/BERT/utils/modeling.py:264-277),
-    // written as x / (1 + exp(-2u)), which is the same function without the cancellation of 1 + tanh for
-    // negative u; two special-function instructions instead of tanhf's branches (the epilogue of a
-    // 256 x 128 unit spent 17000 cycles on tanhf).
-    const float u2 = 1.5957691216057308f * (x + 0.044715f * x * x * x);
-    return __fdividef(x, 1.0f + __expf(-u2));
-  }
+  if (act == kActGelu) return x * rcp_approx(gelu_denominator(x));
   return x;
 }
 
-// MODE selects what the epilogue can do: kModeLean only alpha * acc through TMA tile stores (the host
-// picks it when beta == 0, there is no bias or activation and every scheduled tile keeps 128 consecutive
-// columns), kModePlain every epilogue form and the list-driven stores, kModeSplit in addition the fp32
-// partial sums of split-K parts, kModePeers the copies for the other GPUs of a tile-sharded layer.
-// Code a call cannot reach stays out of the variant it runs; measured on the BERT layer step (39.6 us):
-// the split-K code inside the common kernel +1.3 %, the peers' TMA stores +3.3 %, and the lean variant
-// against the plain one -3 %.
+// MODE selects what the epilogue can do: kModeLean act(alpha * acc + bias) through TMA tile stores only (the
+// host picks it when beta == 0 and every scheduled tile keeps 128 consecutive columns), kModePlain every
+// epilogue form and the list-driven stores, kModeSplit in addition the fp32 partial sums of split-K parts,
+// kModePeers the copies for the other GPUs of a tile-sharded layer.  Code a call cannot reach stays out of
+// the variant it runs: the hot loops share one instruction cache.
 constexpr int kModePlain = 0, kModeSplit = 1, kModePeers = 2, kModeLean = 3;
 template <int DT, int MT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -344,7 +364,7 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
     constexpr int kLpr = C::kLanesPerRow, kRpi = C::kRowsPerInstr;
     const int chunk = lane % kLpr, sub = lane / kLpr;
     const int g = chunk >> 3, c = chunk & 7;
-    const int row_base = (warp - 2) * kRowsPerWarp;         // first row of the warp's slice
+    const int row_base = (warp - kGatherWarp0) * kRowsPerWarp;         // first row of the warp's slice
     int rr[kRowsPerWarp], rn[kRowsPerWarp];
     int m0 = 0, m0_next;
     uint32_t meta = kBlockEnd, meta_next;
@@ -420,22 +440,21 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       for (int e = 0; e < kRowsPerWarp; ++e) rr[e] = rn[e];
     }
     cp_async_wait_all();  // nothing of this thread is in flight when the CTA retires
-  } else if (warp >= kEpiWarp0) {
+  } else {
     // ------------------------------------------------------------------ epilogue
-    // Every warp works alone: it owns 32 tile columns (its TMEM lane quarter) and every other 32-column
-    // chunk of the unit's batch, stages a chunk (32 rows x 64 bytes, 64-byte swizzle) in one of two
-    // buffers of its own and sends it off, as one TMA tile store where its 32 rows are consecutive rows of
-    // Ct, else with 16-byte stores through the kept-column list.  No barrier between warps: with staging
-    // groups shared by four warps a 256 x 128 unit took 3500-5000 cycles here, most of them waiting.
+    // Every warp works alone: it owns 32 tile columns (its TMEM lane quarter) and every other 64-column
+    // group of the unit's batch, stages a group (32 rows x 128 bytes, 128-byte swizzle) in a buffer of its
+    // own and sends it off, as one TMA tile store where its 32 rows are consecutive rows of Ct, else with
+    // 16-byte stores through the kept-column list.  No barrier between warps.  What bounds it is the SM's
+    // store path (32 bytes per cycle: 2048 cycles for a 256 x 128 unit; 6.4 TB/s over the GPU), whatever
+    // the kind of store; direct stores instead of TMA take that time from the gather's load/store queue
+    // (2048 x 4096 layer at 6400 rows: 51 thousand cycles per CTA instead of 44).
     const int ew = warp - kEpiWarp0;             // 0..7
-    const int half = ew >> 2;                    // takes the 32-column chunks half, half+2, ...
+    const int half = ew >> 2;                    // takes the 64-column groups half, half+2, ...
     const int q = warp & 3;                      // TMEM lane quarter this warp may read
     const int j = q * 32 + lane;                 // tile column owned by this thread
     const int peer_rot = (PEERS && ep.n_peers > 0) ? cta % ep.n_peers : 0;   // the peer this CTA writes first
     uint8_t* const own_stage = epi + ew * kEpiWarpBytes;
-    // this lane's row of a staging chunk, and the 16-byte pieces of it in swizzled order
-    const int row_off = lane * 64, row_swz = (lane >> 1) & 3;
-    uint32_t n_staged = 0;
     // Work items are held one word per lane, the next one in flight while this one is worked on: whole
     // copies in every lane cost the registers that two TMEM chunks need.
     const int* const items = reinterpret_cast<const int*>(sched + cta) + lane;
@@ -457,7 +476,7 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                       (!PEERS || ep.multicast == nullptr));
       const bool tma_peers = PEERS && tma_store && ep.peer_maps != nullptr;   // the peers' copies leave by TMA too
       // The CTA's last unit: every K block has been consumed, so the pipeline stages are free and
-      // each chunk gets a staging buffer of its own there; none waits for a store before it.
+      // each group gets a staging buffer of its own there; none waits for a store before it.
       const bool last_unit = __shfl_sync(0xffffffffu, word_next, kItemWordTile) < 0;
       const long long c_row = active ? c_row_of(w, j) : 0;
       const int c_row_or_none = active ? static_cast<int>(c_row) : -1;
@@ -467,116 +486,126 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + a * MT + (static_cast<uint32_t>(q * 32) << 16);
       const bool has_acc = w.has_rows;
-      // Not unrolled: the hot code stays small enough for the instruction cache it shares with the other
-      // roles, and one chunk's registers leave room for everything else (with two the kernel spilled, and
-      // a spilled register waits behind the gather's copies in the load/store queue).
+      // Not unrolled, and 32 accumulators in registers at a time: the hot code stays small enough for the
+      // instruction cache it shares with the other roles, and nothing spills (a spilled register waits
+      // behind the gather's copies in the load/store queue: with 64 accumulators a unit took 7000 cycles).
 #pragma unroll 1
-      for (int ci = 0; ci < C::kChunks; ++ci) {
-        const int col0 = (ci * 2 + half) * 32;              // first batch column of the chunk
-        const bool live = col0 < m_cnt;                     // uniform over the warp
-        uint32_t cur[32];
-        if (has_acc && live) {
-          tmem_ld_32x32(taddr + col0, cur);
-          tmem_ld_wait();
-        } else {
+      for (int gi = 0; gi < C::kGroups; ++gi) {
+        const int col0 = (gi * 2 + half) * 64;              // first batch column of the group
+        const int cols = m_cnt - col0;                      // (uniform over the warp)
+        uint8_t* stage = last_unit ? smem + (ew * C::kGroups + gi) * kEpiWarpBytes : own_stage;
+#pragma unroll 1
+        for (int b = 0; b < 2; ++b) {
+          uint32_t v[32];
+          if (has_acc && cols > b * 32) {
+            tmem_ld_32x32(taddr + col0 + b * 32, v);
+            tmem_ld_wait();
+          } else {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) cur[e] = 0u;
-        }
-        if (ci + 1 == C::kChunks) {
-          // every TMEM read of this accumulator by this warp has completed: hand it back to the MMA warp
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[a]));
-        }
-        if (!live) continue;
-        {
+            for (int e = 0; e < 32; ++e) v[e] = 0u;
+          }
+          if (gi + 1 == C::kGroups && b == 1) {
+            // every TMEM read of this accumulator by this warp has completed: hand it back to the MMA warp
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[a]));
+          }
+          if (cols <= b * 32) continue;
           if constexpr (SPLIT) if (w.flags & kItemScratch) {
-            // split-K part: alpha * acc leaves as fp32 for the part's scratch rows (32 rows x 128 bytes,
-            // 128-byte swizzle, both staging buffers); bias, beta and the activation are applied by the
-            // kernel that adds the parts up.  (Tile columns past n_count carry zero weights, so their rows
-            // receive zeros.)
+            // split-K part: alpha * acc leaves as fp32 for the part's scratch rows (32 rows x 128 bytes);
+            // bias, beta and the activation are applied by the kernel that adds the parts up.  (Tile
+            // columns past n_count carry zero weights, so their rows receive zeros.)
             if (lane == 0) bulk_wait_read_all();
             __syncwarp();
-            uint8_t* row_ptr = own_stage + lane * 128;
 #pragma unroll
             for (int cc = 0; cc < 8; ++cc) {
-              *reinterpret_cast<float4*>(row_ptr + ((cc ^ (lane & 7)) << 4)) =
-                  make_float4(alpha * __uint_as_float(cur[cc * 4]), alpha * __uint_as_float(cur[cc * 4 + 1]),
-                              alpha * __uint_as_float(cur[cc * 4 + 2]), alpha * __uint_as_float(cur[cc * 4 + 3]));
+              *reinterpret_cast<float4*>(own_stage + lane * 128 + ((cc ^ (lane & 7)) << 4)) =
+                  make_float4(alpha * __uint_as_float(v[cc * 4]), alpha * __uint_as_float(v[cc * 4 + 1]),
+                              alpha * __uint_as_float(v[cc * 4 + 2]), alpha * __uint_as_float(v[cc * 4 + 3]));
             }
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_store_2d(ep.scratch_map, smem_u32(own_stage), m0 + col0, w.c_row0 + q * 32);
+              tma_store_2d(ep.scratch_map, smem_u32(own_stage), m0 + col0 + b * 32, w.c_row0 + q * 32);
               bulk_commit();
             }
             continue;
           }
-          uint8_t* stage = last_unit ? smem + (ew * C::kChunks + ci) * 2048 : own_stage + (n_staged & 1u) * 2048;
-          if (!last_unit) {
-            // the store before the latest one has read this buffer
-            if (lane == 0) bulk_wait_read_but_one();
+          if (b == 0 && !last_unit) {
+            if (lane == 0) bulk_wait_read_all();            // the store before this one has read the buffer
             __syncwarp();
-            ++n_staged;
           }
+          uint8_t* const row_ptr = stage + lane * 128;
+          auto convert = [&](auto act_c) {
+            constexpr int kAct = decltype(act_c)::value;
 #pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {                  // eight batch columns, one 16-byte piece
-            float y[8];
+            for (int p = 0; p < 4; ++p) {                   // eight batch columns, one 16-byte piece
+              float y[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) y[e] = fmaf(alpha, __uint_as_float(cur[e4 * 8 + e]), bias_j);
-            if constexpr (!LEAN) {
-              if (beta != 0.0f && active && col0 + e4 * 8 < m_cnt) {
-                const uint4 old = *reinterpret_cast<const uint4*>(Ct + c_row * ldc + m0 + col0 + e4 * 8);
-                const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
+              for (int e = 0; e < 8; ++e) y[e] = fmaf(alpha, __uint_as_float(v[p * 8 + e]), bias_j);
+              if constexpr (!LEAN) {
+                const int col = b * 32 + p * 8;
+                if (beta != 0.0f && active && col < cols) {
+                  const uint4 old = *reinterpret_cast<const uint4*>(Ct + c_row * ldc + m0 + col0 + col);
+                  const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  y[e * 2] = fmaf(beta, unpack1<DT>(static_cast<uint16_t>(ow[e] & 0xffffu)), y[e * 2]);
-                  y[e * 2 + 1] = fmaf(beta, unpack1<DT>(static_cast<uint16_t>(ow[e] >> 16)), y[e * 2 + 1]);
+                  for (int e = 0; e < 4; ++e) {
+                    y[e * 2] = fmaf(beta, unpack1<DT>(static_cast<uint16_t>(ow[e] & 0xffffu)), y[e * 2]);
+                    y[e * 2 + 1] = fmaf(beta, unpack1<DT>(static_cast<uint16_t>(ow[e] >> 16)), y[e * 2 + 1]);
+                  }
                 }
               }
-            }
-            if (act == kActRelu) {
+              if constexpr (kAct == kActRelu) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) y[e] = fmaxf(y[e], 0.0f);
-            } else if (act == kActGelu) {
-#pragma unroll
-              for (int e = 0; e < 8; ++e) y[e] = apply_act(y[e], kActGelu);
-            }
-            *reinterpret_cast<uint4*>(stage + row_off + ((e4 ^ row_swz) << 4)) =
-                make_uint4(pack2<DT>(y[0], y[1]), pack2<DT>(y[2], y[3]), pack2<DT>(y[4], y[5]), pack2<DT>(y[6], y[7]));
-          }
-          if (tma_store) {
-            fence_proxy_async_smem();
-            __syncwarp();                          // the whole chunk is staged
-            if (lane == 0) {
-              tma_store_2d(&tmap_c, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
-              if constexpr (PEERS) if (tma_peers) {
-                for (int p = 0; p < ep.n_peers; ++p) {
-                  int pp = p + peer_rot;
-                  if (pp >= ep.n_peers) pp -= ep.n_peers;
-                  tma_store_2d(ep.peer_maps + pp, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
-                }
+                for (int e = 0; e < 8; ++e) y[e] = fmaxf(y[e], 0.0f);
               }
-              bulk_commit();
+              if constexpr (kAct == kActGelu) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) gelu2(y[e * 2], y[e * 2 + 1]);
+              }
+              *reinterpret_cast<uint4*>(row_ptr + (((b * 4 + p) ^ (lane & 7)) << 4)) =
+                  make_uint4(pack2<DT>(y[0], y[1]), pack2<DT>(y[2], y[3]), pack2<DT>(y[4], y[5]), pack2<DT>(y[6], y[7]));
             }
+          };
+          if (act == kActNone) convert(std::integral_constant<int, kActNone>{});
+          else if (act == kActRelu) convert(std::integral_constant<int, kActRelu>{});
+          else convert(std::integral_constant<int, kActGelu>{});
+        }
+        if (cols <= 0) continue;
+        if constexpr (SPLIT) if (w.flags & kItemScratch) continue;
+        if (tma_store) {
+          fence_proxy_async_smem();
+          __syncwarp();                          // the whole group is staged
+          if (lane == 0) {
+            tma_store_2d(&tmap_c, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
+            if constexpr (PEERS) if (tma_peers) {
+              for (int p = 0; p < ep.n_peers; ++p) {
+                int pp = p + peer_rot;
+                if (pp >= ep.n_peers) pp -= ep.n_peers;
+                tma_store_2d(ep.peer_maps + pp, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
+              }
+            }
+            bulk_commit();
           }
-          if constexpr (!LEAN) {
-            if (!tma_store || (PEERS && ep.n_peers > 0 && !tma_peers)) {
-              // copy-out through the kept-column list: this warp's own 32 rows, eight rows per
-              // instruction, 16 bytes per lane; to Ct unless the TMA store took it, and to every peer.
-              // Tile-sharded layers: the peers are the other GPUs' copies of Ct, written over NVLink;
-              // CTAs start at different peers so that the GPUs' stores do not converge on one
-              // destination at a time.
-              __syncwarp();
-              const int piece = lane & 3, rsub = lane >> 2;
-              const bool m_ok = col0 + piece * 8 < m_cnt;
+        }
+        if constexpr (!LEAN) {
+          if (!tma_store || (PEERS && ep.n_peers > 0 && !tma_peers)) {
+            // copy-out through the kept-column list: this warp's own 32 rows, four rows per instruction,
+            // 16 bytes per lane; to Ct unless the TMA store took it, and to every peer.  Tile-sharded
+            // layers: the peers are the other GPUs' copies of Ct, written over NVLink; CTAs start at
+            // different peers so that the GPUs' stores do not converge on one destination at a time.
+            __syncwarp();
+            const int piece = lane & 7, rsub = lane >> 3;
+            const bool m_ok = piece * 8 < cols;
+#pragma unroll
+            for (int r4 = 0; r4 < 32; r4 += 16) {
               int cr[4];
               uint4 val[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const int row = e * 8 + rsub;                   // row inside the warp's quarter
+                const int row = r4 + e * 4 + rsub;              // row inside the warp's quarter
                 cr[e] = __shfl_sync(0xffffffffu, c_row_or_none, row);
-                val[e] = *reinterpret_cast<const uint4*>(stage + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
+                val[e] = *reinterpret_cast<const uint4*>(stage + row * 128 + ((piece ^ (row & 7)) << 4));
               }
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -598,8 +627,8 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                   }
                 }
               }
-              __syncwarp();
             }
+            __syncwarp();
           }
         }
       }
@@ -742,8 +771,8 @@ cudaError_t masked_gemm_launch(int dtype, int unit_rows, const CUtensorMap& tmap
   if (ep.n_peers > 0 || ep.multicast != nullptr) {
     return unit_rows == 256 ? TS_LAUNCH_DT(256, kModePeers) : TS_LAUNCH_DT(128, kModePeers);
   }
-  // lean: the caller has checked that every unit takes the TMA store and that the epilogue is alpha * acc
-  if (lean && tmap_c != nullptr && ep.beta == 0.0f && ep.bias == nullptr && ep.act == kActNone) {
+  // lean: the caller has checked that every unit takes the TMA store
+  if (lean && tmap_c != nullptr && ep.beta == 0.0f) {
     return unit_rows == 256 ? TS_LAUNCH_DT(256, kModeLean) : TS_LAUNCH_DT(128, kModeLean);
   }
   return unit_rows == 256 ? TS_LAUNCH_DT(256, kModePlain) : TS_LAUNCH_DT(128, kModePlain);

@@ -329,11 +329,6 @@ __device__ __forceinline__ void bulk_wait_read_all() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// ... all but the latest store has been read from shared memory
-__device__ __forceinline__ void bulk_wait_read_but_one() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-}
-
 __device__ __forceinline__ void bulk_wait_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }

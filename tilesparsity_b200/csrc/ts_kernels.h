@@ -21,7 +21,7 @@ namespace ts {
 // allows programmatic dependent launch: the kernel reads sched, block_meta and the packed weights before
 // it waits for the kernel before it in the stream, so it must be false when that kernel wrote them.
 // lean: every unit of the schedule has kItemDenseRows set (the kernel then takes its store-only variant
-// when the epilogue is alpha * acc).
+// when beta is 0).
 cudaError_t masked_gemm_launch(int dtype, int unit_rows, const CUtensorMap& tmap_w, const CUtensorMap* tmap_c,
                                const WorkItem* sched, int rounds, int grid, const int* block_meta,
                                int blk_stride, const void* At, long long lda, void* Ct, long long ldc, int M,

@@ -103,6 +103,10 @@ int ts_layer_stats(const ts_layer_t* layer, int64_t* kept_flops_per_row, int64_t
 int ts_masked_gemm(ts_layer_t* layer, int M, const void* At_dev, int64_t lda, void* Ct_dev,
                    int64_t ldc, float alpha, float beta, void* stream);
 
+/* Zeroes the rows of Ct whose column no tile keeps (ts_masked_gemm never writes them); nothing is launched
+ * when every column is kept.  No reference counterpart. */
+int ts_layer_zero_pruned(ts_layer_t* layer, int M, void* Ct_dev, int64_t ldc, void* stream);
+
 /* Fused epilogue of ts_masked_gemm_ex:  Ct[n][m] = act(alpha * acc + beta * Ct[n][m] + bias[n]).
  *   bias_dev     fp32 [N] on the device, indexed by the column of W (row of Ct), or NULL
  *   activation   TS_ACT_NONE, TS_ACT_RELU, or TS_ACT_GELU (the tanh form of the reference's BERT,

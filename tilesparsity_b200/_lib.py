@@ -63,6 +63,7 @@ SIGNATURES = {
     "ts_layer_stats": (C.c_int, [_vp, _i64p, _i64p, _i64p, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "ts_masked_gemm": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp, C.c_int64, C.c_float, C.c_float, _vp]),
     "ts_masked_gemm_ex": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp, C.c_int64, C.POINTER(Epilogue), _vp]),
+    "ts_layer_zero_pruned": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp]),
     "ts_masked_gemm_simt": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp, C.c_int64, C.c_float, C.c_float, _vp]),
     "ts_masked_gemm_host": (C.c_int, [_vp, C.c_int, _vp, _vp, C.c_float, C.c_float, _vp]),
     "ts_masked_gemm_host_async": (C.c_int, [_vp, C.c_int, _vp, _vp, C.c_float, C.c_float, _vp]),
@@ -121,3 +122,22 @@ def last_error() -> str:
 def check(code: int) -> None:
     if code != TS_OK:
         raise TileSparseError(code, last_error())
+
+
+def fast():
+    """The _tsfast extension (host path of the per-batch operators); loads torch."""
+    global _fast
+    if _fast is None:
+        import torch  # noqa: F401  (the extension links against it)
+        path = os.path.join(HERE, "_tsfast.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python tilesparsity_b200/build.py`")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("_tsfast", path)
+        _fast = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_fast)
+        _fast.bind(TileSparseError)
+    return _fast
+
+
+_fast = None

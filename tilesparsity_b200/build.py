@@ -1,24 +1,29 @@
-"""In-tree build of libtilesparse.so for sm_100a.
+"""In-tree build of libtilesparse.so (sm_100a) and of the _tsfast extension.
 
-`python tilesparsity_b200/build.py` compiles every file under csrc/ with nvcc (cross-compiles
-without a GPU) and writes the shared library next to this file, where the loader looks for it.
+`python tilesparsity_b200/build.py` compiles every .cu file under csrc/ with nvcc (cross-compiles
+without a GPU) and links the shared library next to this file, where the loader looks for it; then
+csrc/pyfast.cpp, the host path of the per-batch operators, with g++ against the installed torch.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
+OBJ = os.path.join(CSRC, "obj")
 LIB_PATH = os.path.join(HERE, "libtilesparse.so")
+EXT_PATH = os.path.join(HERE, "_tsfast.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",
-    "-shared",
 ]
 
 
@@ -26,12 +31,16 @@ def sources() -> list[str]:
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _headers() -> list[str]:
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))] + \
+        [os.path.join(HERE, "..", "include", "tilesparse.h")]
+
+
+def _older(path: str, deps: list[str]) -> bool:
+    """Whether `path` is missing or older than one of `deps`."""
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
-    deps.append(os.path.join(HERE, "..", "include", "tilesparse.h"))
+    t = os.path.getmtime(path)
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
@@ -42,21 +51,48 @@ def find_nvcc() -> str:
     return nvcc
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Builds the library if it is missing or older than its sources; returns its path."""
-    if not force and not _stale():
-        return LIB_PATH
-    cmd = [find_nvcc(), *NVCC_FLAGS]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    tmp = LIB_PATH + ".tmp"
-    cmd += ["-o", tmp, *sources()]
+def _run(cmd: list[str]) -> str:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
-    if verbose:
-        sys.stderr.write(proc.stderr)
-    os.replace(tmp, LIB_PATH)
+        raise RuntimeError(cmd[0] + " failed:\n" + proc.stdout + proc.stderr)
+    return proc.stderr
+
+
+def _build_library(force: bool, verbose: bool) -> None:
+    os.makedirs(OBJ, exist_ok=True)
+    nvcc, flags = find_nvcc(), NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else [])
+    objects, todo = [], []
+    for src in sources():
+        obj = os.path.join(OBJ, os.path.basename(src)[:-3] + ".o")
+        objects.append(obj)
+        if force or _older(obj, [src] + _headers()):
+            todo.append([nvcc, *flags, "-c", "-o", obj, src])
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        for err in pool.map(_run, todo):
+            if verbose:
+                sys.stderr.write(err)
+    _run([nvcc, *NVCC_FLAGS, "-shared", "-o", LIB_PATH + ".tmp", *objects])
+    os.replace(LIB_PATH + ".tmp", LIB_PATH)
+
+
+def _build_extension() -> None:
+    root = os.path.dirname(importlib.util.find_spec("torch").origin)
+    inc, lib = os.path.join(root, "include"), os.path.join(root, "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
+    _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+          "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + cuda,
+          "-I" + sysconfig.get_paths()["include"], "-o", EXT_PATH + ".tmp", os.path.join(CSRC, "pyfast.cpp"),
+          "-L" + HERE, "-l:libtilesparse.so", "-Wl,-rpath,$ORIGIN", "-L" + lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
+          "-lc10_cuda", "-lc10"])
+    os.replace(EXT_PATH + ".tmp", EXT_PATH)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Builds what is missing or older than its sources; returns the library's path."""
+    if force or _older(LIB_PATH, sources() + _headers()):
+        _build_library(force, verbose)
+    if force or _older(EXT_PATH, [os.path.join(CSRC, "pyfast.cpp"), os.path.join(HERE, "..", "include", "tilesparse.h")]):
+        _build_extension()
     return LIB_PATH
 
 

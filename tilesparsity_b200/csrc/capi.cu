@@ -136,6 +136,15 @@ struct Schedule {
   float* d_scratch = nullptr;
   long long scratch_ld = 0;
   CUtensorMap* d_scratch_map = nullptr;   // tensor map over d_scratch, in device memory
+  // Tensor maps over the outputs of the latest calls (a program alternates between a few buffers; encoding
+  // one takes about as long as the rest of a call's bookkeeping)
+  struct OutMap {
+    const void* ct = nullptr;
+    long long ldc = 0;
+    CUtensorMap map;
+  };
+  OutMap out_maps[4];
+  int next_out_map = 0;
   bool all_dense = false;                 // every unit's tile keeps 128 consecutive columns (TMA tile stores only)
 };
 
@@ -526,7 +535,8 @@ struct ts_layer {
   std::vector<int> k_counts, n_counts;
   int max_k = 0;
   int* d_kept_k = nullptr;
-  int* d_kept_n = nullptr;
+  int* d_kept_n = nullptr;     // kept columns, then (from n_kept on) the columns no tile keeps
+  int n_kept = 0, n_pruned = 0;
   ts::TileDesc* d_tiles = nullptr;
   std::vector<ts::TileDesc> h_tiles;
   uint16_t* d_wp = nullptr;
@@ -836,6 +846,13 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
   l->ldw = std::max<long long>(64, (l->max_k + 63) / 64 * 64);
   l->wp_rows = static_cast<long long>(std::max(1, n_tiles)) * 128;
   TS_CUDA(cudaMalloc(&l->d_kept_k, std::max<size_t>(1, kk.size()) * sizeof(int)));
+  std::vector<char> kept(l->N, 0);
+  for (int v : nn) kept[v] = 1;
+  l->n_kept = static_cast<int>(nn.size());
+  for (int v = 0; v < l->N; ++v) {
+    if (!kept[v]) nn.push_back(v);
+  }
+  l->n_pruned = static_cast<int>(nn.size()) - l->n_kept;
   TS_CUDA(cudaMalloc(&l->d_kept_n, std::max<size_t>(1, nn.size()) * sizeof(int)));
   TS_CUDA(cudaMalloc(&l->d_tiles, std::max(1, n_tiles) * sizeof(ts::TileDesc)));
   TS_CUDA(cudaMalloc(&l->d_wp, static_cast<size_t>(l->wp_rows) * l->ldw * 2));
@@ -977,9 +994,20 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   ep.scratch = s->d_scratch;
   ep.scratch_ld = s->scratch_ld;
   ep.scratch_map = s->d_scratch_map;
-  CUtensorMap tmap_c;
-  rc = make_out_tmap(&tmap_c, l->dtype, Ct, l->N, M, ldc);
-  if (rc != TS_OK) return rc;
+  const CUtensorMap* tmap_c = nullptr;
+  for (const Schedule::OutMap& m : s->out_maps) {
+    if (m.ct == Ct && m.ldc == ldc) tmap_c = &m.map;
+  }
+  if (!tmap_c) {
+    Schedule::OutMap& m = s->out_maps[s->next_out_map];
+    m.ct = nullptr;
+    rc = make_out_tmap(&m.map, l->dtype, Ct, l->N, M, ldc);
+    if (rc != TS_OK) return rc;
+    m.ct = Ct;
+    m.ldc = ldc;
+    s->next_out_map = (s->next_out_map + 1) % 4;
+    tmap_c = &m.map;
+  }
   // Tile-sharded layers: the peers' copies of a full tile leave by TMA stores as well.  The maps are
   // encoded once per set of peer buffers and kept on the device.
   ep.peer_maps = nullptr;
@@ -1007,7 +1035,7 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   // The first launch after ts_layer_pack_weights may directly follow the packing kernel, so it runs
   // as an ordinary (fully ordered) launch; from then on the weights are old data.
   const bool early = !l->wp_fresh;
-  TS_CUDA(ts::masked_gemm_launch(l->dtype, s->unit_rows, l->tmap, &tmap_c, s->d_units, s->rounds,
+  TS_CUDA(ts::masked_gemm_launch(l->dtype, s->unit_rows, l->tmap, tmap_c, s->d_units, s->rounds,
                                  s->grid, s->d_meta, s->blk_stride, At, lda, Ct, ldc, M, ep, l->d_status,
                                  early, s->all_dense, static_cast<cudaStream_t>(stream)));
   l->wp_fresh = false;
@@ -1020,6 +1048,17 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
 }  // namespace
 
 extern "C" {
+
+int ts_layer_zero_pruned(ts_layer_t* l, int M, void* Ct, int64_t ldc, void* stream) {
+  if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
+  if (M < 0 || (M % 8) != 0) return fail(TS_ERR_INVALID, "M=%d must be a non-negative multiple of 8", M);
+  if (M == 0 || l->n_pruned == 0) return TS_OK;
+  if (!Ct || (reinterpret_cast<uintptr_t>(Ct) & 15u) || ldc < M || (ldc % 8) != 0) {
+    return fail(TS_ERR_INVALID, "Ct must be non-NULL and 16-byte aligned, ldc=%lld a multiple of 8 and >= M=%d", (long long)ldc, M);
+  }
+  TS_CUDA(ts::zero_rows_launch(l->d_kept_n + l->n_kept, l->n_pruned, Ct, ldc, M, static_cast<cudaStream_t>(stream)));
+  return TS_OK;
+}
 
 int ts_masked_gemm_ex(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc,
                       const ts_epilogue_t* epi, void* stream) {

@@ -82,7 +82,23 @@ transpose16_kernel(const uint16_t* __restrict__ in, long long ld_in, uint16_t* _
   }
 }
 
+// Ct[rows[blockIdx.y]][0 .. M) = 0, eight elements per thread.
+__global__ void __launch_bounds__(256)
+zero_rows_kernel(const int* __restrict__ rows, uint16_t* __restrict__ Ct, long long ldc, int M) {
+  const int m = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (m < M) *reinterpret_cast<uint4*>(Ct + static_cast<long long>(__ldg(rows + blockIdx.y)) * ldc + m) = make_uint4(0, 0, 0, 0);
+}
+
 }  // namespace
+
+cudaError_t zero_rows_launch(const int* rows, int n_rows, void* Ct, long long ldc, int M, cudaStream_t stream) {
+  const unsigned bx = static_cast<unsigned>((M / 8 + 255) / 256);
+  for (int r = 0; r < n_rows; r += 65535) {     // rows are the grid's y dimension
+    zero_rows_kernel<<<dim3(bx, static_cast<unsigned>(n_rows - r < 65535 ? n_rows - r : 65535)), 256, 0, stream>>>(
+        rows + r, static_cast<uint16_t*>(Ct), ldc, M);
+  }
+  return cudaGetLastError();
+}
 
 cudaError_t pack_weights_launch(int w_dtype, int out_dtype, const void* W, long long ld_w,
                                 const TileDesc* tiles, int n_tiles, int max_k, void* Wp,

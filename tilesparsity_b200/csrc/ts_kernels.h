@@ -51,6 +51,9 @@ cudaError_t pack_weights_launch(int w_dtype, int out_dtype, const void* W, long 
                                 const TileDesc* tiles, int n_tiles, int max_k, void* Wp,
                                 long long ldw, cudaStream_t stream);
 
+// Ct[rows[i]][0 .. M) = 0 for n_rows rows of a 16-bit matrix (pack.cu).
+cudaError_t zero_rows_launch(const int* rows, int n_rows, void* Ct, long long ldc, int M, cudaStream_t stream);
+
 // Sparse residual term (residual.cu): Ct[n][m] = (col_written[n] ? Ct[n][m] : 0) + alpha * sum over the
 // non-zeros p of column n of val[p] * At[row_idx[p]][m].  col_written may be nullptr (all written).
 cudaError_t residual_spmm_launch(int dtype, const int* col_ptr, const int* row_idx, const void* val,

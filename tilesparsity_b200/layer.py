@@ -18,6 +18,8 @@ from . import _lib
 from ._lib import check, lib
 from .tiles import TileSet, tiles_from_lists, tiles_from_mask
 
+_masked_gemm = _lib.fast().masked_gemm
+
 _TS_DTYPE = {torch.float16: _lib.TS_DTYPE_F16, torch.bfloat16: _lib.TS_DTYPE_BF16,
              torch.float32: _lib.TS_DTYPE_F32}
 
@@ -46,6 +48,8 @@ class TWLayer:
         self._h = C.c_void_p()
         with torch.cuda.device(self.device):
             check(lib.ts_layer_create(C.byref(self._h), self.K, self.N, self.G, _TS_DTYPE[dtype]))
+            if self.device.index is None:
+                self.device = torch.device("cuda", torch.cuda.current_device())
         self.retile(tiles)
 
     def retile(self, tiles: TileSet) -> None:
@@ -60,6 +64,8 @@ class TWLayer:
             self._np, npp = _i32(tiles.tile_n_ptr)
             self._nn, nn = _i32(tiles.kept_n)
             check(lib.ts_layer_set_tiles(self._h, tiles.n_tiles, kp, kk, npp, nn, _lib.TS_INDEX_ABSOLUTE))
+        self._desc = _lib.fast().layer_desc(self._h.value, self.K, self.N, int(self.dtype == torch.bfloat16),
+                                            self.device.index, int(len(np.unique(tiles.kept_n)) == self.N))
 
     # ------------------------------------------------------------------ construction
     @classmethod
@@ -135,6 +141,7 @@ class TWLayer:
         if getattr(self, "_h", None) is not None and self._h.value:
             lib.ts_layer_destroy(self._h)
             self._h = C.c_void_p()
+            self._desc = None
 
     def __del__(self):
         try:
@@ -190,6 +197,10 @@ class TWLayer:
         `multicast` is instead the NVSwitch multicast address of `out` (the switch delivers every
         store to all GPUs' copies, this one included).
         """
+        if not (simt or peers or multicast):
+            if activation not in _lib.ACTIVATIONS:
+                raise ValueError(f"unknown activation {activation!r}")
+            return _masked_gemm(self._desc, At, out, alpha, beta, bias, _lib.ACTIVATIONS[activation])
         if At.dim() != 2 or At.shape[0] != self.K or At.dtype != self.dtype or At.device != self.device:
             raise ValueError(f"At must be a [{self.K}, M] {self.dtype} tensor on {self.device}")
         if At.stride(1) != 1:

@@ -137,6 +137,15 @@ typedef struct ts_epilogue {
 int ts_masked_gemm_ex(ts_layer_t* layer, int M, const void* At_dev, int64_t lda, void* Ct_dev,
                       int64_t ldc, const ts_epilogue_t* epilogue, void* stream);
 
+/* The same with a row-major output C[m][n], C_dev [M][ldc] (what `A @ (W * mask)` returns), written by the
+ * GEMM's epilogue itself instead of by a transposition of Ct.  Possible when the tiles keep all columns, each
+ * a run that starts at a multiple of 8, and no tile pays for split-K at this batch size:
+ * ts_layer_row_output sets *supported to 1 then.  beta and peer buffers are not supported.  The reference
+ * keeps its outputs column-major (basic_nn.cu:412-426). */
+int ts_layer_row_output(ts_layer_t* layer, int M, int* supported);
+int ts_masked_gemm_rows(ts_layer_t* layer, int M, const void* At_dev, int64_t lda, void* C_dev, int64_t ldc,
+                        const ts_epilogue_t* epilogue, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Convolution as an implicit masked GEMM.  The reference prunes a conv kernel [kh][kw][cin][cout] as the
  * matrix [(kh*kw*cin)][cout] with row k = (r*kw + j)*cin + c (img2col_forward, Pruning/VGG/

@@ -103,6 +103,23 @@ int make_out_tmap(CUtensorMap* map, int dtype, const void* Ct, long long n_rows,
   return TS_OK;
 }
 
+// Tensor map over a row-major output C [M][ldc] (N columns): box 32 columns x 64 batch rows, no swizzle.
+int make_rows_tmap(CUtensorMap* map, int dtype, const void* C, long long N, long long M, long long ldc) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(TS_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
+  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldc) * 2};
+  cuuint32_t box[2] = {32, 64};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, dtype == TS_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                               : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                  2, const_cast<void*>(C), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(TS_ERR_CUDA, "cuTensorMapEncodeTiled (row-major output) failed (%d)", (int)r);
+  return TS_OK;
+}
+
 // Tensor map over the fp32 scratch [rows][M] of a split-K schedule: box 32 floats x 32 rows, 128-byte
 // swizzle (one chunk of an epilogue warp).
 int make_scratch_tmap(CUtensorMap* map, const float* scratch, long long rows, long long M) {
@@ -141,6 +158,7 @@ struct Schedule {
   struct OutMap {
     const void* ct = nullptr;
     long long ldc = 0;
+    bool rows = false;
     CUtensorMap map;
   };
   OutMap out_maps[4];
@@ -431,20 +449,30 @@ void build_schedule(const std::vector<ts::TileDesc>& tiles, long long at_rows, i
   const long long total = granules * static_cast<long long>(order.size());
   const long long units256_all = static_cast<long long>(order.size()) * ((M + 255) / 256);
   const bool contiguous = small_activations(at_rows, M) && units256_all <= 3LL * n_ctas;
+  std::vector<std::vector<Unit>> ulists;
   int cap;
   if (forced_unit_rows == 128 || forced_unit_rows == 256) {
     cap = forced_unit_rows / 64;
   } else if (contiguous) {
-    cap = (total + n_ctas - 1) / std::max(1, n_ctas) <= 2 ? 2 : 4;
+    cap = 4;
+    if ((total + n_ctas - 1) / std::max(1, n_ctas) <= 2 && !order.empty() && M > 0) {
+      // Two 64-row granules per SM on average: the 128-row variant has more stages for them, unless the
+      // partition leaves a CTA three, which it would run as two units one after the other (6 tiles of 49
+      // granules: 37 thousand cycles for those CTAs against 20 for the others).
+      partition_contiguous(tiles, order, M, 2, n_ctas, &ulists);
+      cap = 2;
+      for (const auto& l : ulists) {
+        if (l.size() > 1) cap = 4;
+      }
+    }
   } else {
     cap = 2 * units256_all >= n_ctas ? 4 : 2;
   }
   *unit_rows = cap * 64;
-  std::vector<std::vector<Unit>> ulists;
   if (order.empty() || M <= 0) {
     ulists.assign(1, {});
   } else if (contiguous) {
-    partition_contiguous(tiles, order, M, cap, n_ctas, &ulists);
+    if (ulists.empty() || cap != 2) partition_contiguous(tiles, order, M, cap, n_ctas, &ulists);
   } else {
     partition_blocked(tiles, order, at_rows, M, cap, n_ctas, &ulists);
   }
@@ -537,6 +565,7 @@ struct ts_layer {
   int* d_kept_k = nullptr;
   int* d_kept_n = nullptr;     // kept columns, then (from n_kept on) the columns no tile keeps
   int n_kept = 0, n_pruned = 0;
+  bool rows_ok = false;        // every tile keeps consecutive columns from a multiple of 8 on: C can leave row-major
   ts::TileDesc* d_tiles = nullptr;
   std::vector<ts::TileDesc> h_tiles;
   uint16_t* d_wp = nullptr;
@@ -873,6 +902,11 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
     if (dense && nc[t] < 128) dense = nn[np[t]] + nc[t] == l->N;
     td[t].pad_ = dense ? 1 : 0;
   }
+  // (all columns kept, too: a pruned one would have to be cleared column-wise)
+  l->rows_ok = n_tiles > 0 && l->N % 8 == 0 && l->n_pruned == 0;
+  for (int t = 0; t < n_tiles; ++t) {
+    if (nc[t] > 0 && (!td[t].pad_ || nn[np[t]] % 8 != 0)) l->rows_ok = false;
+  }
   if (n_tiles > 0) {
     TS_CUDA(cudaMemcpy(l->d_tiles, td.data(), td.size() * sizeof(ts::TileDesc), cudaMemcpyHostToDevice));
   }
@@ -957,10 +991,11 @@ int ts_layer_stats(const ts_layer_t* l, int64_t* kept_flops_per_row, int64_t* pa
 }  // extern "C"
 
 namespace {
-// The masked GEMM over a matrix At[K][lda] (conv_wp == 0) or over a convolution's input planes.
+// The masked GEMM over a matrix At[K][lda] (conv_wp == 0) or over a convolution's input planes; rows: Ct is a
+// row-major C[M][ldc] (the caller has checked row_output_ok).
 int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc,
-                    const ts_epilogue_t* epi, void* stream, int conv_wp) {
-  int rc = check_gemm_args(l, M, At, lda, Ct, ldc);
+                    const ts_epilogue_t* epi, void* stream, int conv_wp, bool rows = false) {
+  int rc = check_gemm_args(l, M, At, lda, Ct, rows ? std::max<int64_t>(ldc, (M + 7) / 8 * 8) : ldc);
   if (rc != TS_OK) return rc;
   if (!epi) return fail(TS_ERR_INVALID, "epilogue is NULL");
   if (epi->activation < TS_ACT_NONE || epi->activation > TS_ACT_GELU) {
@@ -987,7 +1022,7 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   Schedule* s = nullptr;
   // split-K units write fp32 partial sums to scratch memory of the schedule and a second kernel
   // finishes them; calls that also write peers (tile-sharded layers) keep whole units
-  const bool allow_split = l->split_k && ep.n_peers == 0 && ep.multicast == nullptr;
+  const bool allow_split = l->split_k && ep.n_peers == 0 && ep.multicast == nullptr && !rows;
   rc = get_schedule(l, M, lda, conv_wp, allow_split, &s);
   if (rc != TS_OK) return rc;
   if (s->n_units == 0) return TS_OK;
@@ -996,15 +1031,16 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   ep.scratch_map = s->d_scratch_map;
   const CUtensorMap* tmap_c = nullptr;
   for (const Schedule::OutMap& m : s->out_maps) {
-    if (m.ct == Ct && m.ldc == ldc) tmap_c = &m.map;
+    if (m.ct == Ct && m.ldc == ldc && m.rows == rows) tmap_c = &m.map;
   }
   if (!tmap_c) {
     Schedule::OutMap& m = s->out_maps[s->next_out_map];
     m.ct = nullptr;
-    rc = make_out_tmap(&m.map, l->dtype, Ct, l->N, M, ldc);
+    rc = rows ? make_rows_tmap(&m.map, l->dtype, Ct, l->N, M, ldc) : make_out_tmap(&m.map, l->dtype, Ct, l->N, M, ldc);
     if (rc != TS_OK) return rc;
     m.ct = Ct;
     m.ldc = ldc;
+    m.rows = rows;
     s->next_out_map = (s->next_out_map + 1) % 4;
     tmap_c = &m.map;
   }
@@ -1037,7 +1073,7 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   const bool early = !l->wp_fresh;
   TS_CUDA(ts::masked_gemm_launch(l->dtype, s->unit_rows, l->tmap, tmap_c, s->d_units, s->rounds,
                                  s->grid, s->d_meta, s->blk_stride, At, lda, Ct, ldc, M, ep, l->d_status,
-                                 early, s->all_dense, static_cast<cudaStream_t>(stream)));
+                                 early, s->all_dense, rows, static_cast<cudaStream_t>(stream)));
   l->wp_fresh = false;
   if (s->n_split > 0) {
     TS_CUDA(ts::split_reduce_launch(l->dtype, s->d_split, s->n_split, s->d_scratch, s->scratch_ld, Ct, ldc, M,
@@ -1063,6 +1099,31 @@ int ts_layer_zero_pruned(ts_layer_t* l, int M, void* Ct, int64_t ldc, void* stre
 int ts_masked_gemm_ex(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc,
                       const ts_epilogue_t* epi, void* stream) {
   return run_masked_gemm(l, M, At, lda, Ct, ldc, epi, stream, 0);
+}
+
+int ts_layer_row_output(ts_layer_t* l, int M, int* supported) {
+  if (!l || !supported) return fail(TS_ERR_INVALID, "NULL argument");
+  *supported = 0;
+  if (!l->rows_ok || M <= 0) return TS_OK;
+  if (l->split_k) {   // a layer whose long tiles pay for split-K keeps it, and the K-major output with it
+    std::vector<int> parts;
+    plan_split(l->k_counts, l->n_counts, l->K, M, l->sm_count, &parts);
+    for (int p : parts) {
+      if (p > 1) return TS_OK;
+    }
+  }
+  *supported = 1;
+  return TS_OK;
+}
+
+int ts_masked_gemm_rows(ts_layer_t* l, int M, const void* At, int64_t lda, void* C, int64_t ldc, const ts_epilogue_t* epi, void* stream) {
+  if (!l || !epi) return fail(TS_ERR_INVALID, "NULL argument");
+  if (!l->rows_ok) return fail(TS_ERR_UNSUPPORTED, "the layer's tiles do not allow a row-major output (ts_layer_row_output)");
+  if (epi->beta != 0.0f || epi->n_peers != 0 || epi->multicast_ct) {
+    return fail(TS_ERR_UNSUPPORTED, "a row-major output takes neither beta nor peers");
+  }
+  if (ldc < l->N || (ldc % 8) != 0) return fail(TS_ERR_INVALID, "ldc=%lld must be a multiple of 8 and >= N=%d", (long long)ldc, l->N);
+  return run_masked_gemm(l, M, At, lda, C, ldc, epi, stream, 0, true);
 }
 
 int ts_layer_set_conv(ts_layer_t* l, int cin, int kh, int kw) {
@@ -1431,7 +1492,7 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
   ep.beta = beta;
   TS_CUDA(ts::masked_gemm_launch(dtype, unit_rows, tmap, nullptr, ws.d_units, rounds, grid,
                                  ws.d_meta, blk_stride, A, M, C, M, M, ep, ws.d_status, /*early_start=*/false,
-                                 /*lean=*/false, s));
+                                 /*lean=*/false, /*rows=*/false, s));
   return TS_OK;
 }
 

@@ -54,11 +54,15 @@ constexpr uint32_t kASbo = 1024;         // bytes between 8-row K groups of the 
 constexpr uint32_t kALbo = kKB * 128;    // bytes between its 64-column batch groups
 constexpr uint32_t kWSbo = 1024;         // bytes between 8-row groups of the weight operand
 constexpr int kMaxStages = 6;
-// Gather warps.  Four keep the L2-to-SM path full: 470 cycles per 32 KiB block on B200 with every SM
-// copying, the same with 8 and 16 warps; all four fill every block together, 16 rows each, which is
-// one K step of the MMA.
-constexpr int kGW = 4;
-constexpr int kRowsPerWarp = kKB / kGW;
+// Gather warps: two groups of four that take turns on the K blocks; the warps of a group fill a block
+// together, 16 rows each, which is one K step of the MMA.  The copies alone need only four warps to keep the
+// L2-to-SM path full (470 cycles per 32 KiB on B200 with every SM copying, the same with 8 and 16), but a warp
+// spends 600 cycles on a block whatever its width (record, stage wait, burst, hand-over): narrow units and
+// short chains are bound by that (encoder layer at 32 rows 16.2 -> 15.6 us with the second group).
+constexpr int kWarpsPerBlock = 4;
+constexpr int kWarpGroups = 2;
+constexpr int kGW = kWarpGroups * kWarpsPerBlock;
+constexpr int kRowsPerWarp = kKB / kWarpsPerBlock;
 constexpr int kGatherWarp0 = 2;          // warps 0 and 1: weights, MMA
 constexpr int kEpiWarp0 = kGatherWarp0 + kGW;       // first epilogue warp
 constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
@@ -192,9 +196,10 @@ __device__ __forceinline__ float apply_act(float x, int act) {
 // MODE selects what the epilogue can do: kModeLean act(alpha * acc + bias) through TMA tile stores only (the
 // host picks it when beta == 0 and every scheduled tile keeps 128 consecutive columns), kModePlain every
 // epilogue form and the list-driven stores, kModeSplit in addition the fp32 partial sums of split-K parts,
-// kModePeers the copies for the other GPUs of a tile-sharded layer.  Code a call cannot reach stays out of
+// kModePeers the copies for the other GPUs of a tile-sharded layer; kModeRows is kModeLean with a row-major
+// output (batch row m of C contiguous over the columns of W).  Code a call cannot reach stays out of
 // the variant it runs: the hot loops share one instruction cache.
-constexpr int kModePlain = 0, kModeSplit = 1, kModePeers = 2, kModeLean = 3;
+constexpr int kModePlain = 0, kModeSplit = 1, kModePeers = 2, kModeLean = 3, kModeRows = 4;
 template <int DT, int MT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
@@ -206,7 +211,8 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                    int* __restrict__ status) {
   const float alpha = ep.alpha, beta = ep.beta;
   const int act = ep.act;
-  constexpr bool SPLIT = MODE == kModeSplit, PEERS = MODE == kModePeers, LEAN = MODE == kModeLean;
+  constexpr bool SPLIT = MODE == kModeSplit, PEERS = MODE == kModePeers, ROWS = MODE == kModeRows;
+  constexpr bool LEAN = MODE == kModeLean || ROWS;
   using C = Cfg<MT>;
   constexpr int kStages = C::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -235,7 +241,7 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   if (warp == 0 && elect_one()) {
     for (int s = 0; s < kStages; ++s) {
       // weight TMA thread + the cp.async lanes of the gather warps
-      mbar_init(smem_u32(&bars->full[s]), 1 + 32 * kGW);
+      mbar_init(smem_u32(&bars->full[s]), 1 + 32 * kWarpsPerBlock);
       mbar_init(smem_u32(&bars->empty[s]), 1);       // one tcgen05.commit
     }
     for (int s = 0; s < C::kRecs; ++s) mbar_init(smem_u32(&bars->rec_full[s]), 1);
@@ -356,15 +362,16 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
     }
   } else if (warp < kEpiWarp0) {
     // ------------------------------------------------------------------ activation gather
-    // The four warps fill every block together, 16 rows each (one K step of the MMA).  Per block: wait for
+    // Group p of warps takes the blocks p, p + kWarpGroups, ... (16 rows a warp).  Per block: wait for
     // the stage, issue the warp's rows in one burst of 16-byte copies, hand them to the stage's barrier.
-    // The row numbers of the next block go from the record ring to registers before that wait, so neither
+    // The row numbers of the group's next block go from the record ring to registers before that wait, so neither
     // the record nor a shared-memory read sits between a free stage and its copies (a read between two
     // copies would also stall the warp until the load/store unit has taken the copies before it).
     constexpr int kLpr = C::kLanesPerRow, kRpi = C::kRowsPerInstr;
     const int chunk = lane % kLpr, sub = lane / kLpr;
     const int g = chunk >> 3, c = chunk & 7;
-    const int row_base = (warp - kGatherWarp0) * kRowsPerWarp;         // first row of the warp's slice
+    const uint32_t group = (warp - kGatherWarp0) / kWarpsPerBlock;
+    const int row_base = ((warp - kGatherWarp0) % kWarpsPerBlock) * kRowsPerWarp;         // first row of the warp's slice
     int rr[kRowsPerWarp], rn[kRowsPerWarp];
     int m0 = 0, m0_next;
     uint32_t meta = kBlockEnd, meta_next;
@@ -385,13 +392,13 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       }
       return true;
     };
-    bool ok = read_record(0, m0, meta, rr);
+    bool ok = read_record(group, m0, meta, rr);
     // The schedule is static; the activations may be the previous kernel's output: wait for it
     // before the first row is copied.
     grid_dependency_wait();
 
-    for (uint32_t j = 0; ok && meta != kBlockEnd; ++j) {
-      if (!read_record(j + 1, m0_next, meta_next, rn)) break;
+    for (uint32_t j = group; ok && meta != kBlockEnd; j += kWarpGroups) {
+      if (!read_record(j + kWarpGroups, m0_next, meta_next, rn)) break;
       const int nv = static_cast<int>(meta & 0x7fu) - row_base;                 // valid rows of the slice
       const int m_len = (static_cast<int>((meta >> 8) & 3u) + 1) * 64;          // batch rows of the unit
       const int m = m0 + chunk * 8;
@@ -563,8 +570,21 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll
                 for (int e = 0; e < 4; ++e) gelu2(y[e * 2], y[e * 2 + 1]);
               }
-              *reinterpret_cast<uint4*>(row_ptr + (((b * 4 + p) ^ (lane & 7)) << 4)) =
-                  make_uint4(pack2<DT>(y[0], y[1]), pack2<DT>(y[2], y[3]), pack2<DT>(y[4], y[5]), pack2<DT>(y[6], y[7]));
+              if constexpr (ROWS) {
+                // row-major: two neighbouring lanes (columns n, n + 1) swap halves, so that each holds one
+                // batch row of the column pair; staged as [64 batch rows][32 columns], a store instruction
+                // covers two rows of 64 bytes
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const uint32_t own = pack2<DT>(y[e * 2], y[e * 2 + 1]);
+                  const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+                  const uint32_t pair = (lane & 1) ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+                  *reinterpret_cast<uint32_t*>(stage + (b * 32 + p * 8 + e * 2 + (lane & 1)) * 64 + (lane >> 1) * 4) = pair;
+                }
+              } else {
+                *reinterpret_cast<uint4*>(row_ptr + (((b * 4 + p) ^ (lane & 7)) << 4)) =
+                    make_uint4(pack2<DT>(y[0], y[1]), pack2<DT>(y[2], y[3]), pack2<DT>(y[4], y[5]), pack2<DT>(y[6], y[7]));
+              }
             }
           };
           if (act == kActNone) convert(std::integral_constant<int, kActNone>{});
@@ -576,8 +596,9 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
         if (tma_store) {
           fence_proxy_async_smem();
           __syncwarp();                          // the whole group is staged
-          if (lane == 0) {
-            tma_store_2d(&tmap_c, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
+          if (lane == 0 && q * 32 < w.n_count) {
+            if constexpr (ROWS) tma_store_2d(&tmap_c, smem_u32(stage), tile_row0 + q * 32, m0 + col0);
+            else tma_store_2d(&tmap_c, smem_u32(stage), m0 + col0, tile_row0 + q * 32);
             if constexpr (PEERS) if (tma_peers) {
               for (int p = 0; p < ep.n_peers; ++p) {
                 int pp = p + peer_rot;
@@ -759,13 +780,17 @@ cudaError_t launch_variant(const CUtensorMap& tmap_w, const CUtensorMap& tmap_c,
 cudaError_t masked_gemm_launch(int dtype, int unit_rows, const CUtensorMap& tmap_w, const CUtensorMap* tmap_c,
                                const WorkItem* sched, int rounds, int grid, const int* block_meta,
                                int blk_stride, const void* At, long long lda, void* Ct, long long ldc, int M,
-                               const EpilogueArgs& ep, int* status, bool early_start, bool lean,
+                               const EpilogueArgs& ep, int* status, bool early_start, bool lean, bool rows,
                                cudaStream_t stream) {
 #define TS_LAUNCH(DT, MT, MD)                                                                                  \
   launch_variant<DT, MT, MD>(tmap_w, tmap_c ? *tmap_c : tmap_w, tmap_c ? 1 : 0, sched, rounds, grid, block_meta, \
                              blk_stride, At, lda, Ct, ldc, M, ep, status, early_start, stream)
 #define TS_LAUNCH_DT(MT, MD) (dtype == kBF16 ? TS_LAUNCH(kBF16, MT, MD) : TS_LAUNCH(kF16, MT, MD))
   if (unit_rows != 256 && unit_rows != 128) return cudaErrorInvalidValue;
+  if (rows) {
+    if (!lean || tmap_c == nullptr || ep.beta != 0.0f || ep.scratch_map || ep.n_peers > 0 || ep.multicast) return cudaErrorInvalidValue;
+    return unit_rows == 256 ? TS_LAUNCH_DT(256, kModeRows) : TS_LAUNCH_DT(128, kModeRows);
+  }
   // a schedule with split-K parts never writes peers (the host keeps the two apart)
   if (ep.scratch_map != nullptr) return unit_rows == 256 ? TS_LAUNCH_DT(256, kModeSplit) : TS_LAUNCH_DT(128, kModeSplit);
   if (ep.n_peers > 0 || ep.multicast != nullptr) {

@@ -82,6 +82,51 @@ transpose16_kernel(const uint16_t* __restrict__ in, long long ld_in, uint16_t* _
   }
 }
 
+// The same for matrices whose pointers, row pitches and sizes allow 16-byte accesses on both sides.  A block
+// moves 128 x 128 elements: a thread loads an 8 x 8 block (eight 16-byte pieces, 256 contiguous bytes of a
+// row per 16 lanes), transposes it in registers by byte permutes, and the block's 16-byte pieces change
+// lanes through shared memory, so that the stores are runs of 256 bytes too; the pieces of a row are
+// swizzled by its number, which keeps both sides free of bank conflicts.  Bound by the memory system:
+// 3080 x 3072 (38 MB moved, most of it in L2) 5.4 us, against 15 us for the two-byte form above.
+__global__ void __launch_bounds__(256)
+transpose16_vec_kernel(const uint16_t* __restrict__ in, long long ld_in, uint16_t* __restrict__ out,
+                       long long ld_out, int rows, int cols) {
+  __shared__ uint4 t[128 * 16];            // [column][row / 8], 16-byte pieces
+  const int r0 = blockIdx.y * 128, c0 = blockIdx.x * 128;
+  const int c8 = threadIdx.x & 15, r8 = threadIdx.x >> 4;
+  const int c = c0 + c8 * 8, r = r0 + r8 * 8;
+  uint4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    v[i] = (c < cols && r + i < rows) ? __ldg(reinterpret_cast<const uint4*>(in + static_cast<long long>(r + i) * ld_in + c))
+                                      : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {             // columns 2q, 2q + 1: word q of every row
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 a = v[2 * i], b = v[2 * i + 1];
+      const uint32_t wa = q == 0 ? a.x : (q == 1 ? a.y : (q == 2 ? a.z : a.w));
+      const uint32_t wb = q == 0 ? b.x : (q == 1 ? b.y : (q == 2 ? b.z : b.w));
+      lo[i] = __byte_perm(wa, wb, 0x5410);
+      hi[i] = __byte_perm(wa, wb, 0x7632);
+    }
+    t[(c8 * 8 + 2 * q) * 16 + (r8 ^ c8)] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    t[(c8 * 8 + 2 * q + 1) * 16 + (r8 ^ c8)] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  }
+  __syncthreads();
+  const int p = threadIdx.x & 15;           // rows 8p .. of a column
+  const bool r_ok = r0 + p * 8 < rows;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int cc = i * 16 + (threadIdx.x >> 4);
+    if (r_ok && c0 + cc < cols) {
+      *reinterpret_cast<uint4*>(out + static_cast<long long>(c0 + cc) * ld_out + r0 + p * 8) = t[cc * 16 + (p ^ (cc >> 3))];
+    }
+  }
+}
+
 // Ct[rows[blockIdx.y]][0 .. M) = 0, eight elements per thread.
 __global__ void __launch_bounds__(256)
 zero_rows_kernel(const int* __restrict__ rows, uint16_t* __restrict__ Ct, long long ldc, int M) {
@@ -124,6 +169,13 @@ cudaError_t pack_weights_launch(int w_dtype, int out_dtype, const void* W, long 
 cudaError_t transpose16_launch(const void* in, long long ld_in, void* out, long long ld_out,
                                int rows, int cols, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return cudaSuccess;
+  const bool vec = ((rows | cols | ld_in | ld_out) & 7) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+  if (vec && (rows + 127) / 128 <= 65535) {
+    transpose16_vec_kernel<<<dim3((cols + 127) / 128, (rows + 127) / 128), 256, 0, stream>>>(
+        static_cast<const uint16_t*>(in), ld_in, static_cast<uint16_t*>(out), ld_out, rows, cols);
+    return cudaGetLastError();
+  }
   dim3 grid((cols + 63) / 64, (rows + 63) / 64);
   transpose16_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(in), ld_in,
                                                static_cast<uint16_t*>(out), ld_out, rows, cols);

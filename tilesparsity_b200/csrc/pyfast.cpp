@@ -130,6 +130,68 @@ PyObject* py_masked_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return a[2];
 }
 
+// The transpose of a 16-bit matrix with contiguous rows, or TS_* / a ValueError already set (*out undefined).
+bool transpose(const at::Tensor& x, void* stream, at::Tensor* out) {
+  if (x.dim() != 2 || x.element_size() != 2 || x.stride(1) != 1 || !x.is_cuda()) {
+    fail_value("transpose16 takes a 2-D 16-bit CUDA tensor with contiguous rows");
+    return false;
+  }
+  *out = new_tensor({x.size(1), x.size(0)}, x.scalar_type(), x.get_device());
+  const int rc = ts_transpose16(x.data_ptr(), x.stride(0), out->data_ptr(), out->stride(0), static_cast<int>(x.size(0)),
+                                static_cast<int>(x.size(1)), stream);
+  if (rc != TS_OK) fail_code(rc);
+  return rc == TS_OK;
+}
+
+// transpose16(x) -> its transpose
+PyObject* py_transpose16(PyObject*, PyObject* arg) {
+  if (!THPVariable_Check(arg)) return fail_value("transpose16 takes a tensor");
+  const at::Tensor& x = THPVariable_Unpack(arg);
+  if (!x.is_cuda()) return fail_value("transpose16 takes a 2-D 16-bit CUDA tensor with contiguous rows");
+  c10::cuda::OptionalCUDAGuard guard(x.device());
+  at::Tensor out;
+  if (!transpose(x, stream_of(x.get_device()), &out)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// linear(layer, A [M, K], transpose_out) -> C [M, N], or Ct [N, M]
+PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 3) return fail_value("linear takes 3 arguments");
+  if (a[0] == Py_None) return fail_code(ts_masked_gemm_ex(nullptr, 0, nullptr, 0, nullptr, 0, nullptr, nullptr));   // a closed layer
+  Layer* l = layer_of(a[0]);
+  if (!l) return nullptr;
+  if (!THPVariable_Check(a[1])) return fail_value("A must be a tensor");
+  const at::Tensor& A = THPVariable_Unpack(a[1]);
+  if (A.dim() != 2 || A.size(1) != l->K || A.scalar_type() != l->dtype || !on_device(A, l->device)) {
+    return fail_value("A must be an [M, K] tensor of the layer's dtype on the layer's device");
+  }
+  const int64_t M = A.size(0);
+  c10::cuda::OptionalCUDAGuard guard(A.device());
+  void* stream = stream_of(l->device);
+  at::Tensor At, out;
+  if (!transpose(A, stream, &At)) return nullptr;
+  ts_epilogue_t ep = {};
+  ep.alpha = 1.0f;
+  int rows = 0, rc = TS_OK;
+  if (a[2] == Py_True) rc = ts_layer_row_output(l->h, static_cast<int>(M), &rows);
+  if (rc != TS_OK) return fail_code(rc);
+  if (rows) {
+    out = new_tensor({M, l->N}, l->dtype, l->device);
+    rc = ts_masked_gemm_rows(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out.data_ptr(), l->N, &ep, stream);
+    if (rc != TS_OK) return fail_code(rc);
+    return THPVariable_Wrap(std::move(out));
+  }
+  rc = new_output(*l, M, false, stream, &out);
+  if (rc == TS_OK) rc = ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out.data_ptr(), M, &ep, stream);
+  if (rc != TS_OK) return fail_code(rc);
+  if (a[2] == Py_True) {
+    at::Tensor C;
+    if (!transpose(out, stream, &C)) return nullptr;
+    return THPVariable_Wrap(std::move(C));
+  }
+  return THPVariable_Wrap(std::move(out));
+}
+
 PyObject* py_bind(PyObject*, PyObject* type) {
   Py_XDECREF(g_error_type);
   Py_INCREF(type);
@@ -141,6 +203,8 @@ PyMethodDef kMethods[] = {
     {"bind", py_bind, METH_O, "Sets the exception type raised for C-ABI errors."},
     {"layer_desc", py_layer_desc, METH_VARARGS, "Capsule describing a layer to the functions below."},
     {"masked_gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_masked_gemm)), METH_FASTCALL, "TWLayer.masked_gemm"},
+    {"transpose16", py_transpose16, METH_O, "layer.transpose16"},
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_linear)), METH_FASTCALL, "layer.masked_linear"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_tsfast", "Host path of the per-batch operators.", -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -18,7 +18,7 @@ from . import _lib
 from ._lib import check, lib
 from .tiles import TileSet, tiles_from_lists, tiles_from_mask
 
-_masked_gemm = _lib.fast().masked_gemm
+_masked_gemm, _linear = _lib.fast().masked_gemm, _lib.fast().linear
 
 _TS_DTYPE = {torch.float16: _lib.TS_DTYPE_F16, torch.bfloat16: _lib.TS_DTYPE_BF16,
              torch.float32: _lib.TS_DTYPE_F32}
@@ -342,24 +342,17 @@ class TEWLayer:
 
 def transpose16(x: torch.Tensor) -> torch.Tensor:
     """[R, C] 16-bit tensor -> its transpose [C, R], materialised by the library's kernel."""
-    if x.dim() != 2 or x.element_size() != 2 or x.stride(1) != 1 or not x.is_cuda:
-        raise ValueError("transpose16 takes a 2-D 16-bit CUDA tensor with contiguous rows")
-    R, Cc = x.shape
-    out = torch.empty((Cc, R), dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib.ts_transpose16(C.c_void_p(x.data_ptr()), x.stride(0), C.c_void_p(out.data_ptr()), out.stride(0),
-                                 R, Cc, _stream_ptr(x.device)))
-    return out
+    return _lib.fast().transpose16(x)
 
 
 def masked_linear(A: torch.Tensor, layer: TWLayer, transpose_out: bool = True) -> torch.Tensor:
     """`A @ (W * mask)` for row-major activations A[M, K]  (mask_dense, modeling.py:992-1007, minus bias).
 
     A is transposed to the K-major layout on the device first (an extra pass the K-major entry point
-    `TWLayer.masked_gemm` does not pay).  Returns C[M, N], or Ct[N, M] with transpose_out=False.
+    `TWLayer.masked_gemm` does not pay); where the tiles allow it the GEMM writes C row-major itself, else
+    its output is transposed back.  Returns C[M, N], or Ct[N, M] with transpose_out=False.
     """
-    Ct = layer.masked_gemm(transpose16(A))
-    return transpose16(Ct) if transpose_out else Ct
+    return _linear(layer._desc, A, bool(transpose_out))
 
 
 def masked_matmul(A: torch.Tensor, W: torch.Tensor, kept_k_lists, col_mask=None, G: int = 128) -> torch.Tensor:

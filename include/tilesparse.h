@@ -277,8 +277,8 @@ int ts_residual_gemm(int dtype, int M, int N, const int32_t* col_ptr_dev, const 
  * compacted tiles column-major with ldb = K, tile t at B + off_B[t]; C is Ct [N][M], tile t at
  * C + off_C[t]; mask_k[t] / mask_n[t] are DEVICE pointers to K_cal[t] / N_cal[t] relative
  * offsets; N_cal, K_cal, off_B, off_C are HOST arrays of block_num entries (block_num <= 32,
- * N_cal[t] <= 128).  All tiles run in one launch on `stream`.  The call uploads a small tile table
- * (synchronous copy into a cached workspace), then enqueues the kernel. */
+ * N_cal[t] <= 128).  All tiles run in one launch on `stream`.  The first call of a shape (sizes,
+ * kept counts, offsets) uploads a small tile table; every call resolves the offset lists on the device. */
 int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const void* B, float beta,
                       void* C, int block_num, const int* N_cal, const int* K_cal,
                       int* const* mask_n, int* const* mask_k, const int* off_B, const int* off_C,

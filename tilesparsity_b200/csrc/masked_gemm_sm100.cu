@@ -200,10 +200,11 @@ __device__ __forceinline__ float apply_act(float x, int act) {
 // output (batch row m of C contiguous over the columns of W).  Code a call cannot reach stays out of
 // the variant it runs: the hot loops share one instruction cache.
 constexpr int kModePlain = 0, kModeSplit = 1, kModePeers = 2, kModeLean = 3, kModeRows = 4;
+constexpr int kFlagTmaStore = 1, kFlagWaitFirst = 2;
 template <int DT, int MT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
 masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
-                   const __grid_constant__ CUtensorMap tmap_c, int use_tma_store,
+                   const __grid_constant__ CUtensorMap tmap_c, int flags,
                    const WorkItem* __restrict__ sched, int rounds,
                    const int* __restrict__ block_meta, int blk_stride,
                    const uint16_t* __restrict__ At, long long lda,
@@ -211,6 +212,9 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
                    int* __restrict__ status) {
   const float alpha = ep.alpha, beta = ep.beta;
   const int act = ep.act;
+  const bool use_tma_store = (flags & kFlagTmaStore) != 0;
+  // the schedule, the records or the weights come from the kernel before this one
+  if (flags & kFlagWaitFirst) grid_dependency_wait();
   constexpr bool SPLIT = MODE == kModeSplit, PEERS = MODE == kModePeers, ROWS = MODE == kModeRows;
   constexpr bool LEAN = MODE == kModeLean || ROWS;
   using C = Cfg<MT>;
@@ -676,16 +680,13 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
 // is channel c of the copy of the padded input shifted by j pixels, read r image rows further down:
 // segment ((j * cin + c) * plane_ld + r * Wp) / 8.  The kept row number itself comes from the tile's
 // list, or list position + offset for lists in the reference's relative form.
-__global__ void __launch_bounds__(256)
-expand_block_meta_kernel(const BlockDesc* __restrict__ blocks, long long n_blocks, int* __restrict__ meta,
-                         const RowMap map) {
-  const long long b = blockIdx.x * 4LL + (threadIdx.x >> 6);
-  const int r = threadIdx.x & 63;
-  if (b >= n_blocks) return;
-  const BlockDesc d = blocks[b];
+// Lists that the caller hands over per call (reference-signature entry point): `lists` carries their
+// addresses, the descriptors hold the tile's number and the byte offset inside its list instead of an address
+// (see stream_list_code), and the work items get their column lists here.
+__device__ __forceinline__ void expand_record(const BlockDesc& d, const int* idx, int r, int* rec, const RowMap& map) {
   int v = 0;
   if (d.meta != kBlockEnd && r < static_cast<int>(d.meta & 0x7fu)) {
-    v = __ldg(d.idx + r);
+    v = __ldg(idx + r);
     if (d.meta & 0x80u) v += static_cast<int>(d.meta >> 10) + r;
     if (map.conv_cin > 0) {
       const int c = v % map.conv_cin, rj = v / map.conv_cin;
@@ -695,9 +696,34 @@ expand_block_meta_kernel(const BlockDesc* __restrict__ blocks, long long n_block
       v = static_cast<int>(static_cast<long long>(v) * map.ld8);
     }
   }
-  int* rec = meta + b * kMetaInts;
   rec[4 + r] = v;
   if (r < 4) rec[r] = r == 0 ? d.m0 : (r == 1 ? static_cast<int>(d.meta) : 0);
+}
+
+__global__ void __launch_bounds__(256)
+expand_block_meta_kernel(const BlockDesc* __restrict__ blocks, long long n_blocks, int* __restrict__ meta,
+                         const RowMap map) {
+  const long long b = blockIdx.x * 4LL + (threadIdx.x >> 6);
+  if (b >= n_blocks) return;
+  const BlockDesc d = blocks[b];
+  expand_record(d, d.idx, threadIdx.x & 63, meta + b * kMetaInts, map);
+}
+
+__global__ void __launch_bounds__(256)
+expand_stream_kernel(const BlockDesc* __restrict__ blocks, int n_blocks, int* __restrict__ meta, WorkItem* __restrict__ items,
+                     int n_items, const RowMap map, const __grid_constant__ StreamLists lists) {
+  grid_launch_dependents();
+  // the GEMM before this kernel may still be reading the records and items of the call before
+  grid_dependency_wait();
+  const int b = blockIdx.x * 4 + (threadIdx.x >> 6);
+  if (b < n_blocks) {
+    const BlockDesc d = blocks[b];
+    const unsigned long long code = reinterpret_cast<unsigned long long>(d.idx);
+    const int* idx = d.meta == kBlockEnd ? nullptr : lists.k[code >> kStreamTileShift] + (code & ((1ull << kStreamTileShift) - 1)) / 4;
+    expand_record(d, idx, threadIdx.x & 63, meta + static_cast<long long>(b) * kMetaInts, map);
+  }
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n_items && items[i].tile >= 0) items[i].n_list = lists.n[items[i].tile];
 }
 
 // Second pass of a split-K schedule: Ct[row][m] = act(sum of the parts' fp32 partial sums + beta * Ct[row][m]
@@ -741,14 +767,12 @@ split_reduce_kernel(const SplitTile* __restrict__ tiles, const float* __restrict
 }
 
 template <int DT, int MT, int MODE>
-cudaError_t launch_variant(const CUtensorMap& tmap_w, const CUtensorMap& tmap_c, int use_tma_store,
+cudaError_t launch_variant(const CUtensorMap& tmap_w, const CUtensorMap& tmap_c, int flags,
                            const WorkItem* sched, int rounds, int grid, const int* block_meta, int blk_stride,
                            const void* At, long long lda, void* Ct, long long ldc, int M,
-                           const EpilogueArgs& ep, int* status, bool early_start, cudaStream_t stream) {
-  // Programmatic dependent launch lets this kernel's set-up overlap the tail of the kernel before
-  // it in the stream.  The kernel reads its schedule and its packed weights before it waits for that
-  // kernel, so the caller allows this only when neither was written by it.
-  const bool pdl = early_start;
+                           const EpilogueArgs& ep, int* status, cudaStream_t stream) {
+  // Programmatic dependent launch lets this kernel's set-up overlap the tail of the kernel before it in
+  // the stream; what it may read before that kernel has completed is the caller's choice (kFlagWaitFirst).
   auto kern = masked_gemm_kernel<DT, MT, MODE>;
   // The dynamic shared-memory limit is a per-device, per-kernel attribute: set it once for each.
   static bool attr_set[64] = {};
@@ -769,8 +793,8 @@ cudaError_t launch_variant(const CUtensorMap& tmap_w, const CUtensorMap& tmap_c,
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_c, use_tma_store, sched, rounds, block_meta, blk_stride,
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_c, flags, sched, rounds, block_meta, blk_stride,
                             static_cast<const uint16_t*>(At), lda, static_cast<uint16_t*>(Ct), ldc, M,
                             ep, status);
 }
@@ -783,9 +807,10 @@ cudaError_t masked_gemm_launch(int dtype, int unit_rows, const CUtensorMap& tmap
                                const EpilogueArgs& ep, int* status, bool early_start, bool lean, bool rows,
                                cudaStream_t stream) {
 #define TS_LAUNCH(DT, MT, MD)                                                                                  \
-  launch_variant<DT, MT, MD>(tmap_w, tmap_c ? *tmap_c : tmap_w, tmap_c ? 1 : 0, sched, rounds, grid, block_meta, \
-                             blk_stride, At, lda, Ct, ldc, M, ep, status, early_start, stream)
+  launch_variant<DT, MT, MD>(tmap_w, tmap_c ? *tmap_c : tmap_w, flags, sched, rounds, grid, block_meta, \
+                             blk_stride, At, lda, Ct, ldc, M, ep, status, stream)
 #define TS_LAUNCH_DT(MT, MD) (dtype == kBF16 ? TS_LAUNCH(kBF16, MT, MD) : TS_LAUNCH(kF16, MT, MD))
+  const int flags = (tmap_c ? kFlagTmaStore : 0) | (early_start ? 0 : kFlagWaitFirst);
   if (unit_rows != 256 && unit_rows != 128) return cudaErrorInvalidValue;
   if (rows) {
     if (!lean || tmap_c == nullptr || ep.beta != 0.0f || ep.scratch_map || ep.n_peers > 0 || ep.multicast) return cudaErrorInvalidValue;
@@ -824,6 +849,22 @@ cudaError_t expand_block_meta_launch(const BlockDesc* blocks, long long n_blocks
   if (n_blocks <= 0) return cudaSuccess;
   expand_block_meta_kernel<<<static_cast<unsigned>((n_blocks + 3) / 4), 256, 0, stream>>>(blocks, n_blocks, meta, map);
   return cudaGetLastError();
+}
+
+cudaError_t expand_stream_launch(const BlockDesc* blocks, int n_blocks, int* meta, WorkItem* items, int n_items,
+                                 const RowMap& map, const StreamLists& lists, cudaStream_t stream) {
+  const int n = (n_blocks + 3) / 4 > (n_items + 255) / 256 ? (n_blocks + 3) / 4 : (n_items + 255) / 256;
+  if (n <= 0) return cudaSuccess;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(n));
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, expand_stream_kernel, blocks, n_blocks, meta, items, n_items, map, lists);
 }
 
 }  // namespace ts

@@ -121,6 +121,16 @@ struct alignas(16) BlockDesc {
 };
 static_assert(sizeof(BlockDesc) == 16, "BlockDesc is copied as one 16-byte word");
 constexpr uint32_t kBlockEnd = 0xFFFFFFFFu;
+// Index lists of one reference-signature call (at most 32 tiles), and what stands for a list's address in the
+// cached schedule of such a call: tile number above bit 40, byte offset below.
+struct StreamLists {
+  const int* k[32];
+  const int* n[32];
+};
+constexpr int kStreamTileShift = 40;
+inline const int* stream_list_code(int tile) {
+  return reinterpret_cast<const int*>(static_cast<unsigned long long>(tile) << kStreamTileShift);
+}
 // The gather warps read a block as one resolved record of kBlockMetaInts ints: {m0, meta, 0, 0}
 // followed by where each of the block's 64 kept rows starts, in 16-byte segments from the base pointer.
 constexpr int kBlockMetaInts = 4 + 64;

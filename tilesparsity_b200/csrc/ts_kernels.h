@@ -18,8 +18,8 @@ namespace ts {
 // to blk_stride records) by end markers; expand_block_meta_launch writes it from the descriptors.
 // tmap_c != nullptr enables TMA stores (tensor map over Ct [N][ldc], box 64 x 128, 128-byte swizzle)
 // for the work items whose flags say their kept columns are consecutive rows of Ct.  early_start
-// allows programmatic dependent launch: the kernel reads sched, block_meta and the packed weights before
-// it waits for the kernel before it in the stream, so it must be false when that kernel wrote them.
+// lets the kernel read sched, block_meta and the packed weights before it waits for the kernel before it
+// in the stream (programmatic dependent launch), so it must be false when that kernel wrote them.
 // lean: every unit of the schedule has kItemDenseRows set (the kernel then takes its store-only variant
 // when beta is 0).  rows: tmap_c is a map over a row-major output C[M][N] (box 32 columns x 64 rows, no
 // swizzle) and every tile's first column is a multiple of 8; needs lean and beta == 0.
@@ -40,6 +40,11 @@ cudaError_t split_reduce_launch(int dtype, const SplitTile* tiles, int n_split, 
 // of the activations starts (`map`: a matrix with its row pitch, or a convolution's input planes).
 cudaError_t expand_block_meta_launch(const BlockDesc* blocks, long long n_blocks, int* meta, const RowMap& map,
                                      cudaStream_t stream);
+
+// The same for the reference-signature entry point, whose index lists arrive with the call: descriptors hold
+// stream_list_code(tile, position) in place of an address, and the work items' column lists are filled in.
+cudaError_t expand_stream_launch(const BlockDesc* blocks, int n_blocks, int* meta, WorkItem* items, int n_items,
+                                 const RowMap& map, const StreamLists& lists, cudaStream_t stream);
 
 // CUDA-core twin of the masked GEMM with the same operands (masked_gemm_simt.cu).
 cudaError_t masked_gemm_simt_launch(int dtype, const TileDesc* tiles, int n_tiles, const void* Wp,

@@ -75,13 +75,18 @@ def _build_library(force: bool, verbose: bool) -> None:
     os.replace(LIB_PATH + ".tmp", LIB_PATH)
 
 
+def numpy_include() -> str:
+    import numpy
+    return numpy.get_include()
+
+
 def _build_extension() -> None:
     root = os.path.dirname(importlib.util.find_spec("torch").origin)
     inc, lib = os.path.join(root, "include"), os.path.join(root, "lib")
     cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
     _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
           "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + cuda,
-          "-I" + sysconfig.get_paths()["include"], "-o", EXT_PATH + ".tmp", os.path.join(CSRC, "pyfast.cpp"),
+          "-I" + sysconfig.get_paths()["include"], "-I" + numpy_include(), "-o", EXT_PATH + ".tmp", os.path.join(CSRC, "pyfast.cpp"),
           "-L" + HERE, "-l:libtilesparse.so", "-Wl,-rpath,$ORIGIN", "-L" + lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
           "-lc10_cuda", "-lc10"])
     os.replace(EXT_PATH + ".tmp", EXT_PATH)

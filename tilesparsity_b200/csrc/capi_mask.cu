@@ -233,23 +233,6 @@ double percentile_lerp(float a, float b, const Ranks& r, bool wide) {
   return static_cast<double>(res);
 }
 
-// A tile ends right after its G-th kept column; no cut at the matrix edge (prune_algo.py:72-89).
-std::vector<int> regroup_bounds(const uint8_t* colkeep, int N, int G) {
-  std::vector<int> b{0};
-  int count = 0;
-  for (int c = 0; c < N; ++c) {
-    if (colkeep[c]) ++count;
-    if (count == G) {
-      if (c + 1 < N) {
-        b.push_back(c + 1);
-        count = 0;
-      }
-    }
-  }
-  b.push_back(N);
-  return b;
-}
-
 std::vector<int> fixed_bounds(int N, int G) {
   std::vector<int> b;
   for (int c = 0; c < N; c += G) b.push_back(c);
@@ -320,12 +303,14 @@ int read_thresholds(const Scratch& sc, int slot, double* out, cudaStream_t s) {
   return TS_OK;
 }
 
-// Row stage shared by every mode: norms of all tile-rows of all layers, a keep flag for each, the
-// per-tile kept-row lists, and (optionally) the dense masks.
-//   sel: 0 = one global percentile over all layers (tw1 / tw2 stage 2), 1 = per-tile percentile
+// One cluster of eight blocks is faster than eleven launches over the whole GPU up to about this many values.
+constexpr long long kGroupSelect = 1 << 20;
+
+// Row stage of the modes group_stages does not serve: norms of all tile-rows of all layers, a keep flag for
+// each, the per-tile kept-row lists, and (optionally) the dense masks.
+//   sel: 0 = one global percentile over all layers, float64 scores only; 1 = per-tile percentile
 //        (BERT type 2), 2 = per-tile top-k by L1 (k = round(K * (1 - q/100))).
 int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>& bounds,
-              const std::vector<uint8_t*>& colkeep_dev, const std::vector<std::vector<uint8_t>>& colkeep_host,
               int sel, double q, bool wide, ts_mask_result* res, double* thr_out, Arena& arena,
               const Scratch& sc, cudaStream_t s, bool f64 = false) {
   const int nl = static_cast<int>(L.size());
@@ -342,7 +327,7 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
   double* norms64 = nullptr;   // float64 scores: norms, percentile and comparison all in double
   uint8_t* keep = nullptr;
   if (f64) {
-    if (sel != 0 || !colkeep_dev.empty()) {
+    if (sel != 0) {
       return ts_internal_fail(TS_ERR_UNSUPPORTED, "float64 scores are supported by the tw1 row stage only");
     }
     TSM_OK(arena.alloc(&norms64, total));
@@ -362,13 +347,8 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
     } else if (sel == 2) {
       TSM_CUDA(ts::tile_row_l1_launch(L[l].score, L[l].ld, L[l].K, bounds_dev[l], nt, norms + off[l], s));
     } else {
-      int uniform = 0;   // leading tiles that are exactly [128 t, 128 (t+1))
-      if (colkeep_dev.empty()) {
-        while (uniform < nt && bounds[l][uniform] == 128 * uniform && bounds[l][uniform + 1] == 128 * (uniform + 1)) ++uniform;
-      }
-      TSM_CUDA(ts::tile_row_norms_launch(L[l].score, L[l].ld, L[l].K, bounds_dev[l], nt,
-                                         colkeep_dev.empty() ? nullptr : colkeep_dev[l], norms + off[l],
-                                         sel == 0 ? 1 : 0, uniform, s));
+      TSM_CUDA(ts::tile_row_norms_launch(L[l].score, L[l].ld, L[l].K, bounds_dev[l], nt, nullptr, norms + off[l],
+                                         /*divide=*/0, 0, s));
     }
   }
   if (f64) {
@@ -380,10 +360,6 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
     if (thr_out) TSM_CUDA(cudaMemcpyAsync(thr_out, sc.thr + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
     TSM_CUDA(cudaStreamSynchronize(s));
     if (st64.error) return ts_internal_fail(TS_ERR_CUDA, "radix select lost its rank (non-finite input?)");
-  } else if (sel == 0) {
-    TSM_OK(percentile_to_device(norms, total, q, wide, false, sc, 1, s));
-    TSM_CUDA(ts::threshold_dev_launch(norms, total, sc.thr + 1, keep, s));
-    // the threshold and the select's error flag are read back with the lists, further down
   } else {
     for (int l = 0; l < nl; ++l) {
       const int nt = static_cast<int>(bounds[l].size()) - 1;
@@ -412,8 +388,7 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
   }
 
   // kept-row lists: one segment per (layer, tile).  Counts, their prefix sums and the compaction all
-  // stay on the device; the dense masks are enqueued behind them; one blocking read-back at the end
-  // brings the thresholds, the select's error flag, the offsets and the lists.
+  // stay on the device; the dense masks are enqueued behind them.
   std::vector<long long> seg(total_tiles + 1, 0);
   for (int l = 0; l < nl; ++l) {
     const int nt = tile_off[l + 1] - tile_off[l];
@@ -443,62 +418,16 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
     TSM_OK(arena.alloc(&toc_dev, tile_of_col[l].size()));
     TSM_CUDA(cudaMemcpyAsync(toc_dev, tile_of_col[l].data(), tile_of_col[l].size() * sizeof(int),
                              cudaMemcpyHostToDevice, s));
-    TSM_CUDA(ts::dense_mask_launch(keep + off[l], colkeep_dev.empty() ? nullptr : colkeep_dev[l], toc_dev,
+    TSM_CUDA(ts::dense_mask_launch(keep + off[l], nullptr, toc_dev,
                                    L[l].K, L[l].N, L[l].mask, L[l].ld_mask, s));
   }
-  // Read-back: threshold, the select's error flag, the offsets and (up to 64 Ki tile-rows) the whole
-  // upper-bound list array in one round trip; beyond that the exact size is awaited first (a second
-  // round trip is cheaper than the extra bytes).  The copies land in page-locked memory when it can be
-  // had, so they are asynchronous and the host blocks once.
-  ts::SelectState st_host;
-  memset(&st_host, 0, sizeof(st_host));
-  const bool want_sel = sel == 0 && !f64;
-  const bool one_trip = total <= (1 << 16);
   std::vector<int> optr(total_tiles + 1, 0);
-  std::vector<int> list;
-  const size_t head_bytes = 256;   // [0, 8): threshold, [64, 64 + sizeof(SelectState)): select state
-  static_assert(sizeof(ts::SelectState) <= head_bytes - 64, "select state does not fit the read-back header");
-  const size_t optr_bytes = (optr.size() * sizeof(int) + 255) & ~static_cast<size_t>(255);
-  const size_t list_bytes = one_trip ? static_cast<size_t>(total) * sizeof(int) : 0;
-  char* pin = static_cast<char*>(arena.pinned(head_bytes + optr_bytes + list_bytes));
-  if (pin) {
-    if (want_sel) {
-      TSM_CUDA(cudaMemcpyAsync(pin, sc.thr + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
-      TSM_CUDA(cudaMemcpyAsync(pin + 64, sc.st, sizeof(st_host), cudaMemcpyDeviceToHost, s));
-    }
-    TSM_CUDA(cudaMemcpyAsync(pin + head_bytes, optr_dev, optr.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-    if (one_trip && total > 0) {
-      TSM_CUDA(cudaMemcpyAsync(pin + head_bytes + optr_bytes, list_dev, list_bytes, cudaMemcpyDeviceToHost, s));
-    }
-    TSM_CUDA(cudaStreamSynchronize(s));   // seg, tile_of_col (host) must outlive their copies; everything is done
-    if (want_sel) {
-      if (thr_out) memcpy(thr_out, pin, sizeof(double));
-      memcpy(&st_host, pin + 64, sizeof(st_host));
-    }
-    memcpy(optr.data(), pin + head_bytes, optr.size() * sizeof(int));
-    if (one_trip) {
-      const int* lp = reinterpret_cast<const int*>(pin + head_bytes + optr_bytes);
-      list.assign(lp, lp + optr[total_tiles]);     // the kept ones: a prefix of the upper-bound array
-    }
-  } else {
-    if (want_sel) {
-      if (thr_out) TSM_CUDA(cudaMemcpyAsync(thr_out, sc.thr + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
-      TSM_CUDA(cudaMemcpyAsync(&st_host, sc.st, sizeof(st_host), cudaMemcpyDeviceToHost, s));
-    }
-    TSM_CUDA(cudaMemcpyAsync(optr.data(), optr_dev, optr.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-    if (one_trip) {
-      list.resize(total);
-      if (total > 0) TSM_CUDA(cudaMemcpyAsync(list.data(), list_dev, total * sizeof(int), cudaMemcpyDeviceToHost, s));
-    }
+  TSM_CUDA(cudaMemcpyAsync(optr.data(), optr_dev, optr.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  TSM_CUDA(cudaStreamSynchronize(s));   // seg, tile_of_col (host) must outlive their copies
+  std::vector<int> list(optr[total_tiles]);
+  if (!list.empty()) {
+    TSM_CUDA(cudaMemcpyAsync(list.data(), list_dev, list.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
     TSM_CUDA(cudaStreamSynchronize(s));
-  }
-  if (st_host.error) return ts_internal_fail(TS_ERR_CUDA, "radix select lost its rank (non-finite input?)");
-  if (!one_trip) {
-    list.resize(optr[total_tiles]);
-    if (!list.empty()) {
-      TSM_CUDA(cudaMemcpyAsync(list.data(), list_dev, list.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-      TSM_CUDA(cudaStreamSynchronize(s));
-    }
   }
 
   res->layers.resize(nl);
@@ -517,7 +446,7 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
       R.kept_k.insert(R.kept_k.end(), list.begin() + optr[gt], list.begin() + optr[gt + 1]);
       R.tile_k_ptr[t + 1] = static_cast<int>(R.kept_k.size());
       for (int c = bounds[l][t]; c < bounds[l][t + 1]; ++c) {
-        if (colkeep_host.empty() || colkeep_host[l][c]) R.kept_n.push_back(c);
+        R.kept_n.push_back(c);
       }
       R.tile_n_ptr[t + 1] = static_cast<int>(R.kept_n.size());
     }
@@ -525,11 +454,153 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
   return TS_OK;
 }
 
+// The column stage (two_d) and the row stage of the modes that rank all tile-rows of all layers together, in
+// five launches at most and one blocking wait: see mask_group.cu.  q_col / q_row: the stages' percentiles.
+int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col, double q_row, bool wide,
+                 ts_mask_result* res, Arena& arena, cudaStream_t s) {
+  const int nl = static_cast<int>(L.size());
+  ts::MaskGroup g;
+  memset(&g, 0, sizeof(g));
+  g.n = nl;
+  g.G = G;
+  std::vector<ts::MaskLayer> table(nl);
+  int cols = 0, tile_slots = 0, recs = 0, col_blocks = 0, norm_blocks = 0;
+  long long norms_n = 0, dense_blocks = 0;
+  for (int l = 0; l < nl; ++l) {
+    ts::MaskLayer& m = table[l];
+    m.score = L[l].score;
+    m.mask = L[l].mask;
+    m.ld = L[l].ld;
+    m.ld_mask = L[l].ld_mask;
+    m.K = L[l].K;
+    m.N = L[l].N;
+    m.col0 = cols;
+    m.max_tiles = two_d ? m.N / G + 1 : (m.N + G - 1) / G;
+    m.tile0 = tile_slots;
+    m.rec0 = recs;
+    m.col_blk0 = col_blocks;
+    m.norm_blk0 = norm_blocks;
+    m.dense_blk0 = static_cast<int>(dense_blocks);
+    m.norm0 = norms_n;
+    cols += m.N;
+    tile_slots += m.max_tiles + 1;
+    recs += m.max_tiles;
+    col_blocks += ts::group_col_blocks(m.N);
+    norm_blocks += ts::group_norm_blocks(m.K, m.max_tiles);
+    if (m.mask) dense_blocks += ts::group_dense_blocks(m.K, m.N);
+    norms_n += static_cast<long long>(m.max_tiles) * m.K;
+  }
+  g.list_blocks = recs;
+  if (nl <= ts::kInlineLayers) {
+    memcpy(g.inl, table.data(), nl * sizeof(ts::MaskLayer));
+  } else {
+    ts::MaskLayer* ext = nullptr;
+    TSM_OK(arena.alloc(&ext, nl));
+    TSM_CUDA(cudaMemcpyAsync(ext, table.data(), nl * sizeof(ts::MaskLayer), cudaMemcpyHostToDevice, s));
+    g.ext = ext;
+  }
+  // Page-locked block the kernels write their results to: thresholds, tiles per layer, tile bounds, list
+  // records, column flags and (for groups of up to 128 Ki tile-rows) the lists themselves.
+  const bool lists_on_host = norms_n <= (1 << 17);
+  size_t at = 0;
+  auto carve = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 63) & ~static_cast<size_t>(63);
+    return o;
+  };
+  const size_t o_thr = carve(2 * sizeof(double)), o_nt = carve(nl * sizeof(int)), o_bounds = carve(tile_slots * sizeof(int)),
+               o_rec = carve(recs * sizeof(int2)), o_keep = carve(cols), o_list = carve(lists_on_host ? norms_n * sizeof(int) : 0);
+  char* host = static_cast<char*>(arena.pinned(at));
+  if (!host) return ts_internal_fail(TS_ERR_NOMEM, "%zu bytes of page-locked memory for the results are not available", at);
+  float* norms = nullptr;
+  double* thr = nullptr;
+  int* cursor = nullptr;
+  int* list = nullptr;
+  TSM_OK(arena.alloc(&norms, norms_n));
+  TSM_OK(arena.alloc(&thr, 2));
+  TSM_OK(arena.alloc(&cursor, 1));
+  if (lists_on_host) list = reinterpret_cast<int*>(host + o_list);
+  else TSM_OK(arena.alloc(&list, norms_n));
+  TSM_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int), s));
+  uint8_t* col_keep = nullptr;
+  int* tile_of_col = nullptr;
+  double* thr_host = reinterpret_cast<double*>(host + o_thr);
+  int* nt_host = reinterpret_cast<int*>(host + o_nt);
+  int* bounds_host = reinterpret_cast<int*>(host + o_bounds);
+  uint8_t* keep_host = reinterpret_cast<uint8_t*>(host + o_keep);
+  if (two_d) {
+    float* cn = nullptr;
+    int *nt = nullptr, *bounds = nullptr;
+    TSM_OK(arena.alloc(&cn, cols));
+    TSM_OK(arena.alloc(&col_keep, cols));
+    TSM_OK(arena.alloc(&tile_of_col, cols));
+    TSM_OK(arena.alloc(&nt, nl));
+    TSM_OK(arena.alloc(&bounds, tile_slots));
+    TSM_CUDA(ts::group_col_norms_launch(g, col_blocks, cn, s));
+    TSM_CUDA(ts::group_percentile_launch(cn, cols, cols, g, q_col, wide ? 1 : 0, thr, thr_host, s));
+    TSM_CUDA(ts::group_columns_launch(g, cn, thr, col_keep, tile_of_col, bounds, nt, keep_host, bounds_host, nt_host, s));
+    g.n_tiles = nt;
+    g.bounds = bounds;
+  }
+  TSM_CUDA(ts::group_row_norms_launch(g, norm_blocks, col_keep, norms, s));
+  TSM_CUDA(ts::group_percentile_launch(norms, norms_n, norms_n, g, q_row, wide ? 1 : 0, thr + 1, thr_host + 1, s));
+  TSM_CUDA(ts::group_apply_launch(g, recs + static_cast<int>(dense_blocks), norms, thr + 1, col_keep, tile_of_col, cursor, list,
+                                  reinterpret_cast<int2*>(host + o_rec), s));
+  TSM_CUDA(cudaStreamSynchronize(s));
+  const int2* rec = reinterpret_cast<const int2*>(host + o_rec);
+  std::vector<int> far;
+  const int* lists = list;
+  if (!lists_on_host) {
+    long long total = 0;
+    for (int l = 0; l < nl; ++l) {
+      const int nt = two_d ? nt_host[l] : table[l].max_tiles;
+      for (int t = 0; t < nt; ++t) total += rec[table[l].rec0 + t].y;
+    }
+    far.resize(total);
+    if (total > 0) {
+      TSM_CUDA(cudaMemcpyAsync(far.data(), list, total * sizeof(int), cudaMemcpyDeviceToHost, s));
+      TSM_CUDA(cudaStreamSynchronize(s));
+    }
+    lists = far.data();
+  }
+  if (two_d) res->thr[0] = thr_host[0];
+  res->thr[1] = thr_host[1];
+  res->layers.resize(nl);
+  for (int l = 0; l < nl; ++l) {
+    ts_mask_result::Layer& R = res->layers[l];
+    const ts::MaskLayer& m = table[l];
+    const int nt = two_d ? nt_host[l] : m.max_tiles;
+    R.K = m.K;
+    R.N = m.N;
+    R.bounds.resize(nt + 1);
+    R.tile_k_ptr.assign(nt + 1, 0);
+    R.tile_n_ptr.assign(nt + 1, 0);
+    int total = 0;
+    for (int t = 0; t < nt; ++t) total += rec[m.rec0 + t].y;
+    R.kept_k.resize(total);
+    for (int t = 0; t <= nt; ++t) R.bounds[t] = two_d ? bounds_host[m.tile0 + t] : std::min(m.N, t * G);
+    if (!two_d) {
+      R.kept_n.resize(m.N);
+      for (int c = 0; c < m.N; ++c) R.kept_n[c] = c;
+    }
+    for (int t = 0; t < nt; ++t) {
+      const int2 r = rec[m.rec0 + t];
+      if (r.y > 0) memcpy(R.kept_k.data() + R.tile_k_ptr[t], lists + r.x, r.y * sizeof(int));
+      R.tile_k_ptr[t + 1] = R.tile_k_ptr[t] + r.y;
+      if (two_d) {
+        for (int c = R.bounds[t]; c < R.bounds[t + 1]; ++c) {
+          if (keep_host[m.col0 + c]) R.kept_n.push_back(c);
+        }
+        R.tile_n_ptr[t + 1] = static_cast<int>(R.kept_n.size());
+      } else {
+        R.tile_n_ptr[t + 1] = R.bounds[t + 1];
+      }
+    }
+  }
+  return TS_OK;
+}
+
 }  // namespace
-
-extern "C" {
-
-}  // extern "C"
 
 namespace {
 int build_tw_mask_impl(int mode, int n_layers, const void* const* scores_dev, const int* Ks, const int* Ns,
@@ -594,52 +665,17 @@ int build_tw_mask_impl(int mode, int n_layers, const void* const* scores_dev, co
     wide = true;
   }
   std::vector<std::vector<int>> bounds(n_layers);
-  std::vector<uint8_t*> colkeep_dev;
-  std::vector<std::vector<uint8_t>> colkeep_host;
   int rc = TS_OK;
+  const int sel = mode == TS_MASK_BERT_PER_TILE ? 1 : (mode == TS_MASK_TOPK_L1 ? 2 : 0);
   do {
-    if (two_d) {
-      // stage 1: global percentile over the column norms of all layers (prune_algo.py:64-67)
-      long long totalN = 0;
-      for (int l = 0; l < n_layers; ++l) totalN += L[l].N;
-      float* cn = nullptr;
-      uint8_t* ck = nullptr;
-      if ((rc = arena.alloc(&cn, totalN)) != TS_OK) break;
-      if ((rc = arena.alloc(&ck, totalN)) != TS_OK) break;
-      long long o = 0;
-      cudaError_t e = cudaSuccess;
-      for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
-        e = ts::col_norms_launch(L[l].score, L[l].ld, L[l].K, L[l].N, cn + o, s);
-        o += L[l].N;
-      }
-      if (e != cudaSuccess) {
-        rc = ts_internal_fail(TS_ERR_CUDA, "column norm kernel failed: %s", cudaGetErrorString(e));
-        break;
-      }
-      const double q_col = mode == TS_MASK_TW_COLS_ROWS ? g1percent : q;
-      if ((rc = percentile_to_device(cn, totalN, q_col, wide, false, sc, 0, s)) != TS_OK) break;
-      e = ts::threshold_dev_launch(cn, totalN, sc.thr + 0, ck, s);
-      std::vector<uint8_t> all(totalN);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(all.data(), ck, totalN, cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess && (rc = read_thresholds(sc, 0, &res->thr[0], s)) != TS_OK) break;
-      if (e != cudaSuccess) {
-        rc = ts_internal_fail(TS_ERR_CUDA, "column threshold failed: %s", cudaGetErrorString(e));
-        break;
-      }
-      o = 0;
-      colkeep_dev.resize(n_layers);
-      colkeep_host.resize(n_layers);
-      for (int l = 0; l < n_layers; ++l) {
-        colkeep_dev[l] = ck + o;
-        colkeep_host[l].assign(all.begin() + o, all.begin() + o + L[l].N);
-        bounds[l] = regroup_bounds(colkeep_host[l].data(), L[l].N, G);
-        o += L[l].N;
-      }
+    if (sel == 0 && !f64) {
+      rc = group_stages(L, G, two_d, mode == TS_MASK_TW_COLS_ROWS ? g1percent : q, q, wide, res, arena, s);
+      if (rc != TS_OK) break;
     } else {
       for (int l = 0; l < n_layers; ++l) bounds[l] = fixed_bounds(L[l].N, G);
+      rc = row_stage(L, bounds, sel, q, wide, res, &res->thr[1], arena, sc, s, f64);
+      if (rc != TS_OK) break;
     }
-    const int sel = mode == TS_MASK_BERT_PER_TILE ? 1 : (mode == TS_MASK_TOPK_L1 ? 2 : 0);
-    if ((rc = row_stage(L, bounds, colkeep_dev, colkeep_host, sel, q, wide, res, &res->thr[1], arena, sc, s, f64)) != TS_OK) break;
 
     if (tew) {
       // element-wise residual (tw_mix_fn, prune_algo.py:151-177): rank |w| - mask over every
@@ -660,7 +696,14 @@ int build_tw_mask_impl(int mode, int n_layers, const void* const* scores_dev, co
       }
       const double q2 = 100.0 - g1percent;
       const bool wide2 = sparsity_is_f64 != 0;
-      if ((rc = percentile_to_device(vals, total, q2, wide2, false, sc, 2, s)) != TS_OK) break;
+      if (total <= kGroupSelect) {
+        ts::MaskGroup none;
+        memset(&none, 0, sizeof(none));
+        e = ts::group_percentile_launch(vals, total, total, none, q2, wide2 ? 1 : 0, sc.thr + 2, nullptr, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(sc.st, 0, sizeof(ts::SelectState), s);
+      } else if ((rc = percentile_to_device(vals, total, q2, wide2, false, sc, 2, s)) != TS_OK) {
+        break;
+      }
       o = 0;
       for (int l = 0; l < n_layers && e == cudaSuccess; ++l) {
         e = ts::tew_apply_launch(vals + o, sc.thr + 2, L[l].K, L[l].N, L[l].mask, L[l].ld_mask, L[l].residual, s);

@@ -147,67 +147,6 @@ tile_row_l1_kernel(const float* __restrict__ score, long long ld, int K,
   out[static_cast<long long>(t) * K + k] = r;
 }
 
-// out[n] = sqrt(sum_k score[k][n]^2 in row order) / K
-//
-// The sum of one column is a chain of K dependent additions (NumPy reduces axis 0 row by row), so
-// the only parallelism is across columns.  A block owns kColsPerBlock columns: all 256 threads fetch
-// the next kColRows x kColsPerBlock slab (global loads in flight) while the first kColsPerBlock
-// threads walk the previous slab in shared memory, so the chain waits on shared memory, never on DRAM.
-constexpr int kColsPerBlock = 16;
-constexpr int kColRows = 128;
-constexpr int kColPerThread = kColsPerBlock * kColRows / 256;  // 8
-
-__global__ void __launch_bounds__(256)
-col_norms_kernel(const float* __restrict__ score, long long ld, int K, int N,
-                 float* __restrict__ out) {
-  __shared__ float slab[2][kColRows][kColsPerBlock];
-  const int n0 = blockIdx.x * kColsPerBlock;
-  const int tid = threadIdx.x;
-  const int lc = tid % kColsPerBlock;       // column inside the slab
-  const int lr = tid / kColsPerBlock;       // first row this thread fetches (stride 16 rows)
-  const bool col_ok = n0 + lc < N;
-  float reg[kColPerThread];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < kColPerThread; ++i) {
-      const int k = k0 + lr + i * (256 / kColsPerBlock);
-      reg[i] = (col_ok && k < K) ? __ldg(score + static_cast<long long>(k) * ld + n0 + lc) : 0.0f;
-    }
-  };
-  auto stash = [&](int buf) {
-#pragma unroll
-    for (int i = 0; i < kColPerThread; ++i) slab[buf][lr + i * (256 / kColsPerBlock)][lc] = reg[i];
-  };
-  fetch(0);
-  stash(0);
-  __syncthreads();
-  float acc = 0.0f;
-  int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += kColRows) {
-    const bool more = k0 + kColRows < K;
-    if (more) fetch(k0 + kColRows);
-    if (tid < kColsPerBlock) {
-      const int rows = min(kColRows, K - k0);
-      int r = 0;
-      if (k0 == 0) {
-        const float x = slab[buf][0][tid];
-        acc = __fmul_rn(x, x);
-        r = 1;
-      }
-#pragma unroll 8
-      for (; r < rows; ++r) {
-        const float x = slab[buf][r][tid];
-        acc = __fadd_rn(acc, __fmul_rn(x, x));
-      }
-    }
-    if (more) stash(buf ^ 1);
-    __syncthreads();
-    buf ^= 1;
-  }
-  if (tid < kColsPerBlock && n0 + tid < N)
-    out[n0 + tid] = __fdiv_rn(__fsqrt_rn(acc), static_cast<float>(K));
-}
-
 // ---------------------------------------------------------------------------------------------
 // Radix select over float32 values (order-preserving 32-bit keys)
 // ---------------------------------------------------------------------------------------------
@@ -824,13 +763,6 @@ cudaError_t tile_row_l1_launch(const float* score, long long ld, int K, const in
   if (K <= 0 || n_tiles <= 0) return cudaSuccess;
   dim3 grid((K + 255) / 256, n_tiles);
   tile_row_l1_kernel<<<grid, 256, 0, s>>>(score, ld, K, bounds_dev, out);
-  return cudaGetLastError();
-}
-
-cudaError_t col_norms_launch(const float* score, long long ld, int K, int N, float* out,
-                             cudaStream_t s) {
-  if (K <= 0 || N <= 0) return cudaSuccess;
-  col_norms_kernel<<<(N + kColsPerBlock - 1) / kColsPerBlock, 256, 0, s>>>(score, ld, K, N, out);
   return cudaGetLastError();
 }
 

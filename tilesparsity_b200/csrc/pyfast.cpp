@@ -7,11 +7,16 @@
 // which keep the rarely used forms (peer buffers, the CUDA-core twin) for themselves.
 #include <Python.h>
 
+#define NPY_NO_DEPRECATED_API NPY_1_7_API_VERSION
+#include <numpy/arrayobject.h>
+
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+
+#include <vector>
 
 #include "../../include/tilesparse.h"
 
@@ -192,6 +197,94 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(out));
 }
 
+PyObject* int_array(int n, int32_t** data) {
+  npy_intp dims[1] = {n};
+  PyObject* a = PyArray_SimpleNew(1, dims, NPY_INT32);
+  *data = a ? static_cast<int32_t*>(PyArray_DATA(reinterpret_cast<PyArrayObject*>(a))) : nullptr;
+  return a;
+}
+
+// build_mask(mode, scores, G, sparsity, sparsity_is_f64, g1percent, want_residual, device)
+//   -> (masks, residuals | None, [(bounds, tile_k_ptr, kept_k, tile_n_ptr, kept_n)], thresholds),
+// or None when a score is not a float32 matrix with contiguous rows on that device (the caller converts).
+PyObject* py_build_mask(PyObject*, PyObject* args) {
+  int mode, G, is_f64, want_residual, device;
+  double sparsity, g1;
+  PyObject* list;
+  if (!PyArg_ParseTuple(args, "iO!ididii", &mode, &PyList_Type, &list, &G, &sparsity, &is_f64, &g1, &want_residual, &device)) return nullptr;
+  const Py_ssize_t n = PyList_GET_SIZE(list);
+  std::vector<const void*> scores(n);
+  std::vector<int> K(n), N(n);
+  std::vector<int64_t> ld(n), ld_mask(n);
+  for (Py_ssize_t l = 0; l < n; ++l) {
+    PyObject* o = PyList_GET_ITEM(list, l);
+    if (!THPVariable_Check(o)) Py_RETURN_NONE;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (t.dim() != 2 || t.scalar_type() != at::kFloat || !on_device(t, device) || t.stride(1) != 1) Py_RETURN_NONE;
+    scores[l] = t.data_ptr();
+    K[l] = static_cast<int>(t.size(0));
+    N[l] = static_cast<int>(t.size(1));
+    ld[l] = t.stride(0);
+  }
+  c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)));
+  void* stream = stream_of(device);
+  std::vector<at::Tensor> masks, resid;
+  std::vector<uint8_t*> mask_ptr(n), resid_ptr(n, nullptr);
+  for (Py_ssize_t l = 0; l < n; ++l) {
+    masks.push_back(new_tensor({K[l], N[l]}, at::kBool, device));   // the kernels write 0 / 1 bytes
+    mask_ptr[l] = static_cast<uint8_t*>(masks[l].data_ptr());
+    ld_mask[l] = N[l];
+    if (want_residual) {
+      resid.push_back(new_tensor({K[l], N[l]}, at::kBool, device));
+      resid[l].zero_();
+      resid_ptr[l] = static_cast<uint8_t*>(resid[l].data_ptr());
+    }
+  }
+  ts_mask_result_t* res = nullptr;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS;
+  rc = ts_build_tw_mask(mode, static_cast<int>(n), scores.data(), K.data(), N.data(), ld.data(), G, sparsity, is_f64, g1, mask_ptr.data(),
+                        ld_mask.data(), want_residual ? resid_ptr.data() : nullptr, &res, stream);
+  Py_END_ALLOW_THREADS;
+  if (rc != TS_OK) return fail_code(rc);
+  PyObject *py_masks = PyList_New(n), *py_tiles = PyList_New(n), *py_resid = nullptr;
+  if (want_residual) {
+    py_resid = PyList_New(n);
+  } else {
+    py_resid = Py_None;
+    Py_INCREF(Py_None);
+  }
+  bool ok = py_masks && py_tiles && py_resid;
+  for (Py_ssize_t l = 0; ok && l < n; ++l) {
+    int nt = 0, nk = 0, nn = 0;
+    ts_mask_result_layer(res, static_cast<int>(l), &nt, &nk, &nn);
+    int32_t *b, *kp, *kk, *np, *nc;
+    PyObject* arrays[5] = {int_array(nt + 1, &b), int_array(nt + 1, &kp), int_array(nk, &kk), int_array(nt + 1, &np), int_array(nn, &nc)};
+    for (PyObject* a : arrays) ok = ok && a;
+    PyObject* tuple = ok ? PyTuple_New(5) : nullptr;
+    ok = ok && tuple;
+    if (!ok) {
+      for (PyObject* a : arrays) Py_XDECREF(a);
+      break;
+    }
+    ts_mask_result_copy(res, static_cast<int>(l), b, kp, kk, np, nc);
+    for (int i = 0; i < 5; ++i) PyTuple_SET_ITEM(tuple, i, arrays[i]);
+    PyList_SET_ITEM(py_tiles, l, tuple);
+    PyList_SET_ITEM(py_masks, l, THPVariable_Wrap(masks[l]));
+    if (want_residual) PyList_SET_ITEM(py_resid, l, THPVariable_Wrap(resid[l]));
+  }
+  double thr[3];
+  ts_mask_result_thresholds(res, thr);
+  ts_mask_result_destroy(res);
+  if (!ok) {
+    Py_XDECREF(py_masks);
+    Py_XDECREF(py_tiles);
+    Py_XDECREF(py_resid);
+    return nullptr;
+  }
+  return Py_BuildValue("(NNN(ddd))", py_masks, py_resid, py_tiles, thr[0], thr[1], thr[2]);
+}
+
 PyObject* py_bind(PyObject*, PyObject* type) {
   Py_XDECREF(g_error_type);
   Py_INCREF(type);
@@ -203,6 +296,7 @@ PyMethodDef kMethods[] = {
     {"bind", py_bind, METH_O, "Sets the exception type raised for C-ABI errors."},
     {"layer_desc", py_layer_desc, METH_VARARGS, "Capsule describing a layer to the functions below."},
     {"masked_gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_masked_gemm)), METH_FASTCALL, "TWLayer.masked_gemm"},
+    {"build_mask", py_build_mask, METH_VARARGS, "masks.build_mask on float32 CUDA scores"},
     {"transpose16", py_transpose16, METH_O, "layer.transpose16"},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_linear)), METH_FASTCALL, "layer.masked_linear"},
     {nullptr, nullptr, 0, nullptr}};
@@ -211,4 +305,7 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_tsfast", "Host path of the per-b
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__tsfast() { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__tsfast() {
+  import_array();
+  return PyModule_Create(&kModule);
+}

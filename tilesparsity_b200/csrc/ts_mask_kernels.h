@@ -15,9 +15,6 @@ cudaError_t tile_row_norms_launch(const float* score, long long ld, int K, const
 // out[t*K + k] = sum of |score[k, c]| over the tile's columns, left to right.
 cudaError_t tile_row_l1_launch(const float* score, long long ld, int K, const int* bounds_dev,
                                int n_tiles, float* out, cudaStream_t s);
-// out[n] = ||score[:, n]||_2 / K, rows accumulated in order.
-cudaError_t col_norms_launch(const float* score, long long ld, int K, int N, float* out,
-                             cudaStream_t s);
 // One digit pass of the radix select: hist[256] must be zero on entry.
 cudaError_t select_hist_launch(const float* vals, long long n, uint32_t prefix, int shift,
                                unsigned int* hist, cudaStream_t s);
@@ -97,5 +94,49 @@ cudaError_t tile_rank_launch(const float* vals, int K, int n_tiles, int mode, in
                              int ni, uint8_t* keep, float* stats, cudaStream_t s);
 cudaError_t threshold_per_tile_launch(const float* vals, int K, int n_tiles, const double* thr,
                                       uint8_t* keep, cudaStream_t s);
+
+// ---------------------------------------------------------------------------------------------
+// Whole groups of layers per launch (mask_group.cu)
+// ---------------------------------------------------------------------------------------------
+struct MaskLayer {
+  const float* score;
+  uint8_t* mask;
+  long long ld, ld_mask;
+  int K, N;
+  int col0;         // offset of its columns in the column arrays
+  int max_tiles;    // tiles it can have at most; exactly these when MaskGroup::n_tiles is null
+  int tile0;        // offset of its max_tiles + 1 tile bounds
+  int rec0;         // offset of its max_tiles list records
+  int col_blk0, norm_blk0, dense_blk0;   // first block of each launch
+  long long norm0;  // offset of its norms when the tiles are fixed
+};
+constexpr int kInlineLayers = 40;
+// The layer table, in the kernel arguments (ext: in device memory, for more than kInlineLayers layers).
+// n_tiles / bounds are null for the fixed partition into tiles of G columns; otherwise they are on the device,
+// written by the column stage, and the norms of all layers follow one another without gaps.
+struct MaskGroup {
+  int n, G;
+  int list_blocks;  // blocks of the apply launch that build lists (the sum of max_tiles)
+  int pad_;
+  const int* n_tiles;
+  const int* bounds;
+  const MaskLayer* ext;
+  MaskLayer inl[kInlineLayers];
+};
+static_assert(sizeof(MaskGroup) <= 3900, "MaskGroup travels in the kernel arguments");
+
+int group_col_blocks(int N);
+int group_norm_blocks(int K, int tiles);
+long long group_dense_blocks(int K, int N);
+cudaError_t group_col_norms_launch(const MaskGroup& g, int blocks, float* out, cudaStream_t s);
+// np.percentile(vals, q) of n float32 values (n is derived from g when g.n_tiles is set; n_max bounds it) into
+// *thr, and into *thr_host (page-locked host memory) when that is not null.
+cudaError_t group_percentile_launch(const float* vals, long long n, long long n_max, const MaskGroup& g, double q, int wide,
+                                    double* thr, double* thr_host, cudaStream_t s);
+cudaError_t group_columns_launch(const MaskGroup& g, const float* col_norms, const double* thr, uint8_t* keep, int* tile_of_col,
+                                 int* bounds, int* n_tiles, uint8_t* keep_host, int* bounds_host, int* n_tiles_host, cudaStream_t s);
+cudaError_t group_row_norms_launch(const MaskGroup& g, int blocks, const uint8_t* col_keep, float* norms, cudaStream_t s);
+cudaError_t group_apply_launch(const MaskGroup& g, int blocks, const float* norms, const double* thr, const uint8_t* col_keep,
+                               const int* tile_of_col, int* cursor, int* list, int2* records, cudaStream_t s);
 
 }  // namespace ts

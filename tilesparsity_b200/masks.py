@@ -77,62 +77,53 @@ def build_mask(name: str, scores, sparsity, granularity: int = 128, g1percent=No
     if g1percent is None:
         g1percent = {"tw1m": 5, "tw2m": 1}.get(name, 0)     # the reference's defaults (prune_algo.py:180,187)
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    sc = []
-    for s in scores:
-        t = s if isinstance(s, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(s))
-        if t.dim() != 2:
+    index = torch.cuda.current_device() if dev.index is None else dev.index
+    wide = int(_is_f64(sparsity) or _is_f64(g1percent))
+    args = (int(granularity), float(sparsity), wide, float(g1percent), int(tew and want_residual), index)
+    sc = list(scores)
+    got = _lib.fast().build_mask(mode, sc, *args)      # None: a score that has to be converted first
+    if got is None:
+        sc = [s if isinstance(s, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(s)) for s in sc]
+        if any(t.dim() != 2 for t in sc):
             raise ValueError("scores must be 2-D (use img2col_forward for conv kernels)")
-        sc.append(t)
-    # float64 scores (the reference's accumulated Taylor scores) keep their type: NumPy would do every
-    # step in double, and so does the library's float64 row stage
-    f64 = all(t.dtype == torch.float64 for t in sc)
-    if f64 and name not in ("tw1", "bert_type7"):
-        raise ValueError("float64 scores are supported by tw1 and bert_type7 only; cast them to float32 for " + name)
-    sc = [t.to(device=dev, dtype=torch.float64 if f64 else torch.float32) for t in sc]
-    sc = [t if t.stride(1) == 1 else t.contiguous() for t in sc]
+        # float64 scores (the reference's accumulated Taylor scores) keep their type: NumPy would do every
+        # step in double, and so does the library's float64 row stage
+        f64 = all(t.dtype == torch.float64 for t in sc)
+        if f64 and name not in ("tw1", "bert_type7"):
+            raise ValueError("float64 scores are supported by tw1 and bert_type7 only; cast them to float32 for " + name)
+        sc = [t.to(device=dev, dtype=torch.float64 if f64 else torch.float32) for t in sc]
+        sc = [t if t.stride(1) == 1 else t.contiguous() for t in sc]
+        got = _build_mask_f64(mode, sc, granularity, sparsity, dev) if f64 else _lib.fast().build_mask(mode, sc, *args)
+    masks, resid, lists, thr = got
+    tiles = [TileSet(int(m.shape[0]), int(m.shape[1]), int(granularity), *t) for m, t in zip(masks, lists)]
+    return MaskResult(masks, tiles, resid, thr)
+
+
+def _build_mask_f64(mode: int, sc, granularity, sparsity, dev):
+    """The float64 row stage (ts_build_tw_mask_f64), results as _tsfast.build_mask gives them."""
     n = len(sc)
-    masks = [torch.empty((t.shape[0], t.shape[1]), dtype=torch.uint8, device=dev) for t in sc]
-    resid = [torch.zeros((t.shape[0], t.shape[1]), dtype=torch.uint8, device=dev) for t in sc] \
-        if (tew and want_residual) else None
-    VP = C.c_void_p * n
-    IA = C.c_int * n
-    LA = C.c_int64 * n
+    masks = [torch.empty((t.shape[0], t.shape[1]), dtype=torch.bool, device=dev) for t in sc]
+    VP, IA, LA = C.c_void_p * n, C.c_int * n, C.c_int64 * n
     handle = C.c_void_p()
     with torch.cuda.device(dev):
-        if f64:
-            check(lib.ts_build_tw_mask_f64(
-                mode, n, VP(*[t.data_ptr() for t in sc]), IA(*[t.shape[0] for t in sc]), IA(*[t.shape[1] for t in sc]),
-                LA(*[t.stride(0) for t in sc]), int(granularity), float(sparsity),
-                VP(*[m.data_ptr() for m in masks]), LA(*[m.stride(0) for m in masks]), C.byref(handle),
-                C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
-        else:
-            check(lib.ts_build_tw_mask(
-                mode, n, VP(*[t.data_ptr() for t in sc]), IA(*[t.shape[0] for t in sc]), IA(*[t.shape[1] for t in sc]),
-                LA(*[t.stride(0) for t in sc]), int(granularity), float(sparsity),
-                int(_is_f64(sparsity) or _is_f64(g1percent)), float(g1percent), VP(*[m.data_ptr() for m in masks]),
-                LA(*[m.stride(0) for m in masks]), VP(*[r.data_ptr() for r in resid]) if resid else None,
-                C.byref(handle), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
+        check(lib.ts_build_tw_mask_f64(
+            mode, n, VP(*[t.data_ptr() for t in sc]), IA(*[t.shape[0] for t in sc]), IA(*[t.shape[1] for t in sc]),
+            LA(*[t.stride(0) for t in sc]), int(granularity), float(sparsity),
+            VP(*[m.data_ptr() for m in masks]), LA(*[m.stride(0) for m in masks]), C.byref(handle),
+            C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
     try:
-        tiles = []
-        for l, t in enumerate(sc):
+        lists = []
+        for l in range(n):
             nt, nk, nn = C.c_int(), C.c_int(), C.c_int()
             check(lib.ts_mask_result_layer(handle, l, C.byref(nt), C.byref(nk), C.byref(nn)))
-            b = np.zeros(nt.value + 1, np.int32)
-            kp = np.zeros(nt.value + 1, np.int32)
-            npz = np.zeros(nt.value + 1, np.int32)
-            kk = np.zeros(max(nk.value, 1), np.int32)
-            nn_a = np.zeros(max(nn.value, 1), np.int32)
-            p = lambda a: a.ctypes.data_as(C.POINTER(C.c_int32))
-            check(lib.ts_mask_result_copy(handle, l, p(b), p(kp), p(kk), p(npz), p(nn_a)))
-            tiles.append(TileSet(int(t.shape[0]), int(t.shape[1]), int(granularity), b, kp, kk[:nk.value], npz,
-                                 nn_a[:nn.value]))
+            arrays = [np.zeros(size, np.int32) for size in (nt.value + 1, nt.value + 1, nk.value, nt.value + 1, nn.value)]
+            check(lib.ts_mask_result_copy(handle, l, *[a.ctypes.data_as(C.POINTER(C.c_int32)) for a in arrays]))
+            lists.append(tuple(arrays))
         thr = (C.c_double * 3)()
         check(lib.ts_mask_result_thresholds(handle, thr))
     finally:
         lib.ts_mask_result_destroy(handle)
-    # the kernels write 0 / 1 bytes: reinterpreted, not converted
-    return MaskResult([m.view(torch.bool) for m in masks], tiles,
-                      [r.view(torch.bool) for r in resid] if resid else None, tuple(thr))
+    return masks, None, lists, tuple(thr)
 
 
 def build_pattern_mask(name: str, scores, sparsity, device=None):

@@ -163,8 +163,9 @@ __device__ __forceinline__ long long c_row_of(const EpiItem& w, int j) {
 // gelu(x) = x * 0.5 * (1 + tanh(u)), u = sqrt(2/pi) * (x + 0.044715 x^3)  (Pruning/BERT/utils/modeling.py:264-277),
 // for two values, written as x / (1 + exp(-2u)): the same function without the cancellation of 1 + tanh for
 // negative u.  The special-function unit bounds it (16 results per cycle and SM), so the two share one
-// reciprocal, 1 / (a b): three special-function instructions a pair.  exp's argument is cut at 2^60, so that
-// the product stays finite; beyond that the result is below 1e-17 |x| anyway.
+// reciprocal, 1 / (a b): three special-function instructions a pair.  exp's argument is cut at 2^60, so that the
+// product stays finite, and the factor is 0 from there on (it is below 1e-18): a large negative x gives -0 and
+// -inf a NaN, as the tanh form does.
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -175,21 +176,20 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu_denominator(float x) {
-  // -2u * log2(e) = x * (-2 sqrt(2/pi) log2(e)) * (1 + 0.044715 x^2)
-  const float p = fmaf(x * x, -0.10294324f, -2.3022082f);
-  return 1.0f + ex2_approx(fminf(x * p, 60.0f));
-}
+// -2u * log2(e) = x * (-2 sqrt(2/pi) log2(e)) * (1 + 0.044715 x^2)
+__device__ __forceinline__ float gelu_exponent(float x) { return x * fmaf(x * x, -0.10294324f, -2.3022082f); }
+constexpr float kGeluCut = 60.0f;
 __device__ __forceinline__ void gelu2(float& x0, float& x1) {
-  const float a = gelu_denominator(x0), b = gelu_denominator(x1);
+  const float t0 = gelu_exponent(x0), t1 = gelu_exponent(x1);
+  const float a = 1.0f + ex2_approx(fminf(t0, kGeluCut)), b = 1.0f + ex2_approx(fminf(t1, kGeluCut));
   const float r = rcp_approx(a * b);
-  x0 *= r * b;
-  x1 *= r * a;
+  x0 *= t0 < kGeluCut ? r * b : 0.0f;
+  x1 *= t1 < kGeluCut ? r * a : 0.0f;
 }
 
 __device__ __forceinline__ float apply_act(float x, int act) {
   if (act == kActRelu) return fmaxf(x, 0.0f);
-  if (act == kActGelu) return x * rcp_approx(gelu_denominator(x));
+  if (act == kActGelu) return x * rcp_approx(1.0f + ex2_approx(gelu_exponent(x)));
   return x;
 }
 

@@ -62,6 +62,9 @@ EncodeTiledFn encode_tiled_fn() {
       fn = reinterpret_cast<EncodeTiledFn>(p);
     }
   });
+  // A driver call needs a current context, which a host thread that has made no runtime call yet does not have.
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
   return fn;
 }
 
@@ -593,6 +596,8 @@ int current_sm_count(int* out) {
 }  // namespace
 
 struct ts_layer {
+  // One host thread at a time plans and launches a GEMM: schedules and output maps are filled in by the calls.
+  std::mutex mu;
   int K = 0, N = 0, G = 0, dtype = 0;
   int device = 0;
   int sm_count = 0;
@@ -1033,6 +1038,8 @@ namespace {
 // row-major C[M][ldc] (the caller has checked row_output_ok).
 int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc,
                     const ts_epilogue_t* epi, void* stream, int conv_wp, bool rows = false) {
+  if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
+  std::lock_guard<std::mutex> lock(l->mu);
   int rc = check_gemm_args(l, M, At, lda, Ct, rows ? std::max<int64_t>(ldc, (M + 7) / 8 * 8) : ldc);
   if (rc != TS_OK) return rc;
   if (!epi) return fail(TS_ERR_INVALID, "epilogue is NULL");
@@ -1399,9 +1406,9 @@ int ts_layer_schedule_stats(ts_layer_t* l, int M, int* n_ctas, float* cta_cost, 
 }
 
 // Schedules of the reference-signature entry point, per device: one per shape (sizes, kept counts and
-// offsets; the lists' addresses and contents belong to the call), the latest kMaxShim of them, so that a
-// program that alternates between layers neither rebuilds nor uploads anything (calls on one device must be
-// issued on one stream or externally ordered).
+// offsets; the lists' addresses and contents belong to the call), the latest kMaxShim of them and those a
+// captured graph refers to, so that a program that alternates between layers neither rebuilds nor uploads
+// anything (calls on one device must be issued on one stream or externally ordered).
 namespace {
 struct ShimSchedule {
   std::vector<int> key;
@@ -1413,6 +1420,7 @@ struct ShimSchedule {
   const void* B = nullptr;       // the weights `tmap` describes
   CUtensorMap tmap;
   unsigned long long used = 0;   // tick of the latest call
+  bool captured = false;         // a CUDA graph holds its addresses: never dropped
 };
 constexpr size_t kMaxShim = 16;
 struct ShimDevice {
@@ -1511,11 +1519,14 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
     for (int t = 0; t < block_num; ++t) c.key.insert(c.key.end(), {N_cal[t], K_cal[t], off_B[t], off_C[t]});
     c.n_items = static_cast<int>(flat.size());
     c.n_blocks = static_cast<int>(blocks.size());
-    if (sd.schedules.size() >= kMaxShim) {
-      auto oldest = sd.schedules.begin();
-      for (auto it = sd.schedules.begin(); it != sd.schedules.end(); ++it) {
-        if (it->used < oldest->used) oldest = it;
-      }
+    size_t n_free = 0;
+    auto oldest = sd.schedules.end();
+    for (auto it = sd.schedules.begin(); it != sd.schedules.end(); ++it) {
+      if (it->captured) continue;
+      ++n_free;
+      if (oldest == sd.schedules.end() || it->used < oldest->used) oldest = it;
+    }
+    if (n_free >= kMaxShim) {
       TS_CUDA(cudaDeviceSynchronize());
       free_shim(*oldest);
       sd.schedules.erase(oldest);
@@ -1534,6 +1545,9 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
     w = &sd.schedules.back();
   }
   w->used = ++sd.tick;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  TS_CUDA(cudaStreamIsCapturing(s, &capture));
+  if (capture != cudaStreamCaptureStatusNone) w->captured = true;
   if (w->B != B) {
     w->B = nullptr;
     int rc = make_weight_tmap(&w->tmap, dtype, B, N, K);

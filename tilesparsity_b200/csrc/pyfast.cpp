@@ -14,6 +14,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <vector>
@@ -23,6 +24,14 @@
 namespace {
 
 PyObject* g_error_type = nullptr;   // TileSparseError(code, message)
+
+// The interpreter's lock is given back while the library works, as ctypes does: a call may build a schedule, or wait for
+// room in the launch queue behind work that needs the interpreter.
+template <typename F>
+int unlocked(F&& f) {
+  pybind11::gil_scoped_release nogil;
+  return f();
+}
 
 struct Layer {
   ts_layer_t* h;
@@ -67,7 +76,7 @@ int new_output(const Layer& l, int64_t M, bool read_back, void* stream, at::Tens
   if (read_back) {
     out->zero_();
   } else if (!l.all_columns && M > 0) {
-    return ts_layer_zero_pruned(l.h, static_cast<int>(M), out->data_ptr(), M, stream);
+    return unlocked([&] { return ts_layer_zero_pruned(l.h, static_cast<int>(M), out->data_ptr(), M, stream); });
   }
   return TS_OK;
 }
@@ -91,6 +100,7 @@ bool read_float(PyObject* o, float* out) {
 
 // masked_gemm(layer, At, out | None, alpha, beta, bias | None, act) -> out
 PyObject* py_masked_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 7) return fail_value("masked_gemm takes 7 arguments");
   if (a[0] == Py_None) return fail_code(ts_masked_gemm_ex(nullptr, 0, nullptr, 0, nullptr, 0, nullptr, nullptr));   // a closed layer
   Layer* l = layer_of(a[0]);
@@ -128,11 +138,14 @@ PyObject* py_masked_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return fail_value("out must be an [N, M] tensor of the layer's dtype with M contiguous");
     }
   }
-  const int rc = ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out->data_ptr(), out->stride(0), &ep, stream);
+  const int rc = unlocked([&] {
+    return ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out->data_ptr(), out->stride(0), &ep, stream);
+  });
   if (rc != TS_OK) return fail_code(rc);
   if (out == &fresh) return THPVariable_Wrap(std::move(fresh));
   Py_INCREF(a[2]);
   return a[2];
+  END_HANDLE_TH_ERRORS
 }
 
 // The transpose of a 16-bit matrix with contiguous rows, or TS_* / a ValueError already set (*out undefined).
@@ -142,14 +155,17 @@ bool transpose(const at::Tensor& x, void* stream, at::Tensor* out) {
     return false;
   }
   *out = new_tensor({x.size(1), x.size(0)}, x.scalar_type(), x.get_device());
-  const int rc = ts_transpose16(x.data_ptr(), x.stride(0), out->data_ptr(), out->stride(0), static_cast<int>(x.size(0)),
-                                static_cast<int>(x.size(1)), stream);
+  const int rc = unlocked([&] {
+    return ts_transpose16(x.data_ptr(), x.stride(0), out->data_ptr(), out->stride(0), static_cast<int>(x.size(0)),
+                          static_cast<int>(x.size(1)), stream);
+  });
   if (rc != TS_OK) fail_code(rc);
   return rc == TS_OK;
 }
 
 // transpose16(x) -> its transpose
 PyObject* py_transpose16(PyObject*, PyObject* arg) {
+  HANDLE_TH_ERRORS
   if (!THPVariable_Check(arg)) return fail_value("transpose16 takes a tensor");
   const at::Tensor& x = THPVariable_Unpack(arg);
   if (!x.is_cuda()) return fail_value("transpose16 takes a 2-D 16-bit CUDA tensor with contiguous rows");
@@ -157,10 +173,12 @@ PyObject* py_transpose16(PyObject*, PyObject* arg) {
   at::Tensor out;
   if (!transpose(x, stream_of(x.get_device()), &out)) return nullptr;
   return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
 }
 
 // linear(layer, A [M, K], transpose_out) -> C [M, N], or Ct [N, M]
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 3) return fail_value("linear takes 3 arguments");
   if (a[0] == Py_None) return fail_code(ts_masked_gemm_ex(nullptr, 0, nullptr, 0, nullptr, 0, nullptr, nullptr));   // a closed layer
   Layer* l = layer_of(a[0]);
@@ -182,12 +200,14 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (rc != TS_OK) return fail_code(rc);
   if (rows) {
     out = new_tensor({M, l->N}, l->dtype, l->device);
-    rc = ts_masked_gemm_rows(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out.data_ptr(), l->N, &ep, stream);
+    rc = unlocked([&] { return ts_masked_gemm_rows(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out.data_ptr(), l->N, &ep, stream); });
     if (rc != TS_OK) return fail_code(rc);
     return THPVariable_Wrap(std::move(out));
   }
   rc = new_output(*l, M, false, stream, &out);
-  if (rc == TS_OK) rc = ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out.data_ptr(), M, &ep, stream);
+  if (rc == TS_OK) {
+    rc = unlocked([&] { return ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out.data_ptr(), M, &ep, stream); });
+  }
   if (rc != TS_OK) return fail_code(rc);
   if (a[2] == Py_True) {
     at::Tensor C;
@@ -195,6 +215,7 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(C));
   }
   return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject* int_array(int n, int32_t** data) {
@@ -208,6 +229,7 @@ PyObject* int_array(int n, int32_t** data) {
 //   -> (masks, residuals | None, [(bounds, tile_k_ptr, kept_k, tile_n_ptr, kept_n)], thresholds),
 // or None when a score is not a float32 matrix with contiguous rows on that device (the caller converts).
 PyObject* py_build_mask(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
   int mode, G, is_f64, want_residual, device;
   double sparsity, g1;
   PyObject* list;
@@ -241,11 +263,10 @@ PyObject* py_build_mask(PyObject*, PyObject* args) {
     }
   }
   ts_mask_result_t* res = nullptr;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS;
-  rc = ts_build_tw_mask(mode, static_cast<int>(n), scores.data(), K.data(), N.data(), ld.data(), G, sparsity, is_f64, g1, mask_ptr.data(),
-                        ld_mask.data(), want_residual ? resid_ptr.data() : nullptr, &res, stream);
-  Py_END_ALLOW_THREADS;
+  const int rc = unlocked([&] {
+    return ts_build_tw_mask(mode, static_cast<int>(n), scores.data(), K.data(), N.data(), ld.data(), G, sparsity, is_f64, g1,
+                            mask_ptr.data(), ld_mask.data(), want_residual ? resid_ptr.data() : nullptr, &res, stream);
+  });
   if (rc != TS_OK) return fail_code(rc);
   PyObject *py_masks = PyList_New(n), *py_tiles = PyList_New(n), *py_resid = nullptr;
   if (want_residual) {
@@ -283,6 +304,7 @@ PyObject* py_build_mask(PyObject*, PyObject* args) {
     return nullptr;
   }
   return Py_BuildValue("(NNN(ddd))", py_masks, py_resid, py_tiles, thr[0], thr[1], thr[2]);
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject* py_bind(PyObject*, PyObject* type) {

@@ -352,7 +352,10 @@ def masked_linear(A: torch.Tensor, layer: TWLayer, transpose_out: bool = True) -
     `TWLayer.masked_gemm` does not pay); where the tiles allow it the GEMM writes C row-major itself, else
     its output is transposed back.  Returns C[M, N], or Ct[N, M] with transpose_out=False.
     """
-    return _linear(layer._desc, A, bool(transpose_out))
+    if type(layer) is TWLayer:
+        return _linear(layer._desc, A, bool(transpose_out))
+    Ct = layer.masked_gemm(transpose16(A))       # a TEW layer, or whatever else multiplies K-major activations
+    return transpose16(Ct) if transpose_out else Ct
 
 
 def masked_matmul(A: torch.Tensor, W: torch.Tensor, kept_k_lists, col_mask=None, G: int = 128) -> torch.Tensor:

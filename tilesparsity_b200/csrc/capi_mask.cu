@@ -510,8 +510,10 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
   };
   const size_t o_thr = carve(2 * sizeof(double)), o_nt = carve(nl * sizeof(int)), o_bounds = carve(tile_slots * sizeof(int)),
                o_rec = carve(recs * sizeof(int2)), o_keep = carve(cols), o_list = carve(lists_on_host ? norms_n * sizeof(int) : 0);
+  // (in device memory and copied at the end where page-locked memory cannot be had)
   char* host = static_cast<char*>(arena.pinned(at));
-  if (!host) return ts_internal_fail(TS_ERR_NOMEM, "%zu bytes of page-locked memory for the results are not available", at);
+  const bool staged = host == nullptr;
+  if (staged) TSM_OK(arena.alloc(&host, at));
   float* norms = nullptr;
   double* thr = nullptr;
   int* cursor = nullptr;
@@ -546,10 +548,17 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
   TSM_CUDA(ts::group_percentile_launch(norms, norms_n, norms_n, g, q_row, wide ? 1 : 0, thr + 1, thr_host + 1, s));
   TSM_CUDA(ts::group_apply_launch(g, recs + static_cast<int>(dense_blocks), norms, thr + 1, col_keep, tile_of_col, cursor, list,
                                   reinterpret_cast<int2*>(host + o_rec), s));
+  std::vector<char> copy(staged ? at : 0);
+  if (staged) TSM_CUDA(cudaMemcpyAsync(copy.data(), host, at, cudaMemcpyDeviceToHost, s));
   TSM_CUDA(cudaStreamSynchronize(s));
+  if (staged) host = copy.data();
+  thr_host = reinterpret_cast<double*>(host + o_thr);
+  nt_host = reinterpret_cast<int*>(host + o_nt);
+  bounds_host = reinterpret_cast<int*>(host + o_bounds);
+  keep_host = reinterpret_cast<uint8_t*>(host + o_keep);
   const int2* rec = reinterpret_cast<const int2*>(host + o_rec);
   std::vector<int> far;
-  const int* lists = list;
+  const int* lists = reinterpret_cast<const int*>(host + o_list);
   if (!lists_on_host) {
     long long total = 0;
     for (int l = 0; l < nl; ++l) {

@@ -488,7 +488,7 @@ group_apply_kernel(const __grid_constant__ MaskGroup g, const float* __restrict_
   const int l = find_layer(g, block, [](const MaskLayer& m) { return m.dense_blk0; });
   const MaskLayer& L = layer_at(g, l);
   const unsigned int per_row = static_cast<unsigned int>((L.N + 15) / 16);
-  const unsigned int groups = per_row * static_cast<unsigned int>(L.K);   // (the caller keeps this below 2^31)
+  const unsigned int groups = per_row * static_cast<unsigned int>(L.K);   // (2^32 would be 275 GB of scores)
   const bool one_tile = !tile_of_col && g.G % 16 == 0;                    // 16 columns never straddle a tile
   const float* v = norms + norm_base(g, l);
   const bool vec = (L.N % 16) == 0 && (L.ld_mask % 16) == 0 && (reinterpret_cast<uintptr_t>(L.mask) & 15u) == 0;

@@ -1,0 +1,237 @@
+"""The host fast path, the row-major output, mixed unit widths and the grouped mask stages, at the sizes where each
+changes form.  GEMM results against float64 products of the same 16-bit inputs: the fp32 accumulation over K <= 3072
+rounds far below the 16-bit result, whose half unit is 2^-11 (fp16) or 2^-8 (bf16) of a value; TOL below is four
+times that, as a 2-norm ratio."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import tw_masks as om
+from tilesparsity_b200 import synth
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
+
+
+def _layer(K, N, keep, dtype, seed, col_keep=None):
+    from tilesparsity_b200 import TWLayer
+    g = synth.rng(seed)
+    col = (g.random(N) < col_keep) if col_keep is not None else None
+    from tilesparsity_b200.tiles import tile_bounds_from_col_mask
+    nt = len(tile_bounds_from_col_mask(np.ones(N, bool) if col is None else col, 128)) - 1
+    lists = [np.sort(g.permutation(K)[:keep]).astype(np.int32) for _ in range(nt)]
+    W = torch.from_numpy(g.standard_normal((K, N), dtype=np.float32) * np.float32(0.05)).cuda()
+    return TWLayer.from_lists(W, lists, col, 128, dtype), W
+
+
+def _dense(W, layer, dtype):
+    """W .* mask in float64, from the 16-bit weights."""
+    mask = torch.from_numpy(layer.tiles.dense_mask()).to(W.device)
+    return W.to(dtype).double() * mask
+
+
+def _rel(out, ref):
+    return float((out.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K,N,col_keep", [
+    (8, 64, 128, None),           # one tile, eight rows
+    (64, 256, 136, None),         # a last tile of eight columns
+    (72, 256, 248, None),         # a last tile of 120 columns: its last warp's box is cut off
+    (3080, 768, 768, None),       # odd numbers of granules, three per SM
+    (1000, 3072, 1536, None),
+    (264, 260, 204, None),        # N not a multiple of eight: output transposed back, two-byte transposes
+    (520, 512, 640, 0.7),         # pruned columns: output transposed back, zeros in them
+])
+def test_row_major_linear(M, K, N, col_keep, dtype):
+    from tilesparsity_b200 import masked_linear
+    layer, W = _layer(K, N, max(8, K // 3), dtype, M + K + N, col_keep)
+    A = torch.randn((M, K), device="cuda", generator=torch.Generator("cuda").manual_seed(M)).to(dtype)
+    torch.empty((64 << 20,), dtype=torch.uint8, device="cuda").fill_(0x7f)     # what the allocator hands out next is not zero
+    ref = A.double() @ _dense(W, layer, dtype)
+    C = masked_linear(A, layer)
+    layer.check()
+    assert C.shape == (M, N) and C.is_contiguous() and _rel(C, ref) <= TOL[dtype]
+    Ct = masked_linear(A, layer, transpose_out=False)
+    assert Ct.shape == (N, M) and torch.equal(Ct.t(), C)
+    dead = torch.from_numpy(~layer.tiles.col_mask()).cuda()
+    assert not C[:, dead].any()
+    layer.close()
+
+
+def test_row_major_linear_takes_a_tew_layer():
+    from tilesparsity_b200 import TEWLayer, build_mask, masked_linear
+    W = torch.randn((256, 384), device="cuda", generator=torch.Generator("cuda").manual_seed(1)) * 0.05
+    res = build_mask("tw2m", [W.abs()], 60.0, 128, 2.0, want_residual=True)
+    layer = TEWLayer(W, res.tiles[0], res.residuals[0], torch.float16)
+    A = torch.randn((72, 256), device="cuda").half()
+    ref = A.double() @ (W.half().double() * res.masks[0])
+    assert _rel(masked_linear(A, layer), ref) <= TOL[torch.float16]
+    # columns without any kept element are cleared in a caller's buffer
+    out = torch.full((384, 72), float("nan"), dtype=torch.float16, device="cuda")
+    assert _rel(layer.masked_gemm(A.t().contiguous(), out=out).t(), ref) <= TOL[torch.float16]
+    layer.close()
+
+
+@pytest.mark.parametrize("rows,cols,skip", [(8, 8, 0), (128, 136, 0), (120, 1024, 8), (1, 8, 0), (130, 250, 0), (136, 264, 4)])
+def test_transpose(rows, cols, skip):
+    """skip: the view starts that many elements into a wider matrix (16-byte pieces only where it is a multiple of 8)."""
+    from tilesparsity_b200 import transpose16
+    x = torch.randint(-32768, 32767, (rows, cols + skip), dtype=torch.int16, device="cuda")[:, skip:]
+    assert torch.equal(transpose16(x), x.t())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("col_keep", [None, 0.8])
+def test_new_outputs_are_whole(dtype, col_keep):
+    """An output the call makes itself: every kept column written, every pruned one zero, whatever its memory held."""
+    layer, W = _layer(128, 520, 40, dtype, 11, col_keep)
+    At = torch.randn((128, 264), device="cuda").to(dtype)
+    ref = _dense(W, layer, dtype).t() @ At.double()
+    for _ in range(3):
+        junk = torch.full((520, 264), float("nan"), dtype=dtype, device="cuda")
+        del junk
+        out = layer.masked_gemm(At)
+        assert _rel(out, ref) <= TOL[dtype]
+        assert not out[torch.from_numpy(~layer.tiles.col_mask()).cuda()].any()
+    layer.close()
+
+
+@pytest.mark.parametrize("col_keep", [None, 0.8])
+def test_gelu_at_the_ends_of_the_range(col_keep):
+    """The tanh form's limits: 0 for large negative sums (whatever their neighbours), the sum itself for large positive
+    ones, NaN for NaN and for -inf.  Bias carries the values: eight batch rows of zeros."""
+    layer, _ = _layer(64, 256, 16, torch.bfloat16, 5, col_keep)
+    vals = [-1e30, 1e30, -1e30, -1e30, -50.0, 50.0, -7.9, 0.5, float("inf"), -3e38, float("nan"), -1.0, float("-inf"), 2.0]
+    bias = torch.tensor((vals * 19)[:256], device="cuda")
+    out = layer.masked_gemm(torch.zeros((64, 72), dtype=torch.bfloat16, device="cuda"), bias=bias, activation="gelu")
+    x = bias.double()
+    ref = x * 0.5 * (1 + torch.tanh((2 / np.pi) ** 0.5 * (x + 0.044715 * x ** 3)))
+    kept = torch.from_numpy(layer.tiles.col_mask()).cuda()
+    got, want = out.double()[kept], ref[kept, None].expand(-1, 72)
+    assert torch.equal(got.isnan(), want.isnan())
+    ok = ~want.isnan()
+    # (bf16 rounding, and 1e-12 where the tanh form in any precision cancels to nothing)
+    assert torch.allclose(got[ok], want[ok], rtol=2 ** -8, atol=1e-12)
+    layer.close()
+
+
+def test_mixed_unit_widths():
+    """4.05 units per SM: units of two widths (checked to be so), against float64."""
+    layer, W = _layer(768, 1536, 384, torch.float16, 3)
+    At = torch.randn((768, 12800), device="cuda").half()
+    assert layer.schedule_stats(12800)["balance"] > 0.9
+    assert _rel(layer.masked_gemm(At), _dense(W, layer, torch.float16).t() @ At.double()) <= TOL[torch.float16]
+    layer.check()
+    layer.close()
+
+
+def test_outputs_that_alternate_and_threads():
+    """More output buffers than the layer remembers, from four threads with a stream each."""
+    layer, W = _layer(256, 512, 100, torch.float16, 9)
+    x = torch.randn((256, 520), device="cuda").half()
+    ref = layer.masked_gemm(x)
+    outs = [[torch.zeros_like(ref) for _ in range(6)] for _ in range(4)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(mine):
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                for _ in range(20):
+                    for o in mine:
+                        layer.masked_gemm(x, out=o)
+            s.synchronize()
+        except Exception as e:      # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(m,)) for m in outs]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors
+    assert all(torch.equal(o, ref) for m in outs for o in m)
+    layer.close()
+
+
+def test_an_output_that_cannot_be_allocated_is_an_error():
+    layer, _ = _layer(64, 8192, 16, torch.float16, 2)
+    x = torch.zeros((64, 8), dtype=torch.float16, device="cuda")
+    before = layer.masked_gemm(x)
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        layer.masked_gemm(torch.empty((64, 1 << 24), dtype=torch.float16, device="cuda"))    # 275 GB of output
+    assert torch.equal(layer.masked_gemm(x), before)
+    layer.close()
+
+
+def _stream_case(M, N, K, n_pruned, k_pruned, seed):
+    from tilesparsity_b200 import stream_gemm, tiles
+    r = synth.rng(seed)
+    n_ori, n_cal = tiles.reference_partition(N, n_pruned, 128)
+    first = [int(sum(n_ori[:t])) for t in range(len(n_ori))]
+    k_cal = [k_pruned] * len(n_cal)
+    mk = [stream_gemm.mask_gen(r, K, k) for k in k_cal]
+    mn = [stream_gemm.mask_gen(r, o, c) for o, c in zip(n_ori, n_cal)]
+    B = torch.zeros((N, K), dtype=torch.float16, device="cuda")
+    A = torch.randn((K, M), device="cuda").half()
+    ref = torch.zeros((N, M), dtype=torch.float64, device="cuda")
+    for t, c0 in enumerate(first):
+        w = torch.randn((n_cal[t], k_pruned), device="cuda").half() * 0.05
+        B[c0:c0 + n_cal[t], :k_pruned] = w
+        rows = torch.from_numpy(mk[t] + np.arange(k_pruned)).cuda().long()
+        cols = torch.from_numpy(mn[t] + np.arange(n_cal[t]) + c0).cuda().long()
+        ref[cols] = w.double() @ A[rows].double()
+    C = torch.zeros((N, M), dtype=torch.float16, device="cuda")
+    call = stream_gemm.prepare_stream_gemm_nn(M, N, K, 1.0, A, B, 0.0, C, len(n_cal), n_cal, k_cal, [torch.from_numpy(m).cuda() for m in mn],
+                                              [torch.from_numpy(m).cuda() for m in mk], [K * c for c in first], [M * c for c in first])
+    return call, C, ref
+
+
+def test_stream_calls_share_schedules_by_shape():
+    """Same shape with other lists and buffers, and more shapes than are kept: every call uses its own lists.  A graph's
+    schedule outlives them."""
+    cases = [_stream_case(264, 512, 256, 256, 64, s) for s in (1, 2)]
+    graph = torch.cuda.CUDAGraph()
+    cases[0][0]()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        cases[0][0]()
+    cases += [_stream_case(8 * m, 384, 128, 256, 40, m) for m in range(1, 20)]
+    for _ in range(2):
+        for call, C, ref in cases:
+            C.fill_(0)
+            call()
+            assert _rel(C, ref) <= TOL[torch.float16]
+    cases[0][1].fill_(0)
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert _rel(cases[0][1], cases[0][2]) <= TOL[torch.float16]
+
+
+@pytest.mark.parametrize("algo,sparsity,shapes", [
+    ("tw1", 75.0, [(128, 128 * 128)]),                       # 16384 tile rows: one block's percentile
+    ("tw1", 75.0, [(129, 128 * 128)]),                       # 16512: a cluster's
+    ("tw1", np.float64(60.0), [(1100, 128 * 128)]),          # more lists than fit the page-locked block
+    ("tw1", 50.0, [(40 + i, 136 + 8 * (i % 5)) for i in range(41)]),      # more layers than the kernel arguments hold
+    ("tw2", 70.0, [(33 + i, 100 + 7 * (i % 9)) for i in range(41)]),
+    ("tw2", 0.0, [(64, 256), (70, 130)]),                    # nothing pruned but the minimum
+    ("tw2", 99.0, [(64, 300)]),                              # tiles without rows
+    ("tw1m", 75.0, [(1025, 1024)]),                          # residual: more values than a cluster ranks
+])
+def test_grouped_masks_match_oracle(algo, sparsity, shapes):
+    from tilesparsity_b200 import build_mask
+    g = np.random.Generator(np.random.PCG64(len(shapes) * 1000 + shapes[0][0]))
+    scores = [np.abs(g.standard_normal(s, dtype=np.float32)) for s in shapes]
+    ref = om.pruning_fun(algo)(scores, sparsity, 128)
+    dev = [torch.from_numpy(s).cuda() for s in scores]
+    dev[0] = torch.nn.functional.pad(dev[0], (0, 3))[:, :dev[0].shape[1]]        # a row pitch that allows no 16-byte loads
+    res = build_mask(algo, dev, sparsity, 128, want_residual=algo.endswith("m"))
+    for l, (m, r) in enumerate(zip(res.masks, ref)):
+        r = np.asarray(r, dtype=bool)
+        assert np.array_equal(m.cpu().numpy(), r), l
+        if not algo.endswith("m"):
+            assert np.array_equal(res.tiles[l].dense_mask(), r), l

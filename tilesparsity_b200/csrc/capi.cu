@@ -140,7 +140,53 @@ int make_scratch_tmap(CUtensorMap* map, const float* scratch, long long rows, lo
   return TS_OK;
 }
 
+// Device memory of a layer comes in blocks that are carved up and handed on: a pruning program re-tiles its layers
+// every step, and a cudaMalloc / cudaFree pair per array (ten of them, each of which may wait for the device)
+// took longer than everything else a re-tiling does.
+struct DeviceBlock {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+inline size_t carve(size_t* at, size_t bytes) {
+  const size_t o = *at;
+  *at += (bytes + 255) & ~static_cast<size_t>(255);
+  return o;
+}
+// The smallest of `spare` that holds `bytes` without wasting more than three quarters, or a new block.  The caller
+// has waited for the device since a block came into `spare`.
+int take_block(std::vector<DeviceBlock>* spare, size_t bytes, DeviceBlock* out) {
+  size_t best = spare->size();
+  for (size_t i = 0; i < spare->size(); ++i) {
+    const size_t b = (*spare)[i].bytes;
+    if (b >= bytes && b / 4 <= bytes && (best == spare->size() || b < (*spare)[best].bytes)) best = i;
+  }
+  if (best < spare->size()) {
+    *out = (*spare)[best];
+    spare->erase(spare->begin() + best);
+    return TS_OK;
+  }
+  void* p = nullptr;
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && !spare->empty()) {   // give back what is kept before giving up
+    cudaGetLastError();
+    for (DeviceBlock& b : *spare) cudaFree(b.p);
+    spare->clear();
+    e = cudaMalloc(&p, bytes);
+  }
+  TS_CUDA(e);
+  *out = DeviceBlock{p, bytes};
+  return TS_OK;
+}
+constexpr size_t kSpareBlocks = 4;
+void give_block(std::vector<DeviceBlock>* spare, DeviceBlock* b) {
+  if (!b->p) return;
+  if (spare->size() < kSpareBlocks) spare->push_back(*b);
+  else cudaFree(b->p);
+  *b = DeviceBlock{};
+}
+
 struct Schedule {
+  DeviceBlock mem;             // holds everything below
   ts::WorkItem* d_units = nullptr;
   ts::BlockDesc* d_blocks = nullptr;
   int* d_meta = nullptr;       // one resolved record (ts::kBlockMetaInts ints) per descriptor of d_blocks
@@ -169,21 +215,6 @@ struct Schedule {
   int next_out_map = 0;
   bool all_dense = false;                 // every unit's tile keeps 128 consecutive columns (TMA tile stores only)
 };
-
-void free_schedule(Schedule& s) {
-  cudaFree(s.d_units);
-  cudaFree(s.d_blocks);
-  cudaFree(s.d_meta);
-  cudaFree(s.d_split);
-  cudaFree(s.d_scratch);
-  cudaFree(s.d_scratch_map);
-  s.d_scratch_map = nullptr;
-  s.d_units = nullptr;
-  s.d_blocks = nullptr;
-  s.d_meta = nullptr;
-  s.d_split = nullptr;
-  s.d_scratch = nullptr;
-}
 
 inline bool small_activations(long long at_rows, int M);   // defined with the scheduler below
 
@@ -316,20 +347,12 @@ void partition_contiguous(const std::vector<ts::TileDesc>& tiles, const std::vec
     if (ends) ends->push_back(line);
     return true;
   };
-  double lo = 0.0, hi = 0.0, weight = 0.0;
+  double lo = 0.0, weight = 0.0;
   for (int t : order) {
     lo = std::max<double>(lo, unit_cost(tiles[t].k_count, 1));
-    hi += static_cast<double>(unit_cost(tiles[t].k_count, 1)) * granules;
     weight += static_cast<double>((tiles[t].k_count + 63) / 64 + 2) * granules;
   }
-  lo = std::max(lo, hi / std::max(1, n_ctas) * 0.25);
-  for (int it = 0; it < 40 && hi - lo > 0.25; ++it) {
-    const double mid = 0.5 * (lo + hi);
-    if (fill(mid, nullptr)) hi = mid;
-    else lo = mid;
-  }
   std::vector<long long> ends_a, ends_b;
-  fill(hi, &ends_a);
   // (b) equal weight: granule i belongs to the piece its weight midpoint falls into
   {
     const double share = weight / n_ctas;
@@ -349,6 +372,16 @@ void partition_contiguous(const std::vector<ts::TileDesc>& tiles, const std::vec
     }
     ends_b.push_back(line);
   }
+  const double worst_b = cut(ends_b, nullptr);
+  // (a): the costs are whole numbers, a granule costs at least its weight, and (b) shows its largest to be enough
+  lo = std::max(lo, weight / n_ctas);
+  double hi = worst_b;
+  while (hi - lo > 0.25) {
+    const double mid = 0.5 * (lo + hi);
+    if (fill(mid, nullptr)) hi = mid;
+    else lo = mid;
+  }
+  fill(hi, &ends_a);
   // (c) per-tile split
   std::vector<long long> ends_c;
   const int nt = static_cast<int>(order.size());
@@ -378,7 +411,7 @@ void partition_contiguous(const std::vector<ts::TileDesc>& tiles, const std::vec
       }
     }
   }
-  const double worst_a = cut(ends_a, nullptr), worst_b = cut(ends_b, nullptr);
+  const double worst_a = cut(ends_a, nullptr);
   const double worst_c = ends_c.empty() ? 1e300 : cut(ends_c, nullptr);
   const std::vector<long long>* pick = &ends_a;
   if (worst_c <= std::min(worst_a, worst_b) * 1.03) pick = &ends_c;
@@ -416,55 +449,71 @@ void partition_blocked(const std::vector<ts::TileDesc>& tiles, const std::vector
       }
     }
   }
-  // Longest-processing-time list scheduling of `us` in its order; returns the largest load.
-  auto assign = [&](const std::vector<Unit>& us, std::vector<std::vector<Unit>>* out) -> float {
-    const int g = std::max<int>(1, std::min<int>(n_ctas, static_cast<int>(us.size())));
-    out->assign(g, {});
-    typedef std::pair<float, int> Load;  // (load, cta), smallest load first, then lowest cta
-    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
-    for (int b = 0; b < g; ++b) heap.push({0.0f, b});
+  // Longest-processing-time list scheduling of `us` in its order: cta_of[i] receives unit i's CTA (the least loaded
+  // one, then the lowest); returns the largest load.  A heap whose top is replaced in place.
+  std::vector<std::pair<float, int>> heap;
+  auto assign = [&](const std::vector<Unit>& us, std::vector<int>* cta_of) -> float {
+    const size_t g = std::max<size_t>(1, std::min<size_t>(n_ctas, us.size()));
+    heap.resize(g);
+    for (size_t b = 0; b < g; ++b) heap[b] = {0.0f, static_cast<int>(b)};
+    cta_of->resize(us.size());
     float worst = 0.0f;
-    for (const Unit& u : us) {
-      Load l = heap.top();
-      heap.pop();
-      (*out)[l.second].push_back(u);
-      l.first += u.cost;
+    for (size_t i = 0; i < us.size(); ++i) {
+      std::pair<float, int> l = heap[0];
+      (*cta_of)[i] = l.second;
+      l.first += us[i].cost;
       worst = std::max(worst, l.first);
-      heap.push(l);
+      size_t h = 0;
+      for (size_t c = 1; c < g; c = 2 * h + 1) {
+        if (c + 1 < g && heap[c + 1] < heap[c]) ++c;
+        if (!(heap[c] < l)) break;
+        heap[h] = heap[c];
+        h = c;
+      }
+      heap[h] = l;
     }
     return worst;
   };
-  float best = assign(units, lists);
+  std::vector<int> cta_of;
+  float best = assign(units, &cta_of);
   // A few units per SM: the last round can be nearly empty (4.05 units per SM run as long as 5).  Then the
   // first tiles keep units of `big` granules and the rest of the line is cut into units of one granule less,
   // so many of each that every SM gets the same number of both.  Narrower units move more weight bytes per
   // flop, so this is taken where the model promises at least 7 %: the 3072 x 768 call of the reference's
-  // perf table (600 units) 33.3 -> MIX_US us; at 5.4 units per SM (model -6 %) it measured no gain.  From 16
+  // perf table (600 units) 33.3 -> @MIX@ us; at 5.4 units per SM (model -6 %) it measured no gain.  From 16
   // rounds on the loss is below 7 % and the units stay whole.
   const int rounds = static_cast<int>((units.size() + n_ctas - 1) / n_ctas);
   if (!blocked && rounds <= 16) {
     const double per_cta = static_cast<double>(granules) * order.size() / n_ctas;
     const int big = std::min(cap, static_cast<int>(std::ceil(per_cta / rounds)));
     const int first = static_cast<int>(std::ceil(per_cta - rounds * (big - 1)));
+    std::vector<Unit> mixed;
+    std::vector<int> mixed_cta;
     for (int waves = std::max(0, first); big > 1 && waves <= std::min(rounds, first + 1); ++waves) {
       long long left = static_cast<long long>(waves) * n_ctas;      // units of `big` granules still to cut
-      std::vector<Unit> mixed;
+      float total = 0.0f;
+      mixed.clear();
       for (int t : order) {
         for (int g = 0; g < granules;) {
           const int len = std::min(left > 0 ? big : big - 1, granules - g);
           mixed.push_back(Unit{t, g * 64, len * 64, unit_cost(tiles[t].k_count, len)});
+          total += mixed.back().cost;
           g += len;
           --left;
         }
       }
-      std::vector<std::vector<Unit>> cand;
-      const float worst = assign(mixed, &cand);
+      if (total >= 0.93f * best * n_ctas) continue;
+      const float worst = assign(mixed, &mixed_cta);
       if (worst < 0.93f * best) {
         best = worst;
-        lists->swap(cand);
+        units.swap(mixed);
+        cta_of.swap(mixed_cta);
       }
     }
   }
+  lists->assign(std::max<size_t>(1, std::min<size_t>(n_ctas, units.size())), {});
+  for (auto& l : *lists) l.reserve(units.size() / lists->size() + 2);
+  for (size_t i = 0; i < units.size(); ++i) (*lists)[cta_of[i]].push_back(units[i]);
 }
 
 // Work distribution for the persistent kernel.  Units are (tile, run of batch rows); a run is a
@@ -605,6 +654,8 @@ struct ts_layer {
   std::vector<int> tile_k_ptr, kept_k, tile_n_ptr, kept_n;  // absolute indices
   std::vector<int> k_counts, n_counts;
   int max_k = 0;
+  DeviceBlock tile_mem;                 // kept rows, kept columns, tiles, packed weights
+  std::vector<DeviceBlock> spare;       // blocks of dropped schedules, at most kSpareBlocks
   int* d_kept_k = nullptr;
   int* d_kept_n = nullptr;     // kept columns, then (from n_kept on) the columns no tile keeps
   int n_kept = 0, n_pruned = 0;
@@ -647,16 +698,17 @@ struct ts_layer {
 
 namespace {
 
-void free_tiles(ts_layer* l) {
-  cudaFree(l->d_kept_k);
-  cudaFree(l->d_kept_n);
-  cudaFree(l->d_tiles);
-  cudaFree(l->d_wp);
+// The caller has waited for the device: queued launches may use the schedules' memory until then.
+void drop_schedules(ts_layer* l) {
+  for (auto& kv : l->schedules) give_block(&l->spare, &kv.second.mem);
+  l->schedules.clear();
+}
+
+void drop_tiles(ts_layer* l) {
   l->d_kept_k = l->d_kept_n = nullptr;
   l->d_tiles = nullptr;
   l->d_wp = nullptr;
-  for (auto& kv : l->schedules) free_schedule(kv.second);
-  l->schedules.clear();
+  drop_schedules(l);
   l->packed = false;
   l->ct_dirty = true;   // another tile set leaves other places of the staging output unwritten
 }
@@ -672,18 +724,9 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
   }
   if (l->schedules.size() >= 16) {  // bounded cache: drop everything, rebuild on demand
     TS_CUDA(cudaDeviceSynchronize());
-    for (auto& kv : l->schedules) free_schedule(kv.second);
-    l->schedules.clear();
+    drop_schedules(l);
   }
   Schedule s;
-  // frees what has been allocated so far if a step below fails
-  struct Guard {
-    Schedule* s;
-    bool armed;
-    ~Guard() {
-      if (armed) free_schedule(*s);
-    }
-  } guard{&s, true};
   std::vector<ts::WorkItem> flat;
   std::vector<ts::BlockDesc> blocks;
   ts::RowMap map;
@@ -706,11 +749,11 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
   if (allow_split) plan_split(l->k_counts, l->n_counts, at_rows, M, l->sm_count, &parts);
   bool any_split = false;
   for (int p : parts) any_split = any_split || p > 1;
+  std::vector<ts::SplitTile> st;
+  long long scratch_rows = 0;
   if (any_split) {
     std::vector<ts::TileDesc> vt;
     std::vector<int> kb0;
-    std::vector<ts::SplitTile> st;
-    int scratch_rows = 0;
     for (size_t t = 0; t < l->h_tiles.size(); ++t) {
       const ts::TileDesc& td = l->h_tiles[t];
       if (parts[t] <= 1) {
@@ -746,14 +789,6 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
                    &s.unit_rows, &s.cta_cost, &blocks, &s.blk_stride, &kb0);
     s.n_split = static_cast<int>(st.size());
     s.scratch_ld = M;
-    TS_CUDA(cudaMalloc(&s.d_split, st.size() * sizeof(ts::SplitTile)));
-    TS_CUDA(cudaMemcpy(s.d_split, st.data(), st.size() * sizeof(ts::SplitTile), cudaMemcpyHostToDevice));
-    TS_CUDA(cudaMalloc(&s.d_scratch, static_cast<size_t>(scratch_rows) * M * sizeof(float)));
-    CUtensorMap smap;
-    int mrc = make_scratch_tmap(&smap, s.d_scratch, scratch_rows, M);
-    if (mrc != TS_OK) return mrc;
-    TS_CUDA(cudaMalloc(&s.d_scratch_map, sizeof(CUtensorMap)));
-    TS_CUDA(cudaMemcpy(s.d_scratch_map, &smap, sizeof(CUtensorMap), cudaMemcpyHostToDevice));
   } else {
     build_schedule(l->h_tiles, at_rows, M, l->forced_unit_rows, l->sm_count, &flat, &s.rounds, &s.grid, &s.n_units,
                    &s.unit_rows, &s.cta_cost, &blocks, &s.blk_stride);
@@ -762,18 +797,43 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
   for (const ts::WorkItem& w : flat) {
     if (w.tile >= 0 && !(w.flags & ts::kItemDenseRows)) s.all_dense = false;
   }
+  // One block: what is uploaded first, then what the device fills in.
+  size_t bytes = 0;
+  const size_t o_units = carve(&bytes, flat.size() * sizeof(ts::WorkItem)), o_blocks = carve(&bytes, blocks.size() * sizeof(ts::BlockDesc)),
+               o_split = carve(&bytes, st.size() * sizeof(ts::SplitTile)), o_map = carve(&bytes, st.empty() ? 0 : sizeof(CUtensorMap)),
+               upload = bytes, o_meta = carve(&bytes, blocks.size() * ts::kBlockMetaInts * sizeof(int)),
+               o_scratch = carve(&bytes, static_cast<size_t>(scratch_rows) * M * sizeof(float));
   if (!flat.empty()) {
-    TS_CUDA(cudaMalloc(&s.d_units, flat.size() * sizeof(ts::WorkItem)));
-    TS_CUDA(cudaMemcpy(s.d_units, flat.data(), flat.size() * sizeof(ts::WorkItem),
-                       cudaMemcpyHostToDevice));
-    TS_CUDA(cudaMalloc(&s.d_blocks, blocks.size() * sizeof(ts::BlockDesc)));
-    TS_CUDA(cudaMemcpy(s.d_blocks, blocks.data(), blocks.size() * sizeof(ts::BlockDesc),
-                       cudaMemcpyHostToDevice));
-    TS_CUDA(cudaMalloc(&s.d_meta, blocks.size() * ts::kBlockMetaInts * sizeof(int)));
-    TS_CUDA(ts::expand_block_meta_launch(s.d_blocks, static_cast<long long>(blocks.size()), s.d_meta, map, nullptr));
-    TS_CUDA(cudaStreamSynchronize(nullptr));
+    int rc = take_block(&l->spare, bytes, &s.mem);
+    if (rc != TS_OK) return rc;
+    char* base = static_cast<char*>(s.mem.p);
+    s.d_units = reinterpret_cast<ts::WorkItem*>(base + o_units);
+    s.d_blocks = reinterpret_cast<ts::BlockDesc*>(base + o_blocks);
+    s.d_meta = reinterpret_cast<int*>(base + o_meta);
+    std::vector<char> host(upload);
+    memcpy(host.data() + o_units, flat.data(), flat.size() * sizeof(ts::WorkItem));
+    memcpy(host.data() + o_blocks, blocks.data(), blocks.size() * sizeof(ts::BlockDesc));
+    if (!st.empty()) {
+      s.d_split = reinterpret_cast<ts::SplitTile*>(base + o_split);
+      s.d_scratch = reinterpret_cast<float*>(base + o_scratch);
+      s.d_scratch_map = reinterpret_cast<CUtensorMap*>(base + o_map);
+      CUtensorMap smap;
+      rc = make_scratch_tmap(&smap, s.d_scratch, scratch_rows, M);
+      memcpy(host.data() + o_split, st.data(), st.size() * sizeof(ts::SplitTile));
+      memcpy(host.data() + o_map, &smap, sizeof(smap));
+    }
+    cudaError_t e = rc == TS_OK ? cudaMemcpy(base, host.data(), upload, cudaMemcpyHostToDevice) : cudaSuccess;
+    if (rc == TS_OK && e == cudaSuccess) {
+      e = ts::expand_block_meta_launch(s.d_blocks, static_cast<long long>(blocks.size()), s.d_meta, map, nullptr);
+      const cudaError_t done = cudaStreamSynchronize(nullptr);
+      if (e == cudaSuccess) e = done;
+    }
+    if (rc != TS_OK || e != cudaSuccess) {
+      cudaFree(s.mem.p);
+      TS_CUDA(e);
+      return rc;
+    }
   }
-  guard.armed = false;
   auto ins = l->schedules.emplace(key, s);
   *out = &ins.first->second;
   return TS_OK;
@@ -846,7 +906,9 @@ int ts_layer_create(ts_layer_t** out, int K, int N, int G, int dtype) {
 int ts_layer_destroy(ts_layer_t* l) {
   if (!l) return TS_OK;
   cudaDeviceSynchronize();
-  free_tiles(l);
+  drop_tiles(l);
+  cudaFree(l->tile_mem.p);
+  for (DeviceBlock& b : l->spare) cudaFree(b.p);
   cudaFree(l->d_status);
   cudaFree(l->d_peer_maps);
   cudaFree(l->d_at);
@@ -905,7 +967,7 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
   }
   TS_CUDA(cudaSetDevice(l->device));
   TS_CUDA(cudaDeviceSynchronize());
-  free_tiles(l);
+  drop_tiles(l);
   l->n_tiles = n_tiles;
   l->tile_k_ptr = kp;
   l->tile_n_ptr = np;
@@ -917,7 +979,6 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
   for (int v : kc) l->max_k = std::max(l->max_k, v);
   l->ldw = std::max<long long>(64, (l->max_k + 63) / 64 * 64);
   l->wp_rows = static_cast<long long>(std::max(1, n_tiles)) * 128;
-  TS_CUDA(cudaMalloc(&l->d_kept_k, std::max<size_t>(1, kk.size()) * sizeof(int)));
   std::vector<char> kept(l->N, 0);
   for (int v : nn) kept[v] = 1;
   l->n_kept = static_cast<int>(nn.size());
@@ -925,11 +986,23 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
     if (!kept[v]) nn.push_back(v);
   }
   l->n_pruned = static_cast<int>(nn.size()) - l->n_kept;
-  TS_CUDA(cudaMalloc(&l->d_kept_n, std::max<size_t>(1, nn.size()) * sizeof(int)));
-  TS_CUDA(cudaMalloc(&l->d_tiles, std::max(1, n_tiles) * sizeof(ts::TileDesc)));
-  TS_CUDA(cudaMalloc(&l->d_wp, static_cast<size_t>(l->wp_rows) * l->ldw * 2));
-  if (!kk.empty()) TS_CUDA(cudaMemcpy(l->d_kept_k, kk.data(), kk.size() * sizeof(int), cudaMemcpyHostToDevice));
-  if (!nn.empty()) TS_CUDA(cudaMemcpy(l->d_kept_n, nn.data(), nn.size() * sizeof(int), cudaMemcpyHostToDevice));
+  size_t bytes = 0;
+  const size_t o_k = carve(&bytes, kk.size() * sizeof(int)), o_n = carve(&bytes, nn.size() * sizeof(int)),
+               o_tiles = carve(&bytes, n_tiles * sizeof(ts::TileDesc)), upload = bytes,
+               o_wp = carve(&bytes, static_cast<size_t>(l->wp_rows) * l->ldw * 2);
+  if (l->tile_mem.bytes < bytes || l->tile_mem.bytes / 4 > bytes) {
+    cudaFree(l->tile_mem.p);
+    l->tile_mem = DeviceBlock{};
+    int rc = take_block(&l->spare, bytes, &l->tile_mem);
+    if (rc != TS_OK) return rc;
+  }
+  char* base = static_cast<char*>(l->tile_mem.p);
+  l->d_kept_k = reinterpret_cast<int*>(base + o_k);
+  l->d_kept_n = reinterpret_cast<int*>(base + o_n);
+  l->d_tiles = reinterpret_cast<ts::TileDesc*>(base + o_tiles);
+  std::vector<char> host(upload);
+  if (!kk.empty()) memcpy(host.data() + o_k, kk.data(), kk.size() * sizeof(int));
+  if (!nn.empty()) memcpy(host.data() + o_n, nn.data(), nn.size() * sizeof(int));
   std::vector<ts::TileDesc> td(n_tiles);
   for (int t = 0; t < n_tiles; ++t) {
     td[t].k_list = l->d_kept_k + kp[t];
@@ -950,9 +1023,10 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
   for (int t = 0; t < n_tiles; ++t) {
     if (nc[t] > 0 && (!td[t].pad_ || nn[np[t]] % 8 != 0)) l->rows_ok = false;
   }
-  if (n_tiles > 0) {
-    TS_CUDA(cudaMemcpy(l->d_tiles, td.data(), td.size() * sizeof(ts::TileDesc), cudaMemcpyHostToDevice));
-  }
+  if (n_tiles > 0) memcpy(host.data() + o_tiles, td.data(), td.size() * sizeof(ts::TileDesc));
+  TS_CUDA(cudaMemcpy(base, host.data(), upload, cudaMemcpyHostToDevice));
+  TS_CUDA(cudaStreamSynchronize(nullptr));   // (a copy from pageable memory may return before it has landed)
+  l->d_wp = reinterpret_cast<uint16_t*>(base + o_wp);
   l->h_tiles = td;
   return make_weight_tmap(&l->tmap, l->dtype, l->d_wp, l->wp_rows, l->ldw);
 }
@@ -982,8 +1056,7 @@ int ts_layer_set_unit_rows(ts_layer_t* l, int unit_rows) {
   if (unit_rows == l->forced_unit_rows) return TS_OK;
   TS_CUDA(cudaSetDevice(l->device));
   TS_CUDA(cudaDeviceSynchronize());   // cached schedules may be in use by queued launches
-  for (auto& kv : l->schedules) free_schedule(kv.second);
-  l->schedules.clear();
+  drop_schedules(l);
   l->forced_unit_rows = unit_rows;
   return TS_OK;
 }

@@ -77,8 +77,11 @@ class ConvTWLayer:
     def masked_conv(self, planes: torch.Tensor, geo: dict, out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
                     activation: str | None = None) -> torch.Tensor:
         """Ct [cout, m_padded] over the padded pixel space (pruned output channels stay as they are in `out`)."""
-        if out is None:
-            out = torch.zeros((self.cout, geo["m_padded"]), dtype=self.dtype, device=self.device)
+        if out is None:      # only pruned channels have to be cleared
+            out = torch.empty((self.cout, geo["m_padded"]), dtype=self.dtype, device=self.device)
+            with torch.cuda.device(self.device):
+                check(lib.ts_layer_zero_pruned(self.layer._h, geo["m_padded"], C.c_void_p(out.data_ptr()), out.stride(0),
+                                               _stream_ptr(self.device)))
         ep = _lib.Epilogue()
         ep.alpha, ep.beta = 1.0, 0.0
         if bias is not None:

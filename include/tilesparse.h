@@ -183,6 +183,14 @@ int ts_conv_repack(const void* Ct_dev, int64_t ldc, int B, int H, int W, int C, 
 int ts_masked_conv(ts_layer_t* layer, int B, int H, int W, const void* planes_dev, int64_t plane_ld, void* Ct_dev,
                    int64_t ldc, const ts_epilogue_t* epilogue, void* stream);
 
+/* The same with the result written as NHWC pixels y_nhwc_dev [B][H][W][N] by the GEMM's epilogue (no Ct, no
+ * ts_conv_unpack_output).  ts_conv_nhwc_output sets *supported to 1 where that is possible and the better form:
+ * the tiles keep all channels, each a run that starts at a multiple of 8, no tile pays for split-K, and the padded
+ * image is small enough.  beta and peer buffers are not supported.  The reference has no convolution path. */
+int ts_conv_nhwc_output(ts_layer_t* layer, int B, int H, int W, int* supported);
+int ts_masked_conv_nhwc(ts_layer_t* layer, int B, int H, int W, const void* planes_dev, int64_t plane_ld, void* y_nhwc_dev,
+                        const ts_epilogue_t* epilogue, void* stream);
+
 /* y[b][yy][xx][n] = Ct[n][(b*Hp + yy)*Wp + xx]: the padded-space output back to NHWC [B][H][W][N].
  * N and ldc must be multiples of 8 and both pointers 16-byte aligned. */
 int ts_conv_unpack_output(const void* Ct_dev, int64_t ldc, int B, int H, int W, int kh, int kw, int N, void* y_nhwc_dev,

@@ -235,3 +235,61 @@ def test_grouped_masks_match_oracle(algo, sparsity, shapes):
         assert np.array_equal(m.cpu().numpy(), r), l
         if not algo.endswith("m"):
             assert np.array_equal(res.tiles[l].dense_mask(), r), l
+
+
+@pytest.mark.parametrize("B,H,W,cin,cout,kh,kw,algo", [
+    (2, 5, 7, 16, 40, 3, 3, "tw1"),        # one narrow tile; two blocks of 8 channels in, five out
+    (3, 14, 14, 72, 256, 3, 3, "tw1"),     # nine blocks of channels in: no lane layout but one or two fits
+    (1, 9, 20, 24, 136, 5, 3, "tw1"),      # a second tile of eight channels
+    (2, 1, 1, 8, 8, 1, 1, "tw1"),          # one pixel
+    (5, 3, 260, 64, 128, 1, 5, "tw1"),     # rows of many groups
+    (3, 14, 14, 64, 264, 3, 3, "tw2"),     # pruned channels: through the padded space
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_convolution_output_forms_agree(B, H, W, cin, cout, kh, kw, algo, dtype):
+    """forward (NHWC from the GEMM where the tiles allow it) == GEMM into the padded space + unpacking, bit for bit, and
+    == conv2d in float64."""
+    from tilesparsity_b200 import ConvTWLayer, build_mask, masks
+    g = torch.Generator("cuda").manual_seed(B * 1000 + W)
+    w = torch.randn((kh, kw, cin, cout), device="cuda", generator=g) * (2.0 / (kh * kw * cin)) ** 0.5
+    res = build_mask(algo, masks.img2col_forward([w]), 40.0, 128)
+    layer = ConvTWLayer(w, res.tiles[0], dtype)
+    x = torch.randn((B, H, W, cin), device="cuda", generator=g).to(dtype)
+    bias = torch.randn((cout,), device="cuda", generator=g)
+    junk = torch.full((B, H, W, cout), float("nan"), dtype=dtype, device="cuda")
+    del junk
+    y = layer.forward(x, bias=bias, activation="relu")
+    planes, geo = layer.pack_input(x)
+    padded = layer.masked_conv(planes, geo, out=torch.zeros((cout, geo["m_padded"]), dtype=dtype, device="cuda"), bias=bias,
+                               activation="relu")
+    layer.layer.check()
+    assert torch.equal(y, layer.unpack_output(padded, geo))
+    wm = (w.to(dtype).double() * res.masks[0].view(kh, kw, cin, cout)).permute(3, 2, 0, 1)
+    ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), wm, bias.double(), padding=(kh // 2, kw // 2)).clamp_min(0)
+    kept = torch.from_numpy(res.tiles[0].col_mask()).cuda()
+    ref = ref.permute(0, 2, 3, 1) * kept
+    assert _rel(y, ref) <= TOL[dtype]
+    layer.close()
+
+
+def test_retiling_reuses_memory_soundly():
+    """A layer re-tiled between products, larger and smaller, and products of more batch sizes than schedules are kept
+    (split-K ones among them): every product is that of its own tiles."""
+    from tilesparsity_b200 import TWLayer, tiles
+    K, N = 4096, 256
+    W = torch.randn((K, N), device="cuda") * 0.05
+    layer = None
+    for step, keep in enumerate([3000, 500, 2600, 64, 4096, 200]):
+        g = synth.rng(step)
+        t = tiles.tiles_from_lists(K, N, 128, [np.sort(g.permutation(K)[:keep]).astype(np.int32) for _ in range(2)])
+        if layer is None:
+            layer = TWLayer(t, torch.float16, W.device)
+        else:
+            layer.retile(t)
+        layer.pack(W)
+        Wm = _dense(W, layer, torch.float16)
+        for M in [8 * m for m in range(1, 19)] + [2048]:
+            x = torch.randn((K, M), device="cuda").half()
+            assert _rel(layer.masked_gemm(x), Wm.t() @ x.double()) <= TOL[torch.float16]
+    layer.check()
+    layer.close()

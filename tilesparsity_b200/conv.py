@@ -74,6 +74,15 @@ class ConvTWLayer:
         g.update(B=geo["B"], H=geo["H"], W=geo["W"])
         return planes, g
 
+    @staticmethod
+    def _epilogue(bias, activation) -> "_lib.Epilogue":
+        ep = _lib.Epilogue()
+        ep.alpha, ep.beta = 1.0, 0.0
+        if bias is not None:
+            ep.bias_dev = bias.data_ptr()
+        ep.activation = _lib.ACTIVATIONS[activation]
+        return ep
+
     def masked_conv(self, planes: torch.Tensor, geo: dict, out: torch.Tensor | None = None, bias: torch.Tensor | None = None,
                     activation: str | None = None) -> torch.Tensor:
         """Ct [cout, m_padded] over the padded pixel space (pruned output channels stay as they are in `out`)."""
@@ -82,11 +91,7 @@ class ConvTWLayer:
             with torch.cuda.device(self.device):
                 check(lib.ts_layer_zero_pruned(self.layer._h, geo["m_padded"], C.c_void_p(out.data_ptr()), out.stride(0),
                                                _stream_ptr(self.device)))
-        ep = _lib.Epilogue()
-        ep.alpha, ep.beta = 1.0, 0.0
-        if bias is not None:
-            ep.bias_dev = bias.data_ptr()
-        ep.activation = _lib.ACTIVATIONS[activation]
+        ep = self._epilogue(bias, activation)
         with torch.cuda.device(self.device):
             check(lib.ts_masked_conv(self.layer._h, geo["B"], geo["H"], geo["W"], C.c_void_p(planes.data_ptr()),
                                      geo["plane_ld"], C.c_void_p(out.data_ptr()), out.stride(0), C.byref(ep),
@@ -104,6 +109,15 @@ class ConvTWLayer:
     def forward(self, x: torch.Tensor, bias: torch.Tensor | None = None, activation: str | None = None) -> torch.Tensor:
         """conv2d(x, W .* mask) (+ bias, activation) for NHWC x, stride 1, same padding; NHWC result."""
         planes, geo = self.pack_input(x)
+        direct = C.c_int()
+        check(lib.ts_conv_nhwc_output(self.layer._h, geo["B"], geo["H"], geo["W"], C.byref(direct)))
+        if direct.value:
+            y = torch.empty((geo["B"], geo["H"], geo["W"], self.cout), dtype=self.dtype, device=self.device)
+            ep = self._epilogue(bias, activation)
+            with torch.cuda.device(self.device):
+                check(lib.ts_masked_conv_nhwc(self.layer._h, geo["B"], geo["H"], geo["W"], C.c_void_p(planes.data_ptr()),
+                                              geo["plane_ld"], C.c_void_p(y.data_ptr()), C.byref(ep), _stream_ptr(self.device)))
+            return y
         return self.unpack_output(self.masked_conv(planes, geo, bias=bias, activation=activation), geo)
 
     def algorithmic_bytes(self, B: int, H: int, W: int) -> int:

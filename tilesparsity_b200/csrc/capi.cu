@@ -480,7 +480,7 @@ void partition_blocked(const std::vector<ts::TileDesc>& tiles, const std::vector
   // first tiles keep units of `big` granules and the rest of the line is cut into units of one granule less,
   // so many of each that every SM gets the same number of both.  Narrower units move more weight bytes per
   // flop, so this is taken where the model promises at least 7 %: the 3072 x 768 call of the reference's
-  // perf table (600 units) 33.3 -> @MIX@ us; at 5.4 units per SM (model -6 %) it measured no gain.  From 16
+  // perf table (600 units) 33.4 -> 33.2 us; at 5.4 units per SM (model -6 %) it measured no gain.  From 16
   // rounds on the loss is below 7 % and the units stay whole.
   const int rounds = static_cast<int>((units.size() + n_ctas - 1) / n_ctas);
   if (!blocked && rounds <= 16) {
@@ -1107,10 +1107,12 @@ int ts_layer_stats(const ts_layer_t* l, int64_t* kept_flops_per_row, int64_t* pa
 }  // extern "C"
 
 namespace {
-// The masked GEMM over a matrix At[K][lda] (conv_wp == 0) or over a convolution's input planes; rows: Ct is a
-// row-major C[M][ldc] (the caller has checked row_output_ok).
+// The masked GEMM over a matrix At[K][lda] (conv_wp == 0) or over a convolution's input planes; form: what Ct is (the
+// caller has checked that the layer allows it); nhwc: the image sizes for kOutNhwc.
 int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc,
-                    const ts_epilogue_t* epi, void* stream, int conv_wp, bool rows = false) {
+                    const ts_epilogue_t* epi, void* stream, int conv_wp, ts::OutForm form = ts::kOutColumns,
+                    const ts::EpilogueArgs* nhwc = nullptr) {
+  const bool rows = form != ts::kOutColumns;
   if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
   std::lock_guard<std::mutex> lock(l->mu);
   int rc = check_gemm_args(l, M, At, lda, Ct, rows ? std::max<int64_t>(ldc, (M + 7) / 8 * 8) : ldc);
@@ -1148,8 +1150,17 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   ep.scratch_ld = s->scratch_ld;
   ep.scratch_map = s->d_scratch_map;
   const CUtensorMap* tmap_c = nullptr;
+  if (form == ts::kOutNhwc) {
+    ep.nhwc_h = nhwc->nhwc_h;
+    ep.nhwc_w = nhwc->nhwc_w;
+    ep.nhwc_hp = nhwc->nhwc_hp;
+    ep.nhwc_wp8 = nhwc->nhwc_wp8;
+    ep.nhwc_mul_wp8 = nhwc->nhwc_mul_wp8;
+    ep.nhwc_mul_hp = nhwc->nhwc_mul_hp;
+    tmap_c = &l->tmap;   // not used: no output map
+  }
   for (const Schedule::OutMap& m : s->out_maps) {
-    if (m.ct == Ct && m.ldc == ldc && m.rows == rows) tmap_c = &m.map;
+    if (form != ts::kOutNhwc && m.ct == Ct && m.ldc == ldc && m.rows == rows) tmap_c = &m.map;
   }
   if (!tmap_c) {
     Schedule::OutMap& m = s->out_maps[s->next_out_map];
@@ -1191,7 +1202,7 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   const bool early = !l->wp_fresh;
   TS_CUDA(ts::masked_gemm_launch(l->dtype, s->unit_rows, l->tmap, tmap_c, s->d_units, s->rounds,
                                  s->grid, s->d_meta, s->blk_stride, At, lda, Ct, ldc, M, ep, l->d_status,
-                                 early, s->all_dense, rows, static_cast<cudaStream_t>(stream)));
+                                 early, s->all_dense, form, static_cast<cudaStream_t>(stream)));
   l->wp_fresh = false;
   if (s->n_split > 0) {
     TS_CUDA(ts::split_reduce_launch(l->dtype, s->d_split, s->n_split, s->d_scratch, s->scratch_ld, Ct, ldc, M,
@@ -1241,7 +1252,7 @@ int ts_masked_gemm_rows(ts_layer_t* l, int M, const void* At, int64_t lda, void*
     return fail(TS_ERR_UNSUPPORTED, "a row-major output takes neither beta nor peers");
   }
   if (ldc < l->N || (ldc % 8) != 0) return fail(TS_ERR_INVALID, "ldc=%lld must be a multiple of 8 and >= N=%d", (long long)ldc, l->N);
-  return run_masked_gemm(l, M, At, lda, C, ldc, epi, stream, 0, true);
+  return run_masked_gemm(l, M, At, lda, C, ldc, epi, stream, 0, ts::kOutRows);
 }
 
 int ts_layer_set_conv(ts_layer_t* l, int cin, int kh, int kw) {
@@ -1322,6 +1333,53 @@ int ts_masked_conv(ts_layer_t* l, int B, int H, int W, const void* planes_dev, i
   if (rc != TS_OK) return rc;
   if (plane_ld < need) return fail(TS_ERR_INVALID, "plane_ld=%lld is smaller than %lld", (long long)plane_ld, (long long)need);
   return run_masked_gemm(l, static_cast<int>(m), planes_dev, plane_ld, Ct_dev, ldc, epi, stream, wp);
+}
+
+int ts_conv_nhwc_output(ts_layer_t* l, int B, int H, int W, int* supported) {
+  if (!l || !supported) return fail(TS_ERR_INVALID, "NULL argument");
+  *supported = 0;
+  if (!l->rows_ok || l->conv_cin <= 0) return TS_OK;
+  int hp = 0, wp = 0;
+  int64_t m = 0;
+  int rc = ts_conv_geometry(B, H, W, l->conv_kh, l->conv_kw, &hp, &wp, &m, nullptr);
+  if (rc != TS_OK) return rc;
+  // the epilogue's reciprocal divisions: floor(i / d) = umulhi(i, ceil(2^32 / d)) holds for i * d < 2^32
+  if (m / 8 * std::max(wp / 8, hp) >= (1LL << 32)) return TS_OK;
+  if (l->split_k) {
+    std::vector<int> parts;
+    plan_split(l->k_counts, l->n_counts, static_cast<long long>(l->conv_kw) * l->conv_cin, static_cast<int>(m), l->sm_count, &parts);
+    for (int p : parts) {
+      if (p > 1) return TS_OK;
+    }
+  }
+  *supported = 1;
+  return TS_OK;
+}
+
+int ts_masked_conv_nhwc(ts_layer_t* l, int B, int H, int W, const void* planes_dev, int64_t plane_ld, void* y_nhwc_dev,
+                        const ts_epilogue_t* epi, void* stream) {
+  if (!l || !epi) return fail(TS_ERR_INVALID, "NULL argument");
+  if (l->conv_cin <= 0) return fail(TS_ERR_INVALID, "the layer has no convolution geometry (call ts_layer_set_conv)");
+  int hp = 0, wp = 0;
+  int64_t m = 0, need = 0;
+  int rc = ts_conv_geometry(B, H, W, l->conv_kh, l->conv_kw, &hp, &wp, &m, &need);
+  if (rc != TS_OK) return rc;
+  if (plane_ld < need) return fail(TS_ERR_INVALID, "plane_ld=%lld is smaller than %lld", (long long)plane_ld, (long long)need);
+  if (!l->rows_ok || m / 8 * std::max(wp / 8, hp) >= (1LL << 32)) {
+    return fail(TS_ERR_UNSUPPORTED, "the layer's tiles or the image size do not allow an NHWC output (ts_conv_nhwc_output)");
+  }
+  if (epi->beta != 0.0f || epi->n_peers != 0 || epi->multicast_ct) {
+    return fail(TS_ERR_UNSUPPORTED, "an NHWC output takes neither beta nor peers");
+  }
+  ts::EpilogueArgs g;
+  memset(&g, 0, sizeof(g));
+  g.nhwc_h = H;
+  g.nhwc_w = W;
+  g.nhwc_hp = hp;
+  g.nhwc_wp8 = wp / 8;
+  g.nhwc_mul_wp8 = wp / 8 > 1 ? 0xffffffffu / static_cast<uint32_t>(wp / 8) + 1u : 0u;
+  g.nhwc_mul_hp = hp > 1 ? 0xffffffffu / static_cast<uint32_t>(hp) + 1u : 0u;
+  return run_masked_gemm(l, static_cast<int>(m), planes_dev, plane_ld, y_nhwc_dev, l->N, epi, stream, wp, ts::kOutNhwc, &g);
 }
 
 int ts_conv_unpack_output(const void* Ct_dev, int64_t ldc, int B, int H, int W, int kh, int kw, int N, void* y_nhwc_dev,
@@ -1638,7 +1696,7 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
   ep.alpha = alpha;
   ep.beta = beta;
   TS_CUDA(ts::masked_gemm_launch(dtype, w->unit_rows, w->tmap, nullptr, w->d_units, w->rounds, w->grid, w->d_meta, w->blk_stride,
-                                 A, M, C, M, M, ep, sd.d_status, /*early_start=*/false, /*lean=*/false, /*rows=*/false, s));
+                                 A, M, C, M, M, ep, sd.d_status, /*early_start=*/false, /*lean=*/false, ts::kOutColumns, s));
   return TS_OK;
 }
 

@@ -95,6 +95,9 @@ struct EpilogueArgs {
   float* scratch;
   long long scratch_ld;
   const CUtensorMap* scratch_map;
+  // Convolutions whose result leaves as NHWC: the image, its padded space (Wp / 8 and Hp) and their reciprocals.
+  int nhwc_h, nhwc_w, nhwc_hp, nhwc_wp8;
+  uint32_t nhwc_mul_wp8, nhwc_mul_hp;
 };
 
 // One tile whose kept rows were split over `parts` units per batch block: part p wrote its fp32 partial
@@ -331,6 +334,10 @@ __device__ __forceinline__ void bulk_store(void* gdst, uint32_t ssrc, uint32_t b
                : "memory");
 }
 
+// A tensor map in device memory was written by the host: later uses by this thread see that version.
+__device__ __forceinline__ void fence_tensormap(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
 __device__ __forceinline__ void bulk_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }

@@ -23,10 +23,12 @@ namespace ts {
 // lean: every unit of the schedule has kItemDenseRows set (the kernel then takes its store-only variant
 // when beta is 0).  rows: tmap_c is a map over a row-major output C[M][N] (box 32 columns x 64 rows, no
 // swizzle) and every tile's first column is a multiple of 8; needs lean and beta == 0.
+// Where the result goes: Ct [N][ldc], a row-major C [M][ldc], or NHWC pixels [B][H][W][ldc].
+enum OutForm { kOutColumns, kOutRows, kOutNhwc };
 cudaError_t masked_gemm_launch(int dtype, int unit_rows, const CUtensorMap& tmap_w, const CUtensorMap* tmap_c,
                                const WorkItem* sched, int rounds, int grid, const int* block_meta,
                                int blk_stride, const void* At, long long lda, void* Ct, long long ldc, int M,
-                               const EpilogueArgs& ep, int* status, bool early_start, bool lean, bool rows,
+                               const EpilogueArgs& ep, int* status, bool early_start, bool lean, OutForm form,
                                cudaStream_t stream);
 
 // Adds up the fp32 partial sums the split-K units of a schedule left in `scratch` and finishes the

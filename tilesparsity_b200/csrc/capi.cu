@@ -449,71 +449,26 @@ void partition_blocked(const std::vector<ts::TileDesc>& tiles, const std::vector
       }
     }
   }
-  // Longest-processing-time list scheduling of `us` in its order: cta_of[i] receives unit i's CTA (the least loaded
-  // one, then the lowest); returns the largest load.  A heap whose top is replaced in place.
-  std::vector<std::pair<float, int>> heap;
-  auto assign = [&](const std::vector<Unit>& us, std::vector<int>* cta_of) -> float {
-    const size_t g = std::max<size_t>(1, std::min<size_t>(n_ctas, us.size()));
-    heap.resize(g);
-    for (size_t b = 0; b < g; ++b) heap[b] = {0.0f, static_cast<int>(b)};
-    cta_of->resize(us.size());
-    float worst = 0.0f;
-    for (size_t i = 0; i < us.size(); ++i) {
-      std::pair<float, int> l = heap[0];
-      (*cta_of)[i] = l.second;
-      l.first += us[i].cost;
-      worst = std::max(worst, l.first);
-      size_t h = 0;
-      for (size_t c = 1; c < g; c = 2 * h + 1) {
-        if (c + 1 < g && heap[c + 1] < heap[c]) ++c;
-        if (!(heap[c] < l)) break;
-        heap[h] = heap[c];
-        h = c;
-      }
-      heap[h] = l;
+  // Longest-processing-time list scheduling in that order: a unit goes to the least loaded CTA, then the lowest.  A heap
+  // whose top is replaced in place.
+  const size_t g = std::max<size_t>(1, std::min<size_t>(n_ctas, units.size()));
+  lists->assign(g, {});
+  for (auto& l : *lists) l.reserve(units.size() / g + 2);
+  std::vector<std::pair<float, int>> heap(g);
+  for (size_t b = 0; b < g; ++b) heap[b] = {0.0f, static_cast<int>(b)};
+  for (const Unit& u : units) {
+    std::pair<float, int> l = heap[0];
+    (*lists)[l.second].push_back(u);
+    l.first += u.cost;
+    size_t h = 0;
+    for (size_t c = 1; c < g; c = 2 * h + 1) {
+      if (c + 1 < g && heap[c + 1] < heap[c]) ++c;
+      if (!(heap[c] < l)) break;
+      heap[h] = heap[c];
+      h = c;
     }
-    return worst;
-  };
-  std::vector<int> cta_of;
-  float best = assign(units, &cta_of);
-  // A few units per SM: the last round can be nearly empty (4.05 units per SM run as long as 5).  Then the
-  // first tiles keep units of `big` granules and the rest of the line is cut into units of one granule less,
-  // so many of each that every SM gets the same number of both.  Narrower units move more weight bytes per
-  // flop, so this is taken where the model promises at least 7 %: the 3072 x 768 call of the reference's
-  // perf table (600 units) 33.4 -> 33.2 us; at 5.4 units per SM (model -6 %) it measured no gain.  From 16
-  // rounds on the loss is below 7 % and the units stay whole.
-  const int rounds = static_cast<int>((units.size() + n_ctas - 1) / n_ctas);
-  if (!blocked && rounds <= 16) {
-    const double per_cta = static_cast<double>(granules) * order.size() / n_ctas;
-    const int big = std::min(cap, static_cast<int>(std::ceil(per_cta / rounds)));
-    const int first = static_cast<int>(std::ceil(per_cta - rounds * (big - 1)));
-    std::vector<Unit> mixed;
-    std::vector<int> mixed_cta;
-    for (int waves = std::max(0, first); big > 1 && waves <= std::min(rounds, first + 1); ++waves) {
-      long long left = static_cast<long long>(waves) * n_ctas;      // units of `big` granules still to cut
-      float total = 0.0f;
-      mixed.clear();
-      for (int t : order) {
-        for (int g = 0; g < granules;) {
-          const int len = std::min(left > 0 ? big : big - 1, granules - g);
-          mixed.push_back(Unit{t, g * 64, len * 64, unit_cost(tiles[t].k_count, len)});
-          total += mixed.back().cost;
-          g += len;
-          --left;
-        }
-      }
-      if (total >= 0.93f * best * n_ctas) continue;
-      const float worst = assign(mixed, &mixed_cta);
-      if (worst < 0.93f * best) {
-        best = worst;
-        units.swap(mixed);
-        cta_of.swap(mixed_cta);
-      }
-    }
+    heap[h] = l;
   }
-  lists->assign(std::max<size_t>(1, std::min<size_t>(n_ctas, units.size())), {});
-  for (auto& l : *lists) l.reserve(units.size() / lists->size() + 2);
-  for (size_t i = 0; i < units.size(); ++i) (*lists)[cta_of[i]].push_back(units[i]);
 }
 
 // Work distribution for the persistent kernel.  Units are (tile, run of batch rows); a run is a

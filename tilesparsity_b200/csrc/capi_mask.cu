@@ -502,14 +502,15 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
   // Page-locked block the kernels write their results to: thresholds, tiles per layer, tile bounds, list
   // records, column flags and (for groups of up to 128 Ki tile-rows) the lists themselves.
   const bool lists_on_host = norms_n <= (1 << 17);
+  const long long list_cap = norms_n + static_cast<long long>(recs) * ts::kListAlign;
   size_t at = 0;
   auto carve = [&](size_t bytes) {
     const size_t o = at;
-    at += (bytes + 63) & ~static_cast<size_t>(63);
+    at += (bytes + 127) & ~static_cast<size_t>(127);
     return o;
   };
   const size_t o_thr = carve(2 * sizeof(double)), o_nt = carve(nl * sizeof(int)), o_bounds = carve(tile_slots * sizeof(int)),
-               o_rec = carve(recs * sizeof(int2)), o_keep = carve(cols), o_list = carve(lists_on_host ? norms_n * sizeof(int) : 0);
+               o_rec = carve(recs * sizeof(int2)), o_keep = carve(cols), o_list = carve(lists_on_host ? list_cap * sizeof(int) : 0);
   // (in device memory and copied at the end where page-locked memory cannot be had)
   char* host = static_cast<char*>(arena.pinned(at));
   const bool staged = host == nullptr;
@@ -522,7 +523,7 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
   TSM_OK(arena.alloc(&thr, 2));
   TSM_OK(arena.alloc(&cursor, 1));
   if (lists_on_host) list = reinterpret_cast<int*>(host + o_list);
-  else TSM_OK(arena.alloc(&list, norms_n));
+  else TSM_OK(arena.alloc(&list, list_cap));
   TSM_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int), s));
   uint8_t* col_keep = nullptr;
   int* tile_of_col = nullptr;
@@ -563,7 +564,7 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
     long long total = 0;
     for (int l = 0; l < nl; ++l) {
       const int nt = two_d ? nt_host[l] : table[l].max_tiles;
-      for (int t = 0; t < nt; ++t) total += rec[table[l].rec0 + t].y;
+      for (int t = 0; t < nt; ++t) total += (rec[table[l].rec0 + t].y + ts::kListAlign - 1) / ts::kListAlign * ts::kListAlign;
     }
     far.resize(total);
     if (total > 0) {

@@ -111,6 +111,8 @@ struct MaskLayer {
   long long norm0;  // offset of its norms when the tiles are fixed
 };
 constexpr int kInlineLayers = 40;
+// Every tile's list of kept rows starts at a multiple of this many ints (a 128-byte line).
+constexpr int kListAlign = 32;
 // The layer table, in the kernel arguments (ext: in device memory, for more than kInlineLayers layers).
 // n_tiles / bounds are null for the fixed partition into tiles of G columns; otherwise they are on the device,
 // written by the column stage, and the norms of all layers follow one another without gaps.

@@ -108,22 +108,45 @@ conv_pack_input_kernel(const uint16_t* __restrict__ x, int B, int H, int W, int 
   }
 }
 
+// How the lanes of a warp are spread in the register-transpose kernels below: 2^lc neighbouring blocks of 8
+// channels (16 bytes of an NHWC pixel each) by 32 >> lc neighbouring groups of 8 pixels (16 bytes of a
+// channel row each).  With lc = 2 an access covers 64-byte pieces of the NHWC side and 128-byte lines of the
+// channel-major side.  (All 32 lanes along the pixels, lc = 0, leave half of every NHWC sector to another block;
+// lc = 3 cuts the plane rows into 64-byte pieces.)  Cold, 64 images of 14 x 14 and 512 channels, three taps: packing
+// 18.5 / 16.4 / 16.4 / 22.6 us with lc = 0 / 1 / 2 / 3, unpacking 14.3 / 12.3 / 12.3 / 12.3; 8 of 112 x 112: packing
+// 64 channels 18.4 / 16.4 / 14.4 / 18.5, unpacking 128 channels 28.7 / 16.4 / 16.4 / 14.5.  The largest lc up to 2
+// that wastes at most a quarter of the lanes past the last channel block.
+int lanes_over_channels(int n_cb) {
+  for (int lc = 2; lc > 0; --lc) {
+    const int padded = ((n_cb + (1 << lc) - 1) >> lc) << lc;
+    if (4 * padded <= 5 * n_cb) return lc;
+  }
+  return 0;
+}
+constexpr int kRegWarps = 4;
+__device__ __forceinline__ int reg_group(int lc) {
+  return (blockIdx.x * kRegWarps + (threadIdx.x >> 5)) * (32 >> lc) + ((threadIdx.x & 31) >> lc);
+}
+__device__ __forceinline__ int reg_channel(int lc) { return ((blockIdx.y << lc) + (threadIdx.x & ((1 << lc) - 1))) * 8; }
+inline dim3 reg_grid(long long n_groups, int n_cb, int lc) {
+  const long long per_block = static_cast<long long>(kRegWarps) * (32 >> lc);
+  return dim3(static_cast<unsigned>((n_groups + per_block - 1) / per_block), static_cast<unsigned>((n_cb + (1 << lc) - 1) >> lc));
+}
+
 // The same packing without shared memory, for images whose padded pixel count stays below the range of
 // the reciprocal divisions: a thread takes one group of 8 padded pixels and 8 channels, reads the
 // 8 + KW - 1 input pixels the group's taps touch (16 bytes = 8 channels each; zeros outside the image),
 // transposes them in registers (two byte permutes per output word) and writes, for every tap and every
-// one of its channels, the 8 pixels as one 16-byte store.  Lanes run along the pixel groups, so a warp's
-// store instruction covers 512 contiguous bytes of one plane row; the loads of a warp touch 32 pixels,
-// whose other channels neighbouring blocks (blockIdx.y) pick up from L2.  Threads past the last image
-// zero the planes' tails.  grid (ceil(plane_ld / 8 / 128), C / 8), block 128.
+// one of its channels, the 8 pixels as one 16-byte store.  Bound by the writes of KW planes.  Threads past the
+// last image zero the planes' tails.  grid reg_grid(plane_ld / 8, C / 8, lc), block 128.
 template <int KW>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * kRegWarps)
 conv_pack_input_reg_kernel(const uint16_t* __restrict__ x, int H, int W, int C, int kh, int Hp, int Wp,
-                           int n_groups, int n_groups_ld, uint32_t mul_wp8, uint32_t mul_hp,
+                           int n_groups, int n_groups_ld, uint32_t mul_wp8, uint32_t mul_hp, int lc,
                            uint16_t* __restrict__ planes, long long plane_ld) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;   // group of 8 padded pixels
-  if (g >= n_groups_ld) return;
-  const int c0 = blockIdx.y * 8;
+  const int g = reg_group(lc);   // group of 8 padded pixels
+  const int c0 = reg_channel(lc);
+  if (g >= n_groups_ld || c0 >= C) return;
   const long long m0 = static_cast<long long>(g) << 3;
   if (g >= n_groups) {
 #pragma unroll
@@ -213,15 +236,14 @@ conv_unpack_output_kernel(const uint16_t* __restrict__ ct, long long ldc, int B,
 }
 
 // The unpacking without shared memory: a thread takes one group of 8 padded pixels and 8 output channels,
-// reads the 8 channel rows (16 bytes each, a warp 512 contiguous bytes per row), transposes in registers
-// and writes the pixels that exist as 16-byte pieces of their NHWC rows (the neighbouring channel blocks
-// complete the sectors in L2).  grid (ceil(m_pad / 8 / 128), N / 8), block 128.
-__global__ void __launch_bounds__(128)
+// reads the 8 channel rows (16 bytes each), transposes in registers and writes the pixels that exist as
+// 16-byte pieces of their NHWC rows; lanes as in the packing.  grid reg_grid(m_pad / 8, N / 8, lc), block 128.
+__global__ void __launch_bounds__(32 * kRegWarps)
 conv_unpack_output_reg_kernel(const uint16_t* __restrict__ ct, long long ldc, int H, int W, int Hp, int Wp, int N,
-                              int n_groups, uint32_t mul_wp8, uint32_t mul_hp, uint16_t* __restrict__ y) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;   // group of 8 padded pixels
-  if (g >= n_groups) return;
-  const int n0 = blockIdx.y * 8;
+                              int n_groups, uint32_t mul_wp8, uint32_t mul_hp, int lc, uint16_t* __restrict__ y) {
+  const int g = reg_group(lc);   // group of 8 padded pixels
+  const int n0 = reg_channel(lc);
+  if (g >= n_groups || n0 >= N) return;
   const int wp8 = Wp >> 3;
   const int row = mul_wp8 ? static_cast<int>(__umulhi(static_cast<uint32_t>(g), mul_wp8)) : g;
   const int x0 = (g - row * wp8) << 3;
@@ -427,12 +449,13 @@ cudaError_t conv_pack_input_launch(const void* x_nhwc, int B, int H, int W, int 
   if (reg_ok) {
     const uint32_t mul_wp8 = Wp / 8 > 1 ? 0xffffffffu / static_cast<uint32_t>(Wp / 8) + 1u : 0u;
     const uint32_t mul_hp = Hp > 1 ? 0xffffffffu / static_cast<uint32_t>(Hp) + 1u : 0u;
-    dim3 grid(static_cast<unsigned>((n_groups_ld + 127) / 128), C / 8);
+    const int lc = lanes_over_channels(C / 8);
+    const dim3 grid = reg_grid(n_groups_ld, C / 8, lc);
     const uint16_t* xin = static_cast<const uint16_t*>(x_nhwc);
     uint16_t* pl = static_cast<uint16_t*>(planes);
 #define TS_PACK(KW)                                                                                             \
-  conv_pack_input_reg_kernel<KW><<<grid, 128, 0, stream>>>(xin, H, W, C, kh, Hp, Wp, static_cast<int>(n_groups), \
-                                                           static_cast<int>(n_groups_ld), mul_wp8, mul_hp, pl, plane_ld)
+  conv_pack_input_reg_kernel<KW><<<grid, 32 * kRegWarps, 0, stream>>>(xin, H, W, C, kh, Hp, Wp, static_cast<int>(n_groups), \
+                                                                      static_cast<int>(n_groups_ld), mul_wp8, mul_hp, lc, pl, plane_ld)
     switch (kw) {
       case 1: TS_PACK(1); break;
       case 3: TS_PACK(3); break;
@@ -463,10 +486,10 @@ cudaError_t conv_unpack_output_launch(const void* ct, long long ldc, int B, int 
   if ((N % 8) == 0 && N / 8 <= 65535 && n_groups < (1LL << 31) && n_groups * std::max<long long>(Wp / 8, Hp) < (1LL << 32)) {
     const uint32_t mul_wp8 = Wp / 8 > 1 ? 0xffffffffu / static_cast<uint32_t>(Wp / 8) + 1u : 0u;
     const uint32_t mul_hp = Hp > 1 ? 0xffffffffu / static_cast<uint32_t>(Hp) + 1u : 0u;
-    dim3 rgrid(static_cast<unsigned>((n_groups + 127) / 128), N / 8);
-    conv_unpack_output_reg_kernel<<<rgrid, 128, 0, stream>>>(static_cast<const uint16_t*>(ct), ldc, H, W, Hp, Wp, N,
-                                                             static_cast<int>(n_groups), mul_wp8, mul_hp,
-                                                             static_cast<uint16_t*>(y_nhwc));
+    const int lc = lanes_over_channels(N / 8);
+    conv_unpack_output_reg_kernel<<<reg_grid(n_groups, N / 8, lc), 32 * kRegWarps, 0, stream>>>(
+        static_cast<const uint16_t*>(ct), ldc, H, W, Hp, Wp, N, static_cast<int>(n_groups), mul_wp8, mul_hp, lc,
+        static_cast<uint16_t*>(y_nhwc));
     return cudaGetLastError();
   }
   dim3 grid((H + kPackRows - 1) / kPackRows, B, (N + kPackCh - 1) / kPackCh);

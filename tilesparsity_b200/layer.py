@@ -65,7 +65,7 @@ class TWLayer:
             self._nn, nn = _i32(tiles.kept_n)
             check(lib.ts_layer_set_tiles(self._h, tiles.n_tiles, kp, kk, npp, nn, _lib.TS_INDEX_ABSOLUTE))
         self._desc = _lib.fast().layer_desc(self._h.value, self.K, self.N, int(self.dtype == torch.bfloat16),
-                                            self.device.index, int(len(np.unique(tiles.kept_n)) == self.N))
+                                            self.device.index, int(np.bincount(tiles.kept_n, minlength=self.N).all()))
 
     # ------------------------------------------------------------------ construction
     @classmethod

@@ -49,14 +49,15 @@ __device__ __forceinline__ int bound_of(const MaskGroup& g, const MaskLayer& L, 
 // Column norms: sqrt(sum_k score[k][n]^2 in row order) / K
 // ---------------------------------------------------------------------------------------------
 // The sum of one column is a chain of K dependent additions (four cycles each: 10 us for 4608 rows), so all
-// that counts is that nothing else slows the chain down: a block owns 32 columns, all four warps keep three
-// slabs of 64 rows in flight (4-byte cp.async, any alignment), and one warp walks the slab that has landed
-// with 16 values in registers ahead of the additions.
-constexpr int kColsPerBlock = 32, kColRows = 64, kColSlabs = 4;
+// that counts is that nothing else slows the chain down: a block owns 32 columns, all four warps keep five
+// slabs of 64 rows in flight (16-byte cp.async where the rows allow it; with 4-byte ones the warp that adds spent most
+// of its time issuing its share of them), and one warp walks the slab that has landed with the next 16 values in
+// registers ahead of the additions.  13 kernels of a VGG16-shaped network: 82 -> 36 us.
+constexpr int kColsPerBlock = 32, kColRows = 64, kColSlabs = 6;
 
 __global__ void __launch_bounds__(128)
 group_col_norms_kernel(const __grid_constant__ MaskGroup g, float* __restrict__ out) {
-  __shared__ float slab[kColSlabs][kColRows][kColsPerBlock];
+  __shared__ __align__(16) float slab[kColSlabs][kColRows][kColsPerBlock];
   const int l = find_layer(g, blockIdx.x, [](const MaskLayer& m) { return m.col_blk0; });
   const MaskLayer& L = layer_at(g, l);
   const int n0 = (blockIdx.x - L.col_blk0) * kColsPerBlock;
@@ -64,8 +65,15 @@ group_col_norms_kernel(const __grid_constant__ MaskGroup g, float* __restrict__ 
   const bool col_ok = n0 + c < L.N;
   const int K = L.K, n_slabs = (K + kColRows - 1) / kColRows;
   const float* src = L.score + n0 + c;
+  const bool vec = (L.ld % 4) == 0 && (reinterpret_cast<uintptr_t>(L.score) & 15u) == 0 && n0 + kColsPerBlock <= L.N;
   auto fetch = [&](int s) {
-    if (s < n_slabs && col_ok) {
+    if (s < n_slabs && vec) {
+#pragma unroll
+      for (int i = 0; i < kColRows / 16; ++i) {        // four rows of 8 x 16 bytes per warp
+        const int r = (w + i * 4) * 4 + (c >> 3), k = s * kColRows + r;
+        if (k < K) cp_async_16_full(smem_u32(&slab[s % kColSlabs][r][(c & 7) * 4]), L.score + static_cast<long long>(k) * L.ld + n0 + (c & 7) * 4);
+      }
+    } else if (s < n_slabs && col_ok) {
 #pragma unroll
       for (int i = 0; i < kColRows / 4; ++i) {
         const int r = w + i * 4, k = s * kColRows + r;
@@ -78,7 +86,7 @@ group_col_norms_kernel(const __grid_constant__ MaskGroup g, float* __restrict__ 
     cp_async_commit();
   };
   for (int s = 0; s < kColSlabs - 1; ++s) fetch(s);
-  float acc = 0.0f;
+  float acc = 0.0f;                        // (a square added to +0 is that square)
   for (int s = 0; s < n_slabs; ++s) {
     cp_async_wait_group<kColSlabs - 2>();
     __syncthreads();                       // slab s has landed; slab s - 1 has been consumed
@@ -87,16 +95,20 @@ group_col_norms_kernel(const __grid_constant__ MaskGroup g, float* __restrict__ 
       const int rows = min(kColRows, K - s * kColRows);
       const float(*row)[kColsPerBlock] = slab[s % kColSlabs];
       int r = 0;
-      if (s == 0) {                        // the first square is the sum, not added to a zero
-        acc = __fmul_rn(row[0][c], row[0][c]);
-        r = 1;
-      }
-      for (; r + 16 <= rows; r += 16) {
-        float x[16];
+      if (rows == kColRows) {              // the next 16 values are read while these are added
+        float x[2][16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = row[r + i][c];
+        for (int i = 0; i < 16; ++i) x[0][i] = row[i][c];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc = __fadd_rn(acc, __fmul_rn(x[i], x[i]));
+        for (int b = 0; b < kColRows / 16; ++b) {
+          if (b + 1 < kColRows / 16) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[(b + 1) & 1][i] = row[(b + 1) * 16 + i][c];
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc = __fadd_rn(acc, __fmul_rn(x[b & 1][i], x[b & 1][i]));
+        }
+        r = kColRows;
       }
       for (; r < rows; ++r) acc = __fadd_rn(acc, __fmul_rn(row[r][c], row[r][c]));
     }
@@ -119,7 +131,8 @@ __device__ __forceinline__ float value_of(uint32_t k) { return __uint_as_float((
 // range spreads values that share their leading bits over the bins, so the shared-memory atomics rarely
 // meet); every block adds up all blocks' histograms through distributed shared memory and makes the same
 // choice, so nothing is sent back.  Then NumPy's rank arithmetic and _lerp, every step one IEEE operation in
-// the type NumPy would use (wide: q is a NumPy float64).  18432 values: PCT_SMALL us; 115 Ki: PCT_BIG us.
+// the type NumPy would use (wide: q is a NumPy float64).  18432 values: 23 us; 115 Ki: 25 us
+// (what the passes wait for is each other: with the keys in registers and all remote reads in flight it was 26).
 constexpr int kPctBins = 2048;
 
 __global__ void __launch_bounds__(1024)
@@ -518,17 +531,27 @@ group_apply_kernel(const __grid_constant__ MaskGroup g, const float* __restrict_
     if (one_tile) {
       on = static_cast<double>(v[static_cast<long long>(n0 / g.G) * L.K + k]) > limit ? 0x01010101u : 0u;
       out[0] = out[1] = out[2] = out[3] = on;
-    }
+    } else if (tile_of_col && vec && ((L.col0 + n0) & 15) == 0 && tile_of_col[L.col0 + n0] == tile_of_col[L.col0 + n0 + 15]) {
+      // (tile numbers ascend with the column: all 16 in one tile, their flags in one load)
+      if (static_cast<double>(v[static_cast<long long>(tile_of_col[L.col0 + n0]) * L.K + k]) > limit) {
+        const uint4 kept = __ldg(reinterpret_cast<const uint4*>(col_keep + L.col0 + n0));
+        out[0] = kept.x;
+        out[1] = kept.y;
+        out[2] = kept.z;
+        out[3] = kept.w;
+      }
+    } else {
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      if (!one_tile && n0 + e < n1) {
-        const int t = tile_of_col ? tile_of_col[L.col0 + n0 + e] : (n0 + e) / g.G;
-        if (t != tile) {
-          tile = t;
-          on = static_cast<double>(v[static_cast<long long>(t) * L.K + k]) > limit ? 1u : 0u;
+      for (int e = 0; e < 16; ++e) {
+        if (n0 + e < n1) {
+          const int t = tile_of_col ? tile_of_col[L.col0 + n0 + e] : (n0 + e) / g.G;
+          if (t != tile) {
+            tile = t;
+            on = static_cast<double>(v[static_cast<long long>(t) * L.K + k]) > limit ? 1u : 0u;
+          }
+          const uint32_t bit = col_keep ? (on & col_keep[L.col0 + n0 + e]) : on;
+          out[e >> 2] |= bit << (8 * (e & 3));
         }
-        const uint32_t bit = col_keep ? (on & col_keep[L.col0 + n0 + e]) : on;
-        out[e >> 2] |= bit << (8 * (e & 3));
       }
     }
     uint8_t* dst = L.mask + static_cast<long long>(k) * L.ld_mask + n0;

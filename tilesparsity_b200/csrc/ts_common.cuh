@@ -91,7 +91,7 @@ struct EpilogueArgs {
   // stores issued by one thread, like the local copy, instead of 16-byte stores from every lane.
   const CUtensorMap* peer_maps;
   // fp32 partial sums of split-K units: scratch[row][m], row pitch scratch_ld elements, and a tensor
-  // map over it in global memory (box 32 floats x 128 rows, 128-byte swizzle) for the units' TMA stores
+  // map over it in global memory (box 32 floats x 32 rows, 128-byte swizzle) for the units' TMA stores
   float* scratch;
   long long scratch_ld;
   const CUtensorMap* scratch_map;

@@ -267,6 +267,14 @@ int ts_plan_schedule(int n_tiles, const int32_t* k_counts, const int32_t* n_coun
                      int unit_rows, int* unit_rows_out, int* n_ctas_out, int* n_units_out, int32_t* units_out,
                      int max_units, float* cta_cost_out);
 
+/* For a layer whose tiles keep more than its mask does, with weights of zero there (a TEW mask as wider tiles):
+ * after ts_masked_gemm(layer, M, At, lda, Ct, ldc, alpha, 0) it computes the NaNs of Ct again over the mask's entries
+ * alone, so that an infinite or NaN activation reaches the columns that keep its row and no others.  Nothing is
+ * written when the product is finite.  kept_bits_dev [N][bits_ld] bytes on the device, bits_ld >= ceil(K / 8): bit
+ * k % 8 of byte k / 8 of row n is mask[k][n].  No reference counterpart (its TEW masks multiply densely). */
+int ts_layer_mask_nonfinite(ts_layer_t* layer, int M, const void* At_dev, int64_t lda, void* Ct_dev, int64_t ldc, float alpha,
+                            const uint8_t* kept_bits_dev, int64_t bits_ld, void* stream);
+
 /* Element-wise residual of a TEW mask as a sparse term, applied after ts_masked_gemm:
  *     Ct[n][m] = (col_written[n] ? Ct[n][m] : 0) + alpha * sum_p val[p] * At[row_idx[p]][m]
  * over the non-zeros p in col_ptr[n] .. col_ptr[n+1] of column n (device arrays; val is 16-bit in

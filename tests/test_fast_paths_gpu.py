@@ -283,3 +283,37 @@ def test_retiling_reuses_memory_soundly():
             assert _rel(layer.masked_gemm(x), Wm.t() @ x.double()) <= TOL[torch.float16]
     layer.check()
     layer.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("algo,K,N,M,alpha", [
+    ("tw1m", 256, 384, 64, 1.0),        # full tiles
+    ("tw2m", 250, 300, 1032, 0.5),      # pruned columns, K no multiple of eight, a second block of batch rows
+    ("tw1m", 4096, 128, 64, 1.0),       # long chains: split-K
+    ("tw1m", 256, 8, 8, -2.0),          # one tile of eight columns
+])
+def test_tew_keeps_non_finite_activations_to_the_columns_that_keep_their_rows(algo, K, N, M, alpha, dtype):
+    """Infinities and NaN in the activations: every output is what the mask's own entries give (an infinity of that
+    sign, NaN where they clash, a finite sum where the column keeps no such row)."""
+    from tilesparsity_b200 import TEWLayer, build_mask
+    g = torch.Generator("cuda").manual_seed(K + N)
+    W = torch.randn((K, N), device="cuda", generator=g) * 0.05
+    res = build_mask(algo, [W.abs()], 75.0, 128, 1.5, want_residual=True)
+    layer = TEWLayer(W, res.tiles[0], res.residuals[0], dtype)
+    kept = res.masks[0] | res.residuals[0]
+    x = torch.randn((K, M), device="cuda", generator=g).to(dtype)
+    inf = float("inf")
+    for i, (k, m, v) in enumerate([(7, 3, inf), (100, 3, -inf), (101, 5, float("nan")), (K - 1, M - 1, -inf), (0, 0, inf), (3, 0, inf)]):
+        x[k, m] = v
+    ref = torch.zeros((N, M), dtype=torch.float64, device="cuda")
+    Wd, xd = W.to(dtype).double(), x.double()
+    for n in range(N):
+        ref[n] = alpha * (Wd[kept[:, n], n] @ xd[kept[:, n]])
+    for out in (None, torch.full((N, M), 7.0, dtype=dtype, device="cuda")):
+        got = layer.masked_gemm(x, out=out, alpha=alpha).double()
+        assert torch.equal(got.isnan(), ref.isnan())
+        assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got[ref.isinf()], ref[ref.isinf()])
+        ok = ref.isfinite()
+        assert 0 < int((~ok).sum()) < ref.numel()
+        assert float((got[ok] - ref[ok]).norm() / ref[ok].norm()) <= TOL[dtype]
+    layer.close()

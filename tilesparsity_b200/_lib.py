@@ -66,6 +66,7 @@ SIGNATURES = {
     "ts_layer_row_output": (C.c_int, [_vp, C.c_int, C.POINTER(C.c_int)]),
     "ts_masked_gemm_rows": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp, C.c_int64, C.POINTER(Epilogue), _vp]),
     "ts_layer_zero_pruned": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp]),
+    "ts_layer_mask_nonfinite": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp, C.c_int64, C.c_float, _vp, C.c_int64, _vp]),
     "ts_masked_gemm_simt": (C.c_int, [_vp, C.c_int, _vp, C.c_int64, _vp, C.c_int64, C.c_float, C.c_float, _vp]),
     "ts_masked_gemm_host": (C.c_int, [_vp, C.c_int, _vp, _vp, C.c_float, C.c_float, _vp]),
     "ts_masked_gemm_host_async": (C.c_int, [_vp, C.c_int, _vp, _vp, C.c_float, C.c_float, _vp]),

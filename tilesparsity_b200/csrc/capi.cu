@@ -1180,6 +1180,20 @@ int ts_layer_zero_pruned(ts_layer_t* l, int M, void* Ct, int64_t ldc, void* stre
   return TS_OK;
 }
 
+int ts_layer_mask_nonfinite(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc, float alpha,
+                            const uint8_t* kept_bits, int64_t bits_ld, void* stream) {
+  if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
+  std::lock_guard<std::mutex> lock(l->mu);
+  int rc = check_gemm_args(l, M, At, lda, Ct, ldc);
+  if (rc != TS_OK) return rc;
+  if (!kept_bits || bits_ld < (l->K + 7) / 8) {
+    return fail(TS_ERR_INVALID, "kept bits are NULL or bits_ld=%lld is smaller than K / 8", (long long)bits_ld);
+  }
+  TS_CUDA(ts::tew_finite_launch(l->dtype, l->d_tiles, l->n_tiles, l->d_wp, l->ldw, kept_bits, bits_ld, At, lda, Ct, ldc, M, alpha,
+                                static_cast<cudaStream_t>(stream)));
+  return TS_OK;
+}
+
 int ts_masked_gemm_ex(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct, int64_t ldc,
                       const ts_epilogue_t* epi, void* stream) {
   return run_masked_gemm(l, M, At, lda, Ct, ldc, epi, stream, 0);

@@ -98,10 +98,11 @@ bool read_float(PyObject* o, float* out) {
   return true;
 }
 
-// masked_gemm(layer, At, out | None, alpha, beta, bias | None, act) -> out
+// masked_gemm(layer, At, out | None, alpha, beta, bias | None, act[, kept bits]) -> out; with the mask's bits (uint8 [N,
+// K / 8]) ts_layer_mask_nonfinite follows
 PyObject* py_masked_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 7) return fail_value("masked_gemm takes 7 arguments");
+  if (n != 7 && n != 8) return fail_value("masked_gemm takes 7 or 8 arguments");
   if (a[0] == Py_None) return fail_code(ts_masked_gemm_ex(nullptr, 0, nullptr, 0, nullptr, 0, nullptr, nullptr));   // a closed layer
   Layer* l = layer_of(a[0]);
   if (!l) return nullptr;
@@ -138,8 +139,18 @@ PyObject* py_masked_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return fail_value("out must be an [N, M] tensor of the layer's dtype with M contiguous");
     }
   }
+  const uint8_t* bits = nullptr;
+  int64_t bits_ld = 0;
+  if (n == 8) {
+    if (!THPVariable_Check(a[7])) return fail_value("the mask's bits must be a tensor");
+    bits = static_cast<const uint8_t*>(THPVariable_Unpack(a[7]).data_ptr());
+    bits_ld = THPVariable_Unpack(a[7]).stride(0);
+  }
   const int rc = unlocked([&] {
-    return ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out->data_ptr(), out->stride(0), &ep, stream);
+    const int r = ts_masked_gemm_ex(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out->data_ptr(), out->stride(0), &ep, stream);
+    if (r != TS_OK || !bits) return r;
+    return ts_layer_mask_nonfinite(l->h, static_cast<int>(M), At.data_ptr(), At.stride(0), out->data_ptr(), out->stride(0), ep.alpha, bits,
+                                   bits_ld, stream);
   });
   if (rc != TS_OK) return fail_code(rc);
   if (out == &fresh) return THPVariable_Wrap(std::move(fresh));

@@ -62,6 +62,12 @@ cudaError_t pack_weights_launch(int w_dtype, int out_dtype, const void* W, long 
 // Ct[rows[i]][0 .. M) = 0 for n_rows rows of a 16-bit matrix (pack.cu).
 cudaError_t zero_rows_launch(const int* rows, int n_rows, void* Ct, long long ldc, int M, cudaStream_t stream);
 
+// Takes back what a non-finite activation does to a TEW layer's widened tiles (tew_finite.cu): bits[n] holds one
+// bit per row of W, set where the mask keeps (row, n).
+cudaError_t tew_finite_launch(int dtype, const TileDesc* tiles, int n_tiles, const void* Wp, long long ldw, const uint8_t* bits,
+                              long long bits_ld, const void* At, long long lda, void* Ct, long long ldc, int M, float alpha,
+                              cudaStream_t stream);
+
 // Sparse residual term (residual.cu): Ct[n][m] = (col_written[n] ? Ct[n][m] : 0) + alpha * sum over the
 // non-zeros p of column n of val[p] * At[row_idx[p]][m].  col_written may be nullptr (all written).
 cudaError_t residual_spmm_launch(int dtype, const int* col_ptr, const int* row_idx, const void* val,

@@ -301,6 +301,13 @@ def _tew_structure(tiles: TileSet, residual: torch.Tensor):
     return total, TileSet(K, N, tiles.G, bounds, k_ptr, kept_k.astype(np.int32), n_ptr, cols.astype(np.int32))
 
 
+def _bits_of(mask: torch.Tensor) -> torch.Tensor:
+    """bool [R, C] -> uint8 [R, ceil(C / 8)], element c in bit c % 8 of byte c // 8."""
+    R, Cc = mask.shape
+    m = torch.nn.functional.pad(mask, (0, -Cc % 8)).view(R, -1, 8)
+    return (m * (1 << torch.arange(8, device=mask.device)).to(torch.uint8)).sum(-1, dtype=torch.uint8)
+
+
 class TEWLayer:
     """A TEW layer: the tile-wise part plus single weights outside it, as one masked GEMM.
 
@@ -314,6 +321,8 @@ class TEWLayer:
     single weight in a sparse product 512 bytes: the widened tile is level at one weight per added row and
     ahead with two (1.5 % of the elements put 1.9 into every row of a 128-column tile).  2048 x 4096 at
     6400 rows with 1.5 %: 92 us for the sparse product alone, 86 us for the whole widened layer (149 us with the two parts apart).
+    An infinite or NaN activation reaches the columns that keep its row and no others: what it does to the rest of
+    its tile, whose weights there are zero, is taken back (tew_finite.cu).
     """
 
     def __init__(self, W: torch.Tensor, tiles: TileSet, residual: torch.Tensor, dtype=torch.float16):
@@ -323,13 +332,16 @@ class TEWLayer:
         if self.nnz:
             kept, tiles = _tew_structure(tiles, residual)
             W = torch.where(kept, W, torch.zeros((), dtype=W.dtype, device=W.device))
+            self._bits = _bits_of(kept.t())
         self.tw = TWLayer(tiles, dtype, W.device)
         self.tw.pack(W)
 
     def masked_gemm(self, At: torch.Tensor, out: torch.Tensor | None = None, alpha: float = 1.0) -> torch.Tensor:
         """Ct[N, M] = alpha * (W .* mask_tew)^T @ At[K, M]."""
-        Ct = self.tw.masked_gemm(At, out=out, alpha=alpha)
-        if out is not None and self.nnz:
+        if not self.nnz:
+            return self.tw.masked_gemm(At, out=out, alpha=alpha)
+        Ct = _masked_gemm(self.tw._desc, At, out, alpha, 0.0, None, 0, self._bits)
+        if out is not None:
             # columns without any kept element read as zero in a caller's buffer too
             with torch.cuda.device(self.device):
                 check(lib.ts_layer_zero_pruned(self.tw._h, At.shape[1], C.c_void_p(Ct.data_ptr()), Ct.stride(0),

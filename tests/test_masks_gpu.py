@@ -211,3 +211,61 @@ def test_block_wise_masks_match_reference_golden_up_to_threshold_ties(name):
                 assert a.all() or not a.any()
                 assert np.array_equal(a, b) or near[idx], f"{name}: block ({i}, {j}) differs away from the threshold"
                 idx += 1
+
+
+# ------------------------------------------------------------------------------------------- NaN and infinities
+def _spoiled(seed, shape, share, axis, value):
+    """Normal scores; `value` in one place of `share` of the rows (axis 0) or columns (axis 1)."""
+    g = np.random.Generator(np.random.PCG64(seed))
+    s = np.abs(g.standard_normal(shape, dtype=np.float32))
+    hit = np.flatnonzero(g.random(shape[axis]) < share)
+    at = g.integers(0, shape[1 - axis], len(hit))
+    if axis == 0:
+        s[hit, at] = value
+    else:
+        s[at, hit] = value
+    return s
+
+
+@pytest.mark.parametrize("rows", [2000, 20000])          # one block's percentile, a cluster's
+@pytest.mark.parametrize("share", [0.05, 0.35])          # the rank, at 75 %, below the infinities, and on one
+def test_tw1_infinite_scores_match_oracle(rows, share):
+    """inf - inf makes the threshold NaN where the rank falls on an infinity, and nothing is kept."""
+    from tilesparsity_b200 import build_mask
+    for seed in range(8):
+        s = _spoiled(seed, (rows, 8), share, 0, np.inf)
+        with np.errstate(invalid="ignore"):
+            ref = om.tw1([s], 75.0, 8)[0]
+        res = build_mask("tw1", [s], 75.0, 8)
+        assert np.array_equal(res.masks[0].cpu().numpy(), ref), seed
+        assert ref.any() == (share < 0.25) and np.isnan(res.thresholds[1]) == (share > 0.25)
+
+
+@pytest.mark.parametrize("rows", [2000, 20000])
+@pytest.mark.parametrize("share", [0.05, 0.35])
+def test_tw1_keeps_no_row_with_a_nan(rows, share):
+    """A NaN exceeds no threshold, and a row without one is kept where its norm exceeds the threshold reported."""
+    from tilesparsity_b200 import build_mask
+    for seed in range(8):
+        s = _spoiled(seed, (rows, 8), share, 0, np.nan)
+        norms = np.linalg.norm(s, axis=1) / 8
+        res = build_mask("tw1", [s], 75.0, 8)
+        assert np.array_equal(res.masks[0].cpu().numpy()[:, 0], norms.astype(np.float64) > res.thresholds[1]), seed
+
+
+@pytest.mark.parametrize("shape", [(300, 128), (40, 128), (1500, 1024)])     # a cluster's percentile, one block's, the whole GPU's
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_tew_residual_with_nan_or_infinity(shape, value):
+    """A fifth of the single elements spoiled: an element joins the mask where its value exceeds the threshold
+    reported, so a NaN never does, and nothing does where the rank falls on an infinity (inf - inf)."""
+    from tilesparsity_b200 import build_mask
+    for seed in range(6):
+        g = np.random.Generator(np.random.PCG64(seed))
+        s = np.abs(g.standard_normal(shape, dtype=np.float32))
+        s[g.random(shape) < 0.2] = value
+        tw = build_mask("tw1", [s], 55.0, 128).masks[0].cpu().numpy()
+        res = build_mask("tw1m", [s], 50.0, 128, 5.0, want_residual=True)
+        extra = (np.sqrt(s * s) - tw).astype(np.float64) > res.thresholds[2]
+        assert np.array_equal(res.residuals[0].cpu().numpy(), extra), seed
+        assert np.array_equal(res.masks[0].cpu().numpy(), tw | extra), seed
+        assert np.isnan(res.thresholds[2]) == np.isinf(value)

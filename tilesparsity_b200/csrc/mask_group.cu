@@ -273,7 +273,7 @@ group_percentile_kernel(const float* __restrict__ vals, long long n_static, cons
       break;
     }
     lo += bin << shift;
-    hi = min(hi, lo + ((1u << shift) - 1u));
+    hi = lo + min(hi - lo, (1u << shift) - 1u);     // (no sum that wraps: keys reach 0xffffffff)
   }
   if (ni != pi && count_le < ni + 1 && !have_above) {   // (the same decision in every block)
     unsigned int m = 0xffffffffu;

@@ -317,3 +317,17 @@ def test_tew_keeps_non_finite_activations_to_the_columns_that_keep_their_rows(al
         assert 0 < int((~ok).sum()) < ref.numel()
         assert float((got[ok] - ref[ok]).norm() / ref[ok].norm()) <= TOL[dtype]
     layer.close()
+
+
+def test_an_allocation_that_fails_is_reported_once():
+    """A tile structure that needs 275 GB of packed weights (nothing is allocated) is an error of that call; the next
+    layer's packing and product know nothing of it."""
+    from tilesparsity_b200 import TWLayer, _lib, tiles
+    K, N = 1 << 19, 1 << 18
+    rows = [np.arange(K, dtype=np.int32)] + [np.arange(8, dtype=np.int32)] * (N // 128 - 1)
+    with pytest.raises(_lib.TileSparseError):
+        TWLayer(tiles.tiles_from_lists(K, N, 128, rows), torch.float16, "cuda")
+    layer, W = _layer(64, 128, 16, torch.float16, 3)
+    x = torch.randn((64, 8), device="cuda").half()
+    assert _rel(layer.masked_gemm(x), _dense(W, layer, torch.float16).t() @ x.double()) <= TOL[torch.float16]
+    layer.close()

@@ -21,7 +21,9 @@ namespace {
 thread_local std::string g_last_error;
 }  // namespace
 
-// Records the calling thread's error text and returns `code`; shared by every C-ABI source file.
+// Records the calling thread's error text and returns `code`; shared by every C-ABI source file.  A failed runtime
+// call also stays behind as the thread's last CUDA error; it has been reported here, and the next launch that asks
+// for one must not find it.
 int ts_internal_fail(int code, const char* fmt, ...) {
   char buf[512];
   va_list ap;
@@ -29,6 +31,7 @@ int ts_internal_fail(int code, const char* fmt, ...) {
   vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
   g_last_error = buf;
+  if (code == TS_ERR_CUDA || code == TS_ERR_NOMEM) cudaGetLastError();
   return code;
 }
 #define fail ts_internal_fail

@@ -331,3 +331,27 @@ def test_an_allocation_that_fails_is_reported_once():
     x = torch.randn((64, 8), device="cuda").half()
     assert _rel(layer.masked_gemm(x), _dense(W, layer, torch.float16).t() @ x.double()) <= TOL[torch.float16]
     layer.close()
+
+
+def test_a_retiling_that_fails_leaves_a_layer_without_tiles():
+    """More packed weights than any GPU holds (275 GB; nothing is allocated): the call is an error, and so is every
+    product of the layer after it.  New outputs have pruned columns to clear, whose list is gone with the old tiles."""
+    from tilesparsity_b200 import TWLayer, _lib, tiles
+    K, N = 1 << 19, 1 << 18
+    col = np.ones(N, bool)
+    col[5::1000] = False
+    n_tiles = len(tiles.tile_bounds_from_col_mask(col, 128)) - 1
+    rows = [np.arange(8, dtype=np.int32)] * n_tiles
+    layer = TWLayer(tiles.tiles_from_lists(K, N, 128, rows, col), torch.float16, "cuda")
+    assert layer.stats()["n_tiles"] == n_tiles
+    rows = [np.arange(K, dtype=np.int32)] + rows[1:]
+    with pytest.raises(_lib.TileSparseError):
+        layer.retile(tiles.tiles_from_lists(K, N, 128, rows, col))
+    x = torch.zeros((K, 8), dtype=torch.float16, device="cuda")
+    for out in (None, torch.zeros((N, 8), dtype=torch.float16, device="cuda")):
+        with pytest.raises(_lib.TileSparseError):
+            layer.masked_gemm(x, out=out)
+    assert _lib.lib.ts_layer_zero_pruned(layer._h, 8, out.data_ptr(), 8, None) == 1       # TS_ERR_INVALID
+    torch.cuda.synchronize()
+    assert layer.stats()["n_tiles"] == 0
+    layer.close()

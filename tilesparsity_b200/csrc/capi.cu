@@ -662,10 +662,21 @@ void drop_schedules(ts_layer* l) {
   l->schedules.clear();
 }
 
+// The layer is one without tiles from here on: nothing it keeps may describe lists that are gone.
 void drop_tiles(ts_layer* l) {
   l->d_kept_k = l->d_kept_n = nullptr;
   l->d_tiles = nullptr;
   l->d_wp = nullptr;
+  l->n_tiles = l->n_kept = l->n_pruned = l->max_k = 0;
+  l->wp_rows = l->ldw = 0;
+  l->rows_ok = false;
+  l->tile_k_ptr.clear();
+  l->tile_n_ptr.clear();
+  l->kept_k.clear();
+  l->kept_n.clear();
+  l->k_counts.clear();
+  l->n_counts.clear();
+  l->h_tiles.clear();
   drop_schedules(l);
   l->packed = false;
   l->ct_dirty = true;   // another tile set leaves other places of the staging output unwritten
@@ -925,29 +936,20 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
   }
   TS_CUDA(cudaSetDevice(l->device));
   TS_CUDA(cudaDeviceSynchronize());
-  drop_tiles(l);
-  l->n_tiles = n_tiles;
-  l->tile_k_ptr = kp;
-  l->tile_n_ptr = np;
-  l->kept_k = kk;
-  l->kept_n = nn;
-  l->k_counts = kc;
-  l->n_counts = nc;
-  l->max_k = 0;
-  for (int v : kc) l->max_k = std::max(l->max_k, v);
-  l->ldw = std::max<long long>(64, (l->max_k + 63) / 64 * 64);
-  l->wp_rows = static_cast<long long>(std::max(1, n_tiles)) * 128;
+  drop_tiles(l);   // (what follows may fail; the new structure is installed at the end)
+  int max_k = 0;
+  for (int v : kc) max_k = std::max(max_k, v);
+  const long long ldw = std::max<long long>(64, (max_k + 63) / 64 * 64), wp_rows = static_cast<long long>(std::max(1, n_tiles)) * 128;
   std::vector<char> kept(l->N, 0);
   for (int v : nn) kept[v] = 1;
-  l->n_kept = static_cast<int>(nn.size());
+  const size_t n_kept = nn.size();
   for (int v = 0; v < l->N; ++v) {
     if (!kept[v]) nn.push_back(v);
   }
-  l->n_pruned = static_cast<int>(nn.size()) - l->n_kept;
   size_t bytes = 0;
   const size_t o_k = carve(&bytes, kk.size() * sizeof(int)), o_n = carve(&bytes, nn.size() * sizeof(int)),
                o_tiles = carve(&bytes, n_tiles * sizeof(ts::TileDesc)), upload = bytes,
-               o_wp = carve(&bytes, static_cast<size_t>(l->wp_rows) * l->ldw * 2);
+               o_wp = carve(&bytes, static_cast<size_t>(wp_rows) * ldw * 2);
   if (l->tile_mem.bytes < bytes || l->tile_mem.bytes / 4 > bytes) {
     cudaFree(l->tile_mem.p);
     l->tile_mem = DeviceBlock{};
@@ -955,16 +957,13 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
     if (rc != TS_OK) return rc;
   }
   char* base = static_cast<char*>(l->tile_mem.p);
-  l->d_kept_k = reinterpret_cast<int*>(base + o_k);
-  l->d_kept_n = reinterpret_cast<int*>(base + o_n);
-  l->d_tiles = reinterpret_cast<ts::TileDesc*>(base + o_tiles);
   std::vector<char> host(upload);
   if (!kk.empty()) memcpy(host.data() + o_k, kk.data(), kk.size() * sizeof(int));
   if (!nn.empty()) memcpy(host.data() + o_n, nn.data(), nn.size() * sizeof(int));
   std::vector<ts::TileDesc> td(n_tiles);
   for (int t = 0; t < n_tiles; ++t) {
-    td[t].k_list = l->d_kept_k + kp[t];
-    td[t].n_list = l->d_kept_n + np[t];
+    td[t].k_list = reinterpret_cast<int*>(base + o_k) + kp[t];
+    td[t].n_list = reinterpret_cast<int*>(base + o_n) + np[t];
     td[t].k_count = kc[t];
     td[t].n_count = nc[t];
     td[t].w_row0 = t * 128;
@@ -977,16 +976,35 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
     td[t].pad_ = dense ? 1 : 0;
   }
   // (all columns kept, too: a pruned one would have to be cleared column-wise)
-  l->rows_ok = n_tiles > 0 && l->N % 8 == 0 && l->n_pruned == 0;
+  bool rows_ok = n_tiles > 0 && l->N % 8 == 0 && nn.size() == n_kept;
   for (int t = 0; t < n_tiles; ++t) {
-    if (nc[t] > 0 && (!td[t].pad_ || nn[np[t]] % 8 != 0)) l->rows_ok = false;
+    if (nc[t] > 0 && (!td[t].pad_ || nn[np[t]] % 8 != 0)) rows_ok = false;
   }
   if (n_tiles > 0) memcpy(host.data() + o_tiles, td.data(), td.size() * sizeof(ts::TileDesc));
   TS_CUDA(cudaMemcpy(base, host.data(), upload, cudaMemcpyHostToDevice));
   TS_CUDA(cudaStreamSynchronize(nullptr));   // (a copy from pageable memory may return before it has landed)
+  int rc = make_weight_tmap(&l->tmap, l->dtype, base + o_wp, wp_rows, ldw);
+  if (rc != TS_OK) return rc;
+  l->d_kept_k = reinterpret_cast<int*>(base + o_k);
+  l->d_kept_n = reinterpret_cast<int*>(base + o_n);
+  l->d_tiles = reinterpret_cast<ts::TileDesc*>(base + o_tiles);
   l->d_wp = reinterpret_cast<uint16_t*>(base + o_wp);
-  l->h_tiles = td;
-  return make_weight_tmap(&l->tmap, l->dtype, l->d_wp, l->wp_rows, l->ldw);
+  l->n_tiles = n_tiles;
+  l->n_kept = static_cast<int>(n_kept);
+  l->n_pruned = static_cast<int>(nn.size() - n_kept);
+  l->max_k = max_k;
+  l->wp_rows = wp_rows;
+  l->ldw = ldw;
+  l->rows_ok = rows_ok;
+  nn.resize(n_kept);
+  l->tile_k_ptr = std::move(kp);
+  l->tile_n_ptr = std::move(np);
+  l->kept_k = std::move(kk);
+  l->kept_n = std::move(nn);
+  l->k_counts = std::move(kc);
+  l->n_counts = std::move(nc);
+  l->h_tiles = std::move(td);
+  return TS_OK;
 }
 
 int ts_layer_pack_weights(ts_layer_t* l, const void* W_dev, int64_t ldw_in, int w_dtype, void* stream) {
@@ -1175,6 +1193,7 @@ extern "C" {
 int ts_layer_zero_pruned(ts_layer_t* l, int M, void* Ct, int64_t ldc, void* stream) {
   if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
   if (M < 0 || (M % 8) != 0) return fail(TS_ERR_INVALID, "M=%d must be a non-negative multiple of 8", M);
+  if (!l->d_kept_n) return fail(TS_ERR_INVALID, "layer has no tiles (call ts_layer_set_tiles)");
   if (M == 0 || l->n_pruned == 0) return TS_OK;
   if (!Ct || (reinterpret_cast<uintptr_t>(Ct) & 15u) || ldc < M || (ldc % 8) != 0) {
     return fail(TS_ERR_INVALID, "Ct must be non-NULL and 16-byte aligned, ldc=%lld a multiple of 8 and >= M=%d", (long long)ldc, M);

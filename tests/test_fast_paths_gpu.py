@@ -2,6 +2,7 @@
 changes form.  GEMM results against float64 products of the same 16-bit inputs: the fp32 accumulation over K <= 3072
 rounds far below the 16-bit result, whose half unit is 2^-11 (fp16) or 2^-8 (bf16) of a value; TOL below is four
 times that, as a 2-norm ratio."""
+import ctypes as C
 import threading
 
 import numpy as np
@@ -354,4 +355,48 @@ def test_a_retiling_that_fails_leaves_a_layer_without_tiles():
     assert _lib.lib.ts_layer_zero_pruned(layer._h, 8, out.data_ptr(), 8, None) == 1       # TS_ERR_INVALID
     torch.cuda.synchronize()
     assert layer.stats()["n_tiles"] == 0
+    layer.close()
+
+
+@pytest.mark.parametrize("n_streams", [2, 4, 6])          # 6: more than a layer has scratch memory for at a time
+def test_split_k_on_several_streams(n_streams):
+    """A layer whose long tiles are cut into ranges, used on several streams at once with other activations each, a
+    captured graph among them: every product is its own (the ranges' partial sums do not meet)."""
+    from tilesparsity_b200 import _lib
+    K, N, M = 8192, 256, 64
+    layer, W = _layer(K, N, 6000, torch.float16, 21)
+    parts = (C.c_int32 * 2)()
+    counts = (C.c_int32 * 2)(6000, 6000), (C.c_int32 * 2)(128, 128)
+    assert _lib.lib.ts_plan_split(2, *counts, K, M, 148, parts) == 0 and max(parts) > 1
+    xs = [torch.randn((K, M), device="cuda", generator=torch.Generator("cuda").manual_seed(i)).half() for i in range(n_streams)]
+    refs = [layer.masked_gemm(x) for x in xs]
+    Wm = _dense(W, layer, torch.float16)
+    assert all(_rel(r, Wm.t() @ x.double()) <= TOL[torch.float16] for r, x in zip(refs, xs))
+    outs = [[torch.zeros_like(refs[0]) for _ in range(50)] for _ in xs]
+    held = torch.zeros_like(refs[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer.masked_gemm(xs[0], out=held)
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(i):
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                for o in outs[i]:
+                    layer.masked_gemm(xs[i], out=o)
+                    if i == 0:
+                        graph.replay()
+            s.synchronize()
+        except Exception as e:      # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(n_streams)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors
+    assert all(torch.equal(o, r) for os, r in zip(outs, refs) for o in os)
+    assert torch.equal(held, refs[0])
+    layer.check()
     layer.close()

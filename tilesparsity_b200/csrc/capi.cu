@@ -188,6 +188,20 @@ void give_block(std::vector<DeviceBlock>* spare, DeviceBlock* b) {
   *b = DeviceBlock{};
 }
 
+// Where the fp32 partial sums of a split-K schedule's units lie between its two kernels, and a tensor map over them,
+// both in device memory.  Calls on one stream follow one another and share one; calls on different streams may run
+// at the same time, so each stream has its own (up to kScratchStreams; then the one unused for longest changes hands
+// behind a wait for the device).  A captured call cannot allocate: the captures take one that exists for themselves.
+struct Scratch {
+  DeviceBlock mem;             // its own block, or empty: part of the schedule's
+  float* sums = nullptr;
+  CUtensorMap* map = nullptr;
+  bool owned = false, captured = false;
+  unsigned long long stream = 0;   // cudaStreamGetId of the owner
+  unsigned long long used = 0;     // tick of the latest call
+};
+constexpr size_t kScratchStreams = 4;
+
 struct Schedule {
   DeviceBlock mem;             // holds everything below
   ts::WorkItem* d_units = nullptr;
@@ -203,9 +217,9 @@ struct Schedule {
   // their partial sums go to ([scratch_rows][scratch_ld]) and the descriptors for the second pass
   int n_split = 0;
   ts::SplitTile* d_split = nullptr;
-  float* d_scratch = nullptr;
-  long long scratch_ld = 0;
-  CUtensorMap* d_scratch_map = nullptr;   // tensor map over d_scratch, in device memory
+  long long scratch_rows = 0, scratch_ld = 0;
+  std::vector<Scratch> scratch;
+  unsigned long long tick = 0;
   // Tensor maps over the outputs of the latest calls (a program alternates between a few buffers; encoding
   // one takes about as long as the rest of a call's bookkeeping)
   struct OutMap {
@@ -658,7 +672,10 @@ namespace {
 
 // The caller has waited for the device: queued launches may use the schedules' memory until then.
 void drop_schedules(ts_layer* l) {
-  for (auto& kv : l->schedules) give_block(&l->spare, &kv.second.mem);
+  for (auto& kv : l->schedules) {
+    give_block(&l->spare, &kv.second.mem);
+    for (Scratch& c : kv.second.scratch) give_block(&l->spare, &c.mem);
+  }
   l->schedules.clear();
 }
 
@@ -680,6 +697,67 @@ void drop_tiles(ts_layer* l) {
   drop_schedules(l);
   l->packed = false;
   l->ct_dirty = true;   // another tile set leaves other places of the staging output unwritten
+}
+
+// The scratch memory a call on `stream` uses.
+int scratch_for(Schedule* s, cudaStream_t stream, Scratch** out) {
+  ++s->tick;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  TS_CUDA(cudaStreamIsCapturing(stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) {
+    Scratch* c = &s->scratch[0];
+    for (Scratch& o : s->scratch) {
+      if (o.captured) c = &o;
+    }
+    c->captured = true;
+    *out = c;
+    return TS_OK;
+  }
+  unsigned long long id = 0;
+  TS_CUDA(cudaStreamGetId(stream, &id));
+  Scratch *free_one = nullptr, *oldest = nullptr;
+  size_t n = 0;
+  for (Scratch& o : s->scratch) {
+    if (o.captured) continue;
+    if (o.owned && o.stream == id) {
+      o.used = s->tick;
+      *out = &o;
+      return TS_OK;
+    }
+    if (!o.owned) free_one = &o;
+    if (!oldest || o.used < oldest->used) oldest = &o;
+    ++n;
+  }
+  if (!free_one && n >= kScratchStreams) {
+    TS_CUDA(cudaDeviceSynchronize());
+    free_one = oldest;
+  }
+  if (!free_one) {
+    Scratch c;
+    size_t bytes = 0;
+    const size_t o_map = carve(&bytes, sizeof(CUtensorMap)),
+                 o_sums = carve(&bytes, static_cast<size_t>(s->scratch_rows) * s->scratch_ld * sizeof(float));
+    TS_CUDA(cudaMalloc(&c.mem.p, bytes));
+    c.mem.bytes = bytes;
+    c.map = reinterpret_cast<CUtensorMap*>(static_cast<char*>(c.mem.p) + o_map);
+    c.sums = reinterpret_cast<float*>(static_cast<char*>(c.mem.p) + o_sums);
+    CUtensorMap map;
+    int rc = make_scratch_tmap(&map, c.sums, s->scratch_rows, s->scratch_ld);
+    cudaError_t e = rc == TS_OK ? cudaMemcpy(c.map, &map, sizeof(map), cudaMemcpyHostToDevice) : cudaSuccess;
+    if (rc == TS_OK && e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    if (rc != TS_OK || e != cudaSuccess) {
+      cudaFree(c.mem.p);
+      TS_CUDA(e);
+      return rc;
+    }
+    s->scratch.push_back(c);
+    free_one = &s->scratch.back();
+  }
+  free_one->owned = true;
+  free_one->stream = id;
+  free_one->used = s->tick;
+  *out = free_one;
+  return TS_OK;
 }
 
 // Schedule for batch size M over activations whose kept rows are `ld` elements apart (a matrix), or
@@ -757,6 +835,7 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
     build_schedule(vt, at_rows, M, l->forced_unit_rows, l->sm_count, &flat, &s.rounds, &s.grid, &s.n_units,
                    &s.unit_rows, &s.cta_cost, &blocks, &s.blk_stride, &kb0);
     s.n_split = static_cast<int>(st.size());
+    s.scratch_rows = scratch_rows;
     s.scratch_ld = M;
   } else {
     build_schedule(l->h_tiles, at_rows, M, l->forced_unit_rows, l->sm_count, &flat, &s.rounds, &s.grid, &s.n_units,
@@ -784,10 +863,12 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
     memcpy(host.data() + o_blocks, blocks.data(), blocks.size() * sizeof(ts::BlockDesc));
     if (!st.empty()) {
       s.d_split = reinterpret_cast<ts::SplitTile*>(base + o_split);
-      s.d_scratch = reinterpret_cast<float*>(base + o_scratch);
-      s.d_scratch_map = reinterpret_cast<CUtensorMap*>(base + o_map);
+      Scratch first;
+      first.sums = reinterpret_cast<float*>(base + o_scratch);
+      first.map = reinterpret_cast<CUtensorMap*>(base + o_map);
+      s.scratch.push_back(first);
       CUtensorMap smap;
-      rc = make_scratch_tmap(&smap, s.d_scratch, scratch_rows, M);
+      rc = make_scratch_tmap(&smap, first.sums, scratch_rows, M);
       memcpy(host.data() + o_split, st.data(), st.size() * sizeof(ts::SplitTile));
       memcpy(host.data() + o_map, &smap, sizeof(smap));
     }
@@ -1122,9 +1203,12 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   rc = get_schedule(l, M, lda, conv_wp, allow_split, &s);
   if (rc != TS_OK) return rc;
   if (s->n_units == 0) return TS_OK;
-  ep.scratch = s->d_scratch;
-  ep.scratch_ld = s->scratch_ld;
-  ep.scratch_map = s->d_scratch_map;
+  Scratch* scratch = nullptr;
+  if (s->n_split > 0) {
+    rc = scratch_for(s, static_cast<cudaStream_t>(stream), &scratch);
+    if (rc != TS_OK) return rc;
+  }
+  ep.scratch_map = scratch ? scratch->map : nullptr;
   const CUtensorMap* tmap_c = nullptr;
   if (form == ts::kOutNhwc) {
     ep.nhwc_h = nhwc->nhwc_h;
@@ -1181,7 +1265,7 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
                                  early, s->all_dense, form, static_cast<cudaStream_t>(stream)));
   l->wp_fresh = false;
   if (s->n_split > 0) {
-    TS_CUDA(ts::split_reduce_launch(l->dtype, s->d_split, s->n_split, s->d_scratch, s->scratch_ld, Ct, ldc, M,
+    TS_CUDA(ts::split_reduce_launch(l->dtype, s->d_split, s->n_split, scratch->sums, s->scratch_ld, Ct, ldc, M,
                                     ep.beta, ep.bias, ep.act, static_cast<cudaStream_t>(stream)));
   }
   return TS_OK;

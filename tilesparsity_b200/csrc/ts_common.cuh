@@ -90,10 +90,8 @@ struct EpilogueArgs {
   // a tile whose kept columns are consecutive rows of Ct then leaves for every peer as TMA tile
   // stores issued by one thread, like the local copy, instead of 16-byte stores from every lane.
   const CUtensorMap* peer_maps;
-  // fp32 partial sums of split-K units: scratch[row][m], row pitch scratch_ld elements, and a tensor
-  // map over it in global memory (box 32 floats x 32 rows, 128-byte swizzle) for the units' TMA stores
-  float* scratch;
-  long long scratch_ld;
+  // Tensor map, in global memory, over the fp32 partial sums of split-K units (box 32 floats x 32 rows, 128-byte
+  // swizzle) for the units' TMA stores; nullptr: the schedule has none
   const CUtensorMap* scratch_map;
   // Convolutions whose result leaves as NHWC: the image, its padded space (Wp / 8 and Hp) and their reciprocals.
   int nhwc_h, nhwc_w, nhwc_hp, nhwc_wp8;

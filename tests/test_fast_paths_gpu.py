@@ -228,6 +228,21 @@ def test_grouped_masks_match_oracle(algo, sparsity, shapes):
             assert np.array_equal(res.tiles[l].dense_mask(), r), l
 
 
+@pytest.mark.parametrize("algo,sparsity", [("tw1", 75.0), ("tw1", np.float64(60.0)), ("tw2", 50.0), ("tw2", 99.0), ("bert_type8", 30.0)])
+def test_groups_of_more_than_a_million_tile_rows_match_oracle(algo, sparsity):
+    """Beyond what one cluster ranks (2^20 norms): two layers, tiles of 8 columns.  At 99 % the columns that are left make
+    fewer norms than that."""
+    from tilesparsity_b200 import build_mask
+    g = np.random.Generator(np.random.PCG64(77))
+    scores = [np.abs(g.standard_normal(s, dtype=np.float32)) for s in ((900, 8192), (400, 4096))]
+    ref = om.pruning_fun(algo)(scores, sparsity, 8) if algo != "bert_type8" else om.bert_type8(scores, sparsity, 8)
+    res = build_mask(algo, [torch.from_numpy(s).cuda() for s in scores], sparsity, 8)
+    for l, (m, r) in enumerate(zip(res.masks, ref)):
+        r = np.asarray(r, dtype=bool)
+        assert np.array_equal(m.cpu().numpy(), r), l
+        assert np.array_equal(res.tiles[l].dense_mask(), r), l
+
+
 @pytest.mark.parametrize("B,H,W,cin,cout,kh,kw,algo", [
     (2, 5, 7, 16, 40, 3, 3, "tw1"),        # one narrow tile; two blocks of 8 channels in, five out
     (3, 14, 14, 72, 256, 3, 3, "tw1"),     # nine blocks of channels in: no lane layout but one or two fits

@@ -303,7 +303,8 @@ int read_thresholds(const Scratch& sc, int slot, double* out, cudaStream_t s) {
   return TS_OK;
 }
 
-// One cluster of eight blocks is faster than eleven launches over the whole GPU up to about this many values.
+// One cluster of eight blocks is faster than eleven launches over the whole GPU up to about this many values (tw1 of
+// 4096 rows, tiles of 8 columns: 103 against 134 us a call at 2^17 norms, 653 and 650 at 2^20, 2204 and 2117 at 2^21).
 constexpr long long kGroupSelect = 1 << 20;
 
 // Row stage of the modes group_stages does not serve: norms of all tile-rows of all layers, a keep flag for
@@ -457,7 +458,7 @@ int row_stage(const std::vector<LayerIn>& L, const std::vector<std::vector<int>>
 // The column stage (two_d) and the row stage of the modes that rank all tile-rows of all layers together, in
 // five launches at most and one blocking wait: see mask_group.cu.  q_col / q_row: the stages' percentiles.
 int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col, double q_row, bool wide,
-                 ts_mask_result* res, Arena& arena, cudaStream_t s) {
+                 ts_mask_result* res, Arena& arena, const Scratch& sc, cudaStream_t s) {
   const int nl = static_cast<int>(L.size());
   ts::MaskGroup g;
   memset(&g, 0, sizeof(g));
@@ -525,12 +526,25 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
   if (lists_on_host) list = reinterpret_cast<int*>(host + o_list);
   else TSM_OK(arena.alloc(&list, list_cap));
   TSM_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int), s));
-  uint8_t* col_keep = nullptr;
-  int* tile_of_col = nullptr;
   double* thr_host = reinterpret_cast<double*>(host + o_thr);
   int* nt_host = reinterpret_cast<int*>(host + o_nt);
   int* bounds_host = reinterpret_cast<int*>(host + o_bounds);
   uint8_t* keep_host = reinterpret_cast<uint8_t*>(host + o_keep);
+  // np.percentile of n values, n known on the host, into thr[slot] and thr_host[slot]
+  auto percentile = [&](const float* vals, long long n, double q, int slot) {
+    if (n <= kGroupSelect) {
+      ts::MaskGroup none;
+      memset(&none, 0, sizeof(none));
+      TSM_CUDA(ts::group_percentile_launch(vals, n, n, none, q, wide ? 1 : 0, thr + slot, thr_host + slot, s));
+      return TS_OK;
+    }
+    TSM_OK(percentile_to_device(vals, n, q, wide, false, sc, slot, s));
+    TSM_CUDA(cudaMemcpyAsync(thr + slot, sc.thr + slot, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    TSM_CUDA(cudaMemcpyAsync(thr_host + slot, sc.thr + slot, sizeof(double), cudaMemcpyDefault, s));
+    return TS_OK;
+  };
+  uint8_t* col_keep = nullptr;
+  int* tile_of_col = nullptr;
   if (two_d) {
     float* cn = nullptr;
     int *nt = nullptr, *bounds = nullptr;
@@ -540,13 +554,25 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
     TSM_OK(arena.alloc(&nt, nl));
     TSM_OK(arena.alloc(&bounds, tile_slots));
     TSM_CUDA(ts::group_col_norms_launch(g, col_blocks, cn, s));
-    TSM_CUDA(ts::group_percentile_launch(cn, cols, cols, g, q_col, wide ? 1 : 0, thr, thr_host, s));
+    TSM_OK(percentile(cn, cols, q_col, 0));
     TSM_CUDA(ts::group_columns_launch(g, cn, thr, col_keep, tile_of_col, bounds, nt, keep_host, bounds_host, nt_host, s));
     g.n_tiles = nt;
     g.bounds = bounds;
   }
   TSM_CUDA(ts::group_row_norms_launch(g, norm_blocks, col_keep, norms, s));
-  TSM_CUDA(ts::group_percentile_launch(norms, norms_n, norms_n, g, q_row, wide ? 1 : 0, thr + 1, thr_host + 1, s));
+  if (two_d && norms_n <= kGroupSelect) {     // the number of norms follows from the tiles, on the device
+    TSM_CUDA(ts::group_percentile_launch(norms, norms_n, norms_n, g, q_row, wide ? 1 : 0, thr + 1, thr_host + 1, s));
+  } else {
+    long long n = norms_n;
+    if (two_d) {
+      std::vector<int> nt(nl);
+      TSM_CUDA(cudaMemcpyAsync(nt.data(), nt_host, nl * sizeof(int), cudaMemcpyDefault, s));
+      TSM_CUDA(cudaStreamSynchronize(s));
+      n = 0;
+      for (int l = 0; l < nl; ++l) n += static_cast<long long>(nt[l]) * L[l].K;
+    }
+    TSM_OK(percentile(norms, n, q_row, 1));
+  }
   TSM_CUDA(ts::group_apply_launch(g, recs + static_cast<int>(dense_blocks), norms, thr + 1, col_keep, tile_of_col, cursor, list,
                                   reinterpret_cast<int2*>(host + o_rec), s));
   std::vector<char> copy(staged ? at : 0);
@@ -679,7 +705,7 @@ int build_tw_mask_impl(int mode, int n_layers, const void* const* scores_dev, co
   const int sel = mode == TS_MASK_BERT_PER_TILE ? 1 : (mode == TS_MASK_TOPK_L1 ? 2 : 0);
   do {
     if (sel == 0 && !f64) {
-      rc = group_stages(L, G, two_d, mode == TS_MASK_TW_COLS_ROWS ? g1percent : q, q, wide, res, arena, s);
+      rc = group_stages(L, G, two_d, mode == TS_MASK_TW_COLS_ROWS ? g1percent : q, q, wide, res, arena, sc, s);
       if (rc != TS_OK) break;
     } else {
       for (int l = 0; l < n_layers; ++l) bounds[l] = fixed_bounds(L[l].N, G);

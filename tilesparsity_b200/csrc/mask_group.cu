@@ -364,18 +364,13 @@ __device__ __forceinline__ float square_at(const Run& s, int i) {
   return __fmul_rn(x, x);
 }
 
-// NumPy's pairwise sum of [o, o + n), 8 <= n <= 128, by the 8 lanes of a group (lane j: elements j, j + 8, ...);
-// all loads of the run are in flight before the first addition.
+// NumPy's pairwise sum of [o, o + n), 8 <= n <= 128, by the 8 lanes of a group (lane j: elements j, j + 8, ...).
+// A plain loop: with its 16 loads written out ahead of the additions the kernel takes more registers and fewer blocks
+// run (8192 x 8192 with pruned columns: 227 us, 182 us so; the 13 kernels of a VGG16-shaped network 274 -> 262 us a call).
 __device__ __forceinline__ float leaf8(const Run& s, int o, int n, int j) {
   const int body = n - (n % 8);
-  float x[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) x[i] = i * 8 < body ? square_at(s, o + i * 8 + j) : 0.0f;
-  float r = x[0];
-#pragma unroll
-  for (int i = 1; i < 16; ++i) {
-    if (i * 8 < body) r = __fadd_rn(r, x[i]);
-  }
+  float r = square_at(s, o + j);
+  for (int i = 8; i < body; i += 8) r = __fadd_rn(r, square_at(s, o + i + j));
   r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 1));   // r0+r1, r2+r3, r4+r5, r6+r7
   r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 2));
   r = __fadd_rn(r, __shfl_xor_sync(0xffffffffu, r, 4));

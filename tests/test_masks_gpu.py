@@ -269,3 +269,24 @@ def test_tew_residual_with_nan_or_infinity(shape, value):
         assert np.array_equal(res.residuals[0].cpu().numpy(), extra), seed
         assert np.array_equal(res.masks[0].cpu().numpy(), tw | extra), seed
         assert np.isnan(res.thresholds[2]) == np.isinf(value)
+
+
+def test_scores_with_a_dimension_of_one_element():
+    """Views whose size-1 dimension has another stride than a fresh tensor's (a transposed [1, K] weight): the masks of
+    their copies."""
+    from tilesparsity_b200 import _lib, build_mask
+    g = torch.Generator("cuda").manual_seed(4)
+    row, one = torch.rand((1, 300), device="cuda", generator=g), torch.rand((1, 1), device="cuda", generator=g)
+    wide = torch.rand((300, 7), device="cuda", generator=g)
+    for view in (row.t(), wide[:, 3:4], wide.as_strided((300, 1), (7, 5)), one.expand(300, 1), one.as_strided((300, 1), (0, 9)),
+                 one.as_strided((1, 1), (0, 0))):
+        if view.stride(0) == 0 and view.stride(1) == 1:      # an expanded column: refused, as before
+            with pytest.raises(_lib.TileSparseError):
+                build_mask("tw1", [view], 75.0, 128)
+            continue
+        copy = torch.empty_strided(view.shape, (view.shape[1], 1), device="cuda").copy_(view)
+        got, want = build_mask("tw1", [view], 75.0, 128), build_mask("tw1", [copy], 75.0, 128)
+        assert torch.equal(got.masks[0], want.masks[0]) and got.thresholds[1] == want.thresholds[1]
+    for empty in (torch.empty((0, 5), device="cuda").t(), torch.empty((5, 0), device="cuda").t()):
+        with pytest.raises(_lib.TileSparseError):
+            build_mask("tw1", [empty], 75.0, 128)

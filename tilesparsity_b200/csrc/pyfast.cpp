@@ -17,6 +17,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "../../include/tilesparse.h"
@@ -253,11 +254,16 @@ PyObject* py_build_mask(PyObject*, PyObject* args) {
     PyObject* o = PyList_GET_ITEM(list, l);
     if (!THPVariable_Check(o)) Py_RETURN_NONE;
     const at::Tensor& t = THPVariable_Unpack(o);
-    if (t.dim() != 2 || t.scalar_type() != at::kFloat || !on_device(t, device) || t.stride(1) != 1) Py_RETURN_NONE;
+    if (t.dim() != 2 || t.scalar_type() != at::kFloat || !on_device(t, device)) Py_RETURN_NONE;
     scores[l] = t.data_ptr();
     K[l] = static_cast<int>(t.size(0));
     N[l] = static_cast<int>(t.size(1));
     ld[l] = t.stride(0);
+    if (t.stride(1) != 1) {
+      // a dimension of one element has any stride, and contiguous() leaves such a tensor as it is
+      if (t.numel() > 0 && (N[l] != 1 || (ld[l] < 1 && K[l] > 1))) Py_RETURN_NONE;
+      ld[l] = std::max<int64_t>(ld[l], N[l]);
+    }
   }
   c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)));
   void* stream = stream_of(device);

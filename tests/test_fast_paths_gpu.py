@@ -415,3 +415,16 @@ def test_split_k_on_several_streams(n_streams):
     assert torch.equal(held, refs[0])
     layer.check()
     layer.close()
+
+
+@pytest.mark.parametrize("K,N,keep,M,col_keep", [(8192, 4096, 4096, 4104, None),      # lists and plan of more than 256 KiB: copied piece by piece
+                                                 (8192, 2048, 4000, 72, 0.9)])        # the lists only, with pruned columns
+def test_large_lists_and_plans(K, N, keep, M, col_keep):
+    layer, W = _layer(K, N, keep, torch.float16, 31, col_keep)
+    x = torch.randn((K, M), device="cuda", generator=torch.Generator("cuda").manual_seed(M)).half()
+    for _ in range(2):
+        assert _rel(layer.masked_gemm(x), _dense(W, layer, torch.float16).t() @ x.double()) <= TOL[torch.float16]
+        layer.retile(layer.tiles)
+        layer.pack(W)
+    layer.check()
+    layer.close()

@@ -9,6 +9,7 @@
 #include <cstring>
 #include <list>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <queue>
 #include <string>
@@ -179,6 +180,31 @@ int take_block(std::vector<DeviceBlock>* spare, size_t bytes, DeviceBlock* out) 
   TS_CUDA(e);
   *out = DeviceBlock{p, bytes};
   return TS_OK;
+}
+// Copies host arrays to their places in a device block, and waits until they have landed (a copy from pageable memory may
+// return before).  Small ones go through one buffer: a copy costs some 10 us to start.  Large ones go as they are:
+// gathering the 8 MB plan of a 16384 x 16384 layer first took longer than the copies.
+struct Piece {
+  size_t at;
+  const void* src;
+  size_t bytes;
+};
+constexpr size_t kGatherBytes = 256 << 10;
+cudaError_t upload_pieces(char* base, const Piece* pieces, int n, size_t total) {
+  cudaError_t e = cudaSuccess;
+  if (total <= kGatherBytes) {
+    std::unique_ptr<char[]> host(new char[total]);
+    for (int i = 0; i < n; ++i) {
+      if (pieces[i].bytes > 0) memcpy(host.get() + pieces[i].at, pieces[i].src, pieces[i].bytes);
+    }
+    if (total > 0) e = cudaMemcpy(base, host.get(), total, cudaMemcpyHostToDevice);
+  } else {
+    for (int i = 0; i < n && e == cudaSuccess; ++i) {
+      if (pieces[i].bytes > 0) e = cudaMemcpy(base + pieces[i].at, pieces[i].src, pieces[i].bytes, cudaMemcpyHostToDevice);
+    }
+  }
+  const cudaError_t done = cudaStreamSynchronize(nullptr);
+  return e == cudaSuccess ? done : e;
 }
 constexpr size_t kSpareBlocks = 4;
 void give_block(std::vector<DeviceBlock>* spare, DeviceBlock* b) {
@@ -858,21 +884,20 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
     s.d_units = reinterpret_cast<ts::WorkItem*>(base + o_units);
     s.d_blocks = reinterpret_cast<ts::BlockDesc*>(base + o_blocks);
     s.d_meta = reinterpret_cast<int*>(base + o_meta);
-    std::vector<char> host(upload);
-    memcpy(host.data() + o_units, flat.data(), flat.size() * sizeof(ts::WorkItem));
-    memcpy(host.data() + o_blocks, blocks.data(), blocks.size() * sizeof(ts::BlockDesc));
+    CUtensorMap smap;
     if (!st.empty()) {
       s.d_split = reinterpret_cast<ts::SplitTile*>(base + o_split);
       Scratch first;
       first.sums = reinterpret_cast<float*>(base + o_scratch);
       first.map = reinterpret_cast<CUtensorMap*>(base + o_map);
       s.scratch.push_back(first);
-      CUtensorMap smap;
       rc = make_scratch_tmap(&smap, first.sums, scratch_rows, M);
-      memcpy(host.data() + o_split, st.data(), st.size() * sizeof(ts::SplitTile));
-      memcpy(host.data() + o_map, &smap, sizeof(smap));
     }
-    cudaError_t e = rc == TS_OK ? cudaMemcpy(base, host.data(), upload, cudaMemcpyHostToDevice) : cudaSuccess;
+    const Piece pieces[4] = {{o_units, flat.data(), flat.size() * sizeof(ts::WorkItem)},
+                             {o_blocks, blocks.data(), blocks.size() * sizeof(ts::BlockDesc)},
+                             {o_split, st.data(), st.size() * sizeof(ts::SplitTile)},
+                             {o_map, &smap, st.empty() ? 0 : sizeof(CUtensorMap)}};
+    cudaError_t e = rc == TS_OK ? upload_pieces(base, pieces, 4, upload) : cudaSuccess;
     if (rc == TS_OK && e == cudaSuccess) {
       e = ts::expand_block_meta_launch(s.d_blocks, static_cast<long long>(blocks.size()), s.d_meta, map, nullptr);
       const cudaError_t done = cudaStreamSynchronize(nullptr);
@@ -1038,9 +1063,6 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
     if (rc != TS_OK) return rc;
   }
   char* base = static_cast<char*>(l->tile_mem.p);
-  std::vector<char> host(upload);
-  if (!kk.empty()) memcpy(host.data() + o_k, kk.data(), kk.size() * sizeof(int));
-  if (!nn.empty()) memcpy(host.data() + o_n, nn.data(), nn.size() * sizeof(int));
   std::vector<ts::TileDesc> td(n_tiles);
   for (int t = 0; t < n_tiles; ++t) {
     td[t].k_list = reinterpret_cast<int*>(base + o_k) + kp[t];
@@ -1061,9 +1083,10 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
   for (int t = 0; t < n_tiles; ++t) {
     if (nc[t] > 0 && (!td[t].pad_ || nn[np[t]] % 8 != 0)) rows_ok = false;
   }
-  if (n_tiles > 0) memcpy(host.data() + o_tiles, td.data(), td.size() * sizeof(ts::TileDesc));
-  TS_CUDA(cudaMemcpy(base, host.data(), upload, cudaMemcpyHostToDevice));
-  TS_CUDA(cudaStreamSynchronize(nullptr));   // (a copy from pageable memory may return before it has landed)
+  const Piece pieces[3] = {{o_k, kk.data(), kk.size() * sizeof(int)},
+                           {o_n, nn.data(), nn.size() * sizeof(int)},
+                           {o_tiles, td.data(), td.size() * sizeof(ts::TileDesc)}};
+  TS_CUDA(upload_pieces(base, pieces, 3, upload));
   int rc = make_weight_tmap(&l->tmap, l->dtype, base + o_wp, wp_rows, ldw);
   if (rc != TS_OK) return rc;
   l->d_kept_k = reinterpret_cast<int*>(base + o_k);

@@ -428,3 +428,17 @@ def test_large_lists_and_plans(K, N, keep, M, col_keep):
         layer.pack(W)
     layer.check()
     layer.close()
+
+
+def test_large_plans_are_given_back():
+    """Four plans of 9 MB each: re-tiling the layer gives all but a few megabytes of them back to the device."""
+    layer, W = _layer(4096, 4096, 1024, torch.float16, 41)
+    x = torch.zeros((4096, 16384), dtype=torch.float16, device="cuda")
+    out = torch.zeros((4096, 16384), dtype=torch.float16, device="cuda")
+    for i in range(4):
+        layer.masked_gemm(x[:, :16384 - 8 * i], out=out[:, :16384 - 8 * i])
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    layer.retile(layer.tiles)
+    assert torch.cuda.mem_get_info()[0] - before >= 4 * 9e6 - (8 << 20) - (4 << 20)      # (4 MB: page granularity)
+    layer.close()

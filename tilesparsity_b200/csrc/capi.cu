@@ -206,12 +206,20 @@ cudaError_t upload_pieces(char* base, const Piece* pieces, int n, size_t total) 
   const cudaError_t done = cudaStreamSynchronize(nullptr);
   return e == cudaSuccess ? done : e;
 }
-constexpr size_t kSpareBlocks = 4;
+// What a layer holds back between its re-tilings: the latest blocks, at most this many and this much together (a plan of
+// an encoder layer takes 1.3 MB; one of tens of megabytes takes longer to make than to allocate).
+constexpr size_t kSpareBlocks = 4, kSpareBytes = 8 << 20;
 void give_block(std::vector<DeviceBlock>* spare, DeviceBlock* b) {
   if (!b->p) return;
-  if (spare->size() < kSpareBlocks) spare->push_back(*b);
-  else cudaFree(b->p);
+  spare->push_back(*b);
   *b = DeviceBlock{};
+  size_t bytes = 0;
+  for (const DeviceBlock& s : *spare) bytes += s.bytes;
+  while (spare->size() > kSpareBlocks || bytes > kSpareBytes) {
+    bytes -= spare->front().bytes;
+    cudaFree(spare->front().p);
+    spare->erase(spare->begin());
+  }
 }
 
 // Where the fp32 partial sums of a split-K schedule's units lie between its two kernels, and a tensor map over them,
@@ -653,7 +661,7 @@ struct ts_layer {
   std::vector<int> k_counts, n_counts;
   int max_k = 0;
   DeviceBlock tile_mem;                 // kept rows, kept columns, tiles, packed weights
-  std::vector<DeviceBlock> spare;       // blocks of dropped schedules, at most kSpareBlocks
+  std::vector<DeviceBlock> spare;       // blocks of dropped schedules
   int* d_kept_k = nullptr;
   int* d_kept_n = nullptr;     // kept columns, then (from n_kept on) the columns no tile keeps
   int n_kept = 0, n_pruned = 0;

@@ -17,7 +17,8 @@
  *    M, lda and ldc must be multiples of 8 (the reference rounds its sizes up to 8, basic_nn.cu:1157)
  *    and base pointers 16-byte aligned.
  *  - A layer may be used on several streams and by several host threads; calls that depend on one another are ordered
- *    by the caller, and so are the launches of CUDA graphs that hold the same layer.
+ *    by the caller, and so are the launches of CUDA graphs that hold the same layer.  Such a graph is good until the
+ *    layer is re-tiled, given other unit sizes or destroyed.
  *  - There is no CPU fallback: without a CUDA device every compute call fails with TS_ERR_CUDA.
  */
 #ifndef TILESPARSE_H_

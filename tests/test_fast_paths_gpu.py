@@ -3,6 +3,7 @@ changes form.  GEMM results against float64 products of the same 16-bit inputs: 
 rounds far below the 16-bit result, whose half unit is 2^-11 (fp16) or 2^-8 (bf16) of a value; TOL below is four
 times that, as a 2-norm ratio."""
 import ctypes as C
+import gc
 import threading
 
 import numpy as np
@@ -437,8 +438,72 @@ def test_large_plans_are_given_back():
     out = torch.zeros((4096, 16384), dtype=torch.float16, device="cuda")
     for i in range(4):
         layer.masked_gemm(x[:, :16384 - 8 * i], out=out[:, :16384 - 8 * i])
+    gc.collect()
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
     layer.retile(layer.tiles)
     assert torch.cuda.mem_get_info()[0] - before >= 4 * 9e6 - (8 << 20) - (4 << 20)      # (4 MB: page granularity)
+    layer.close()
+
+
+def test_plans_of_graphs_that_are_gone_are_given_back():
+    """30 shapes of the reference-signature call, a graph each (plans of 15 MB): while the graphs live all plans do, and
+    once they are gone the next new shape leaves no more than the latest 16."""
+    from tilesparsity_b200 import stream_gemm
+    M, N, K, G = 12800, 4096, 2048, 128
+    flat_a, flat_c = (torch.zeros((n * M,), dtype=torch.float16, device="cuda") for n in (K, N))
+    B = torch.zeros((N, K), dtype=torch.float16, device="cuda")
+    lists = torch.zeros((K,), dtype=torch.int32, device="cuda")
+    n = N // G
+
+    def call(m):
+        return stream_gemm.prepare_stream_gemm_nn(m, N, K, 1.0, flat_a[:K * m].view(K, m), B, 0.0, flat_c[:N * m].view(N, m), n, [G] * n, [K] * n,
+                                                  [lists[:G]] * n, [lists] * n, [K * G * t for t in range(n)], [m * G * t for t in range(n)])
+
+    def in_use():      # what is allocated on the device behind torch's back
+        free, total = torch.cuda.mem_get_info()
+        return total - free - torch.cuda.memory_reserved()
+
+    graphs = []
+    gc.collect()
+    start = in_use()
+    for i in range(30):
+        c = call(M - 8 * i)
+        c()
+        torch.cuda.synchronize()
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            c()
+    for g in graphs:
+        g.replay()
+    torch.cuda.synchronize()
+    held = in_use() - start
+    assert held > 30 * 10e6
+    graphs.clear()
+    g = None
+    torch.cuda.synchronize()
+    call(M - 8 * 30)()
+    torch.cuda.synchronize()
+    assert in_use() - start < held * 0.7
+
+
+def test_a_graph_outlives_many_batch_sizes():
+    """A captured product, then more batch sizes than a layer keeps plans for: the graph's plan stays, and its replay is
+    the product of what its input holds by then."""
+    layer, W = _layer(512, 384, 100, torch.float16, 51)
+    x, out = torch.randn((512, 520), device="cuda").half(), torch.zeros((384, 520), dtype=torch.float16, device="cuda")
+    layer.masked_gemm(x, out=out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer.masked_gemm(x, out=out)
+    for i in range(1, 40):
+        layer.masked_gemm(torch.randn((512, 8 * i), device="cuda").half())
+    x.copy_(torch.randn((512, 520), device="cuda").half())
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert _rel(out, _dense(W, layer, torch.float16).t() @ x.double()) <= TOL[torch.float16]
+    layer.check()
+    del graph
     layer.close()

@@ -3,6 +3,7 @@
 #include "../../include/tilesparse.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cmath>
@@ -236,7 +237,36 @@ struct Scratch {
 };
 constexpr size_t kScratchStreams = 4;
 
+// How many live CUDA graphs hold the device addresses of a plan.  A captured call counts itself in and leaves an object
+// with the graph that counts it out when the graph and what was instantiated from it are gone (from whatever thread that
+// happens on; the plan itself may have gone before).
+typedef std::shared_ptr<std::atomic<int>> GraphUses;
+void CUDART_CB graph_is_gone(void* p) {
+  GraphUses* uses = static_cast<GraphUses*>(p);
+  --**uses;
+  delete uses;
+}
+int note_capture(cudaStream_t stream, const GraphUses& uses) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  TS_CUDA(cudaStreamGetCaptureInfo(stream, &status, nullptr, &graph, nullptr, nullptr));
+  if (status != cudaStreamCaptureStatusActive) return TS_OK;
+  GraphUses* held = new GraphUses(uses);
+  ++**held;
+  cudaUserObject_t object = nullptr;
+  cudaError_t e = cudaUserObjectCreate(&object, held, graph_is_gone, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    graph_is_gone(held);
+  } else {
+    e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
+  }
+  TS_CUDA(e);
+  return TS_OK;
+}
+
 struct Schedule {
+  GraphUses graphs = std::make_shared<std::atomic<int>>(0);
   DeviceBlock mem;             // holds everything below
   ts::WorkItem* d_units = nullptr;
   ts::BlockDesc* d_blocks = nullptr;
@@ -705,12 +735,17 @@ struct ts_layer {
 namespace {
 
 // The caller has waited for the device: queued launches may use the schedules' memory until then.
-void drop_schedules(ts_layer* l) {
-  for (auto& kv : l->schedules) {
-    give_block(&l->spare, &kv.second.mem);
-    for (Scratch& c : kv.second.scratch) give_block(&l->spare, &c.mem);
+void drop_schedules(ts_layer* l, bool keep_captured = false) {
+  for (auto it = l->schedules.begin(); it != l->schedules.end();) {
+    Schedule& s = it->second;
+    if (keep_captured && *s.graphs > 0) {
+      ++it;
+      continue;
+    }
+    give_block(&l->spare, &s.mem);
+    for (Scratch& c : s.scratch) give_block(&l->spare, &c.mem);
+    it = l->schedules.erase(it);
   }
-  l->schedules.clear();
 }
 
 // The layer is one without tiles from here on: nothing it keeps may describe lists that are gone.
@@ -803,9 +838,11 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
     *out = &it->second;
     return TS_OK;
   }
-  if (l->schedules.size() >= 16) {  // bounded cache: drop everything, rebuild on demand
+  size_t droppable = 0;
+  for (const auto& kv : l->schedules) droppable += *kv.second.graphs == 0;
+  if (droppable >= 16) {  // bounded cache: drop everything that no captured graph refers to, rebuild on demand
     TS_CUDA(cudaDeviceSynchronize());
-    drop_schedules(l);
+    drop_schedules(l, /*keep_captured=*/true);
   }
   Schedule s;
   std::vector<ts::WorkItem> flat;
@@ -1234,6 +1271,8 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   rc = get_schedule(l, M, lda, conv_wp, allow_split, &s);
   if (rc != TS_OK) return rc;
   if (s->n_units == 0) return TS_OK;
+  rc = note_capture(static_cast<cudaStream_t>(stream), s->graphs);
+  if (rc != TS_OK) return rc;
   Scratch* scratch = nullptr;
   if (s->n_split > 0) {
     rc = scratch_for(s, static_cast<cudaStream_t>(stream), &scratch);
@@ -1644,7 +1683,7 @@ int ts_layer_schedule_stats(ts_layer_t* l, int M, int* n_ctas, float* cta_cost, 
 
 // Schedules of the reference-signature entry point, per device: one per shape (sizes, kept counts and
 // offsets; the lists' addresses and contents belong to the call), the latest kMaxShim of them and those a
-// captured graph refers to, so that a program that alternates between layers neither rebuilds nor uploads
+// live CUDA graph refers to, so that a program that alternates between layers neither rebuilds nor uploads
 // anything (calls on one device must be issued on one stream or externally ordered).
 namespace {
 struct ShimSchedule {
@@ -1657,7 +1696,7 @@ struct ShimSchedule {
   const void* B = nullptr;       // the weights `tmap` describes
   CUtensorMap tmap;
   unsigned long long used = 0;   // tick of the latest call
-  bool captured = false;         // a CUDA graph holds its addresses: never dropped
+  GraphUses graphs = std::make_shared<std::atomic<int>>(0);
 };
 constexpr size_t kMaxShim = 16;
 struct ShimDevice {
@@ -1756,14 +1795,15 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
     for (int t = 0; t < block_num; ++t) c.key.insert(c.key.end(), {N_cal[t], K_cal[t], off_B[t], off_C[t]});
     c.n_items = static_cast<int>(flat.size());
     c.n_blocks = static_cast<int>(blocks.size());
-    size_t n_free = 0;
-    auto oldest = sd.schedules.end();
-    for (auto it = sd.schedules.begin(); it != sd.schedules.end(); ++it) {
-      if (it->captured) continue;
-      ++n_free;
-      if (oldest == sd.schedules.end() || it->used < oldest->used) oldest = it;
-    }
-    if (n_free >= kMaxShim) {
+    while (true) {      // (several go at once when graphs that held them are gone)
+      size_t n_free = 0;
+      auto oldest = sd.schedules.end();
+      for (auto it = sd.schedules.begin(); it != sd.schedules.end(); ++it) {
+        if (*it->graphs > 0) continue;
+        ++n_free;
+        if (oldest == sd.schedules.end() || it->used < oldest->used) oldest = it;
+      }
+      if (n_free < kMaxShim) break;
       TS_CUDA(cudaDeviceSynchronize());
       free_shim(*oldest);
       sd.schedules.erase(oldest);
@@ -1782,12 +1822,11 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
     w = &sd.schedules.back();
   }
   w->used = ++sd.tick;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  TS_CUDA(cudaStreamIsCapturing(s, &capture));
-  if (capture != cudaStreamCaptureStatusNone) w->captured = true;
+  int rc = note_capture(s, w->graphs);
+  if (rc != TS_OK) return rc;
   if (w->B != B) {
     w->B = nullptr;
-    int rc = make_weight_tmap(&w->tmap, dtype, B, N, K);
+    rc = make_weight_tmap(&w->tmap, dtype, B, N, K);
     if (rc != TS_OK) return rc;
     w->B = B;
   }

@@ -109,9 +109,9 @@ __device__ __forceinline__ WorkItem load_item(const WorkItem* p) {
     int4 v[3];
     WorkItem w;
   } u;
-  u.v[0] = __ldg(q);
-  u.v[1] = __ldg(q + 1);
-  u.v[2] = __ldg(q + 2);
+  u.v[0] = ld_coherent(q);
+  u.v[1] = ld_coherent(q + 1);
+  u.v[2] = ld_coherent(q + 2);
   return u.w;
 }
 
@@ -157,7 +157,7 @@ __device__ __forceinline__ int k_blocks(const WorkItem& w) { return (w.k_count +
 
 // Ct row (global column of W) of tile column j of a work item.
 __device__ __forceinline__ long long c_row_of(const EpiItem& w, int j) {
-  return w.c_row0 + (w.n_list ? __ldg(w.n_list + j) + ((w.flags & kItemRelative) ? j : 0) : j);
+  return w.c_row0 + (w.n_list ? ld_coherent(w.n_list + j) + ((w.flags & kItemRelative) ? j : 0) : j);
 }
 
 // gelu(x) = x * 0.5 * (1 + tanh(u)), u = sqrt(2/pi) * (x + 0.044715 x^3)  (Pruning/BERT/utils/modeling.py:264-277),
@@ -215,7 +215,10 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   const int act = ep.act;
   const bool use_tma_store = (flags & kFlagTmaStore) != 0;
   // the schedule, the records or the weights come from the kernel before this one
-  if (flags & kFlagWaitFirst) grid_dependency_wait();
+  if (flags & kFlagWaitFirst) {
+    grid_dependency_wait();
+    fence_proxy_async();      // the records and the weights are fetched by bulk copies
+  }
   constexpr bool SPLIT = MODE == kModeSplit, PEERS = MODE == kModePeers, NHWC = MODE == kModeNhwc, ROWS = MODE == kModeRows || NHWC;
   constexpr bool LEAN = MODE == kModeLean || ROWS;
   using C = Cfg<MT>;
@@ -471,7 +474,7 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
     // copies in every lane cost the registers that two TMEM chunks need.
     const int* const items = reinterpret_cast<const int*>(sched + cta) + lane;
     auto item_word = [&](int r) -> int {
-      return r < rounds && lane < kItemWords ? __ldg(items + static_cast<size_t>(r) * grid * kItemWords) : -1;
+      return r < rounds && lane < kItemWords ? ld_coherent(items + static_cast<size_t>(r) * grid * kItemWords) : -1;
     };
     int word = item_word(0);
     grid_dependency_wait();   // Ct may still be read or written by the previous kernel
@@ -497,8 +500,8 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       const bool last_unit = __shfl_sync(0xffffffffu, word_next, kItemWordTile) < 0;
       const long long c_row = active ? c_row_of(w, j) : 0;
       const int c_row_or_none = active ? static_cast<int>(c_row) : -1;
-      const float bias_j = (ep.bias != nullptr && active) ? __ldg(ep.bias + c_row) : 0.0f;
-      const int tile_row0 = w.c_row0 + ((tma_store && w.n_list) ? __ldg(w.n_list) : 0);
+      const float bias_j = (ep.bias != nullptr && active) ? ld_coherent(ep.bias + c_row) : 0.0f;
+      const int tile_row0 = w.c_row0 + ((tma_store && w.n_list) ? ld_coherent(w.n_list) : 0);
       if (!mbar_wait(smem_u32(&bars->acc_full[a]), aph, abort_flag)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + a * MT + (static_cast<uint32_t>(q * 32) << 16);
@@ -716,7 +719,7 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
 __device__ __forceinline__ void expand_record(const BlockDesc& d, const int* idx, int r, int* rec, const RowMap& map) {
   int v = 0;
   if (d.meta != kBlockEnd && r < static_cast<int>(d.meta & 0x7fu)) {
-    v = __ldg(idx + r);
+    v = ld_coherent(idx + r);
     if (d.meta & 0x80u) v += static_cast<int>(d.meta >> 10) + r;
     if (map.conv_cin > 0) {
       const int c = v % map.conv_cin, rj = v / map.conv_cin;

@@ -241,9 +241,31 @@ __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Loads of data that the kernel before may have written while this one was already running: after the wait, and coherent.
+// (A load through the read-only path, which __ldg is and a const __restrict__ pointer may become, promises that nobody
+// writes the data while the kernel lives.)
+__device__ __forceinline__ int4 ld_coherent(const int4* p) {
+  int4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_coherent(const int* p) {
+  int v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_coherent(const float* p) {
+  return __int_as_float(ld_coherent(reinterpret_cast<const int*>(p)));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Proxy / tcgen05 fences
 // ---------------------------------------------------------------------------------------------
+// What this thread sees written, its bulk and TMA copies see too.
+__device__ __forceinline__ void fence_proxy_async() {
+  asm volatile("fence.proxy.async;" ::: "memory");
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

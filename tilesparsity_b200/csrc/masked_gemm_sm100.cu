@@ -93,11 +93,8 @@ struct Cfg {
   static constexpr int kStageBytes = kWBytes + kABytes;
   static constexpr int kEpiBytes = kEpiWarps * kEpiWarpBytes;
   static constexpr int kTmemCols = 2 * MT;          // two accumulators of MT fp32 columns
-  // stages + staging + barriers/records + what the 1024-byte alignment of the first stage may skip
-  static constexpr int kUsedBytes = kStages * kStageBytes + kEpiBytes + static_cast<int>(sizeof(Barriers));
-  static constexpr int kSmemBytes = (kUsedBytes + 1023 + 1023) / 1024 * 1024 > 232448 ? 232448
-                                                                                      : (kUsedBytes + 1023 + 1023) / 1024 * 1024;
-  static_assert(kUsedBytes <= kSmemBytes, "stages, staging and barriers exceed the shared memory of one CTA");
+  static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + static_cast<int>(sizeof(Barriers));
+  static_assert(kSmemBytes <= 232448, "stages, staging and barriers exceed the shared memory of one CTA");
   static constexpr int kLanesPerRow = MT / 8;       // 16-byte chunks in one gathered row
   static constexpr int kRowsPerInstr = 32 / kLanesPerRow;
   static constexpr int kGroups = MT / 128;          // 64-column groups of a unit per epilogue warp
@@ -223,15 +220,9 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
   constexpr bool LEAN = MODE == kModeLean || ROWS;
   using C = Cfg<MT>;
   constexpr int kStages = C::kStages;
-  extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment: the swizzle pattern is a function of the shared-memory address bits.
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  if (static_cast<int>(smem - smem_raw) + C::kUsedBytes > C::kSmemBytes) {
-    // the dynamic shared-memory window starts at an address this layout was not sized for
-    if (threadIdx.x == 0) atomicExch(status, kErrUnsupported);
-    return;
-  }
+  // 1024-byte alignment: the swizzle pattern is a function of the shared-memory address bits.  The declaration asks for
+  // it, so no byte is set aside to reach it.
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* epi = smem + kStages * C::kStageBytes;
   Barriers* bars = reinterpret_cast<Barriers*>(epi + C::kEpiBytes);
   volatile int* abort_flag = &bars->abort_flag;

@@ -133,3 +133,15 @@ def test_img2col_round_trip_on_the_host():
     assert torch.equal(back[0].reshape(72, 16), m[0])
     with pytest.raises(ValueError):
         masks.img2col_back_ward([m[1]], [conv])
+
+
+def test_the_extension_of_another_torch_is_not_loaded(monkeypatch):
+    """The extension is linked against torch's C++ ABI: its name carries the version, and a missing one says what to do."""
+    import torch
+
+    from tilesparsity_b200 import _lib
+    assert _lib.fast() is _lib.fast()
+    monkeypatch.setattr(_lib, "_fast", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with pytest.raises(ImportError, match="build.py"):
+        _lib.fast()

@@ -133,8 +133,10 @@ def fast():
     """The _tsfast extension (host path of the per-batch operators); loads torch."""
     global _fast
     if _fast is None:
-        import torch  # noqa: F401  (the extension links against it)
-        path = os.path.join(HERE, "_tsfast.so")
+        import torch    # (the extension links against it)
+
+        from .build import extension_path
+        path = extension_path(torch.__version__)
         if not os.path.exists(path):
             raise ImportError(f"{path} is missing: build it with `python tilesparsity_b200/build.py`")
         import importlib.util

@@ -6,6 +6,7 @@ csrc/pyfast.cpp, the host path of the per-batch operators, with g++ against the 
 """
 from __future__ import annotations
 
+import importlib.metadata
 import importlib.util
 import os
 import shutil
@@ -18,13 +19,18 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "obj")
 LIB_PATH = os.path.join(HERE, "libtilesparse.so")
-EXT_PATH = os.path.join(HERE, "_tsfast.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC",
 ]
+
+
+def extension_path(torch_version: str) -> str:
+    """Where the extension built for this Python and that torch lies.  It is linked against torch's C++ ABI: another
+    version's build has another name and is not loaded."""
+    return os.path.join(HERE, f"_tsfast.{sysconfig.get_config_var('SOABI')}-torch{torch_version}.so")
 
 
 def sources() -> list[str]:
@@ -80,24 +86,25 @@ def numpy_include() -> str:
     return numpy.get_include()
 
 
-def _build_extension() -> None:
+def _build_extension(path: str) -> None:
     root = os.path.dirname(importlib.util.find_spec("torch").origin)
     inc, lib = os.path.join(root, "include"), os.path.join(root, "lib")
     cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
     _run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
           "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + cuda,
-          "-I" + sysconfig.get_paths()["include"], "-I" + numpy_include(), "-o", EXT_PATH + ".tmp", os.path.join(CSRC, "pyfast.cpp"),
+          "-I" + sysconfig.get_paths()["include"], "-I" + numpy_include(), "-o", path + ".tmp", os.path.join(CSRC, "pyfast.cpp"),
           "-L" + HERE, "-l:libtilesparse.so", "-Wl,-rpath,$ORIGIN", "-L" + lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
           "-lc10_cuda", "-lc10"])
-    os.replace(EXT_PATH + ".tmp", EXT_PATH)
+    os.replace(path + ".tmp", path)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Builds what is missing or older than its sources; returns the library's path."""
     if force or _older(LIB_PATH, sources() + _headers()):
         _build_library(force, verbose)
-    if force or _older(EXT_PATH, [os.path.join(CSRC, "pyfast.cpp"), os.path.join(HERE, "..", "include", "tilesparse.h")]):
-        _build_extension()
+    ext = extension_path(importlib.metadata.version("torch"))
+    if force or _older(ext, [os.path.join(CSRC, "pyfast.cpp"), os.path.join(HERE, "..", "include", "tilesparse.h")]):
+        _build_extension(ext)
     return LIB_PATH
 
 

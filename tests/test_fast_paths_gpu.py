@@ -507,3 +507,34 @@ def test_a_graph_outlives_many_batch_sizes():
     layer.check()
     del graph
     layer.close()
+
+
+def test_threads_that_plan_and_ask():
+    """Products of new batch sizes on one thread while others ask for schedules of others: one of them at a time."""
+    layer, W = _layer(256, 512, 100, torch.float16, 61)
+    Wm = _dense(W, layer, torch.float16)
+    xs = [torch.randn((256, 8 * m), device="cuda").half() for m in range(1, 40)]
+    torch.cuda.synchronize()
+    errors, outs = [], {}
+
+    def ask(first):
+        try:
+            for m in range(first, 400, 3):
+                assert layer.schedule_stats(8 * m)["n_units"] > 0
+        except Exception as e:      # reported by the main thread
+            errors.append(e)
+
+    def run():
+        try:
+            for i, x in enumerate(xs):
+                outs[i] = layer.masked_gemm(x)
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=ask, args=(i,)) for i in (1, 2, 3)] + [threading.Thread(target=run)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors
+    for i, x in enumerate(xs):
+        assert _rel(outs[i], Wm.t() @ x.double()) <= TOL[torch.float16]
+    layer.close()

@@ -681,7 +681,7 @@ int current_sm_count(int* out) {
 }  // namespace
 
 struct ts_layer {
-  // One host thread at a time plans and launches a GEMM: schedules and output maps are filled in by the calls.
+  // One host thread at a time re-tiles, plans and launches: schedules and output maps are filled in by the calls.
   std::mutex mu;
   int K = 0, N = 0, G = 0, dtype = 0;
   int device = 0;
@@ -1085,6 +1085,7 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
       }
     }
   }
+  std::lock_guard<std::mutex> lock(l->mu);
   TS_CUDA(cudaSetDevice(l->device));
   TS_CUDA(cudaDeviceSynchronize());
   drop_tiles(l);   // (what follows may fail; the new structure is installed at the end)
@@ -1158,6 +1159,7 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
 
 int ts_layer_pack_weights(ts_layer_t* l, const void* W_dev, int64_t ldw_in, int w_dtype, void* stream) {
   if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
+  std::lock_guard<std::mutex> lock(l->mu);
   if (!l->d_wp) return fail(TS_ERR_INVALID, "layer has no tiles (call ts_layer_set_tiles)");
   if (!W_dev) return fail(TS_ERR_INVALID, "W is NULL");
   if (ldw_in < l->N) return fail(TS_ERR_INVALID, "ldw_in=%lld is smaller than N=%d", (long long)ldw_in, l->N);
@@ -1178,6 +1180,7 @@ int ts_layer_set_unit_rows(ts_layer_t* l, int unit_rows) {
   if (unit_rows != 0 && unit_rows != 128 && unit_rows != 256) {
     return fail(TS_ERR_INVALID, "unit_rows=%d must be 0 (automatic), 128 or 256", unit_rows);
   }
+  std::lock_guard<std::mutex> lock(l->mu);
   if (unit_rows == l->forced_unit_rows) return TS_OK;
   TS_CUDA(cudaSetDevice(l->device));
   TS_CUDA(cudaDeviceSynchronize());   // cached schedules may be in use by queued launches
@@ -1346,6 +1349,7 @@ extern "C" {
 
 int ts_layer_zero_pruned(ts_layer_t* l, int M, void* Ct, int64_t ldc, void* stream) {
   if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
+  std::lock_guard<std::mutex> lock(l->mu);
   if (M < 0 || (M % 8) != 0) return fail(TS_ERR_INVALID, "M=%d must be a non-negative multiple of 8", M);
   if (!l->d_kept_n) return fail(TS_ERR_INVALID, "layer has no tiles (call ts_layer_set_tiles)");
   if (M == 0 || l->n_pruned == 0) return TS_OK;
@@ -1378,6 +1382,7 @@ int ts_masked_gemm_ex(ts_layer_t* l, int M, const void* At, int64_t lda, void* C
 int ts_layer_row_output(ts_layer_t* l, int M, int* supported) {
   if (!l || !supported) return fail(TS_ERR_INVALID, "NULL argument");
   *supported = 0;
+  std::lock_guard<std::mutex> lock(l->mu);
   if (!l->rows_ok || M <= 0) return TS_OK;
   if (l->split_k) {   // a layer whose long tiles pay for split-K keeps it, and the K-major output with it
     std::vector<int> parts;
@@ -1483,6 +1488,7 @@ int ts_masked_conv(ts_layer_t* l, int B, int H, int W, const void* planes_dev, i
 int ts_conv_nhwc_output(ts_layer_t* l, int B, int H, int W, int* supported) {
   if (!l || !supported) return fail(TS_ERR_INVALID, "NULL argument");
   *supported = 0;
+  std::lock_guard<std::mutex> lock(l->mu);
   if (!l->rows_ok || l->conv_cin <= 0) return TS_OK;
   int hp = 0, wp = 0;
   int64_t m = 0;
@@ -1671,6 +1677,7 @@ int ts_layer_check(ts_layer_t* l, void* stream) {
 int ts_layer_schedule_stats(ts_layer_t* l, int M, int* n_ctas, float* cta_cost, int* n_units) {
   if (!l) return fail(TS_ERR_INVALID, "layer is NULL");
   if (M <= 0) return fail(TS_ERR_INVALID, "M=%d must be positive", M);
+  std::lock_guard<std::mutex> lock(l->mu);
   if (!l->d_tiles) return fail(TS_ERR_INVALID, "layer has no tiles");
   Schedule* s = nullptr;
   int rc = get_schedule(l, M, M, 0, l->split_k, &s);

@@ -538,3 +538,36 @@ def test_threads_that_plan_and_ask():
     for i, x in enumerate(xs):
         assert _rel(outs[i], Wm.t() @ x.double()) <= TOL[torch.float16]
     layer.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("all_written", [True, False])
+@pytest.mark.parametrize("K,N,M", [(64, 5, 8), (300, 130, 264), (1000, 64, 520)])
+def test_residual_gemm(K, N, M, all_written, dtype):
+    """ts_residual_gemm against float64, element by element.  fp16 adds up four products at a time in half precision (at
+    most three roundings of 2^-11 of their magnitudes, and the products' own), bf16 in fp32; the output rounds once."""
+    from tilesparsity_b200 import _lib
+    g = torch.Generator("cuda").manual_seed(K + N + M)
+    mask = torch.rand((K, N), device="cuda", generator=g) < 0.05
+    mask[:, 1] = False                                   # a column without elements
+    W = torch.randn((K, N), device="cuda", generator=g).to(dtype) * mask
+    x = torch.randn((K, M), device="cuda", generator=g).to(dtype)
+    Ct = torch.randn((N, M), device="cuda", generator=g).to(dtype)
+    written = torch.ones(N, dtype=torch.uint8, device="cuda")
+    if not all_written:
+        written[::3] = 0
+    at = mask.t().nonzero()                              # by column, rows ascending
+    ptr = torch.zeros(N + 1, dtype=torch.int32, device="cuda")
+    ptr[1:] = mask.sum(0).cumsum(0)
+    rows, val = at[:, 1].int().contiguous(), W.t()[mask.t()].contiguous()
+    alpha = -1.5
+    base = Ct.double() * written[:, None]
+    ref = base + alpha * (W.double().t() @ x.double())
+    size = base.abs() + 1.5 * (W.double().abs().t() @ x.double().abs())
+    p = lambda t: t.data_ptr()
+    assert _lib.lib.ts_residual_gemm(0 if dtype == torch.float16 else 1, M, N, p(ptr), p(rows), p(val), None if all_written else p(written), p(x),
+                                     x.stride(0), p(Ct), Ct.stride(0), alpha, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    unit = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    bound = unit * ref.abs() + (4 * 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -18) * size + 2.0 ** -20
+    assert bool(((Ct.double() - ref).abs() <= bound).all())

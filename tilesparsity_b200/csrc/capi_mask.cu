@@ -1,10 +1,9 @@
-// C ABI of the mask builder: host orchestration of the kernels in mask_build.cu.
+// C ABI of the mask builder: host orchestration of the kernels in mask_build.cu and mask_group.cu.
 //
-// The host side owns the parts of the reference algorithm that are scalar: the percentile's index
-// arithmetic and interpolation (np.percentile, method "linear"), the sparsity remap of the 2-D
-// variant (Pruning/VGG/prune_algo.py:61) and the regrouping of surviving columns into tiles
-// (prune_algo.py:72-89).  They are written as single IEEE-754 operations in the arithmetic type
-// NumPy would use, so that thresholds, and with them the masks, come out bit-identical.
+// The host side owns the sparsity remap of the 2-D variant (Pruning/VGG/prune_algo.py:61) and, where a percentile does
+// not run whole on the device (mask_group.cu), its index arithmetic and interpolation (np.percentile, method "linear").  They are written
+// as single IEEE-754 operations in the arithmetic type NumPy would use, so that thresholds, and with them the masks, come
+// out bit-identical.
 #include "../../include/tilesparse.h"
 
 #include <algorithm>

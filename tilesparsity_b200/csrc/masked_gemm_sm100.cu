@@ -22,20 +22,19 @@
 // activation rows are the MN-major B operand, fetched with 16-byte cp.async into the same swizzle
 // pattern (one kept row is one contiguous 2*MT-byte global segment).
 //
-// Pipeline: four stages of 64 kept rows (six for 128-row units).  The four gather warps fill every
-// block together, a quarter of its rows each; all a warp needs to know about a block is one
-// shared-memory record (descriptor + 64 resolved row numbers) that it prefetched by cp.async during
-// the block before.  Each lane hands its copies to the stage's mbarrier with
-// cp.async.mbarrier.arrive, so a stage is released to the MMA warp the moment its bytes have landed.  Accumulators live in TMEM, double buffered: the
-// epilogue of one work unit overlaps the main loop of the next.  Eight epilogue warps (two per TMEM
-// lane quarter; each half of them takes every other 64-column group of the unit) convert their rows
-// to 16 bit into a 128-byte-swizzled 16 KiB staging group per half.  When the tile's kept columns
-// are consecutive rows of Ct (no column pruning) a group leaves with one TMA store; otherwise each
-// warp writes its 32 rows with 16-byte coalesced stores through the kept-column list.
+// Pipeline: four stages of 64 kept rows (six for 128-row units).  Two groups of four gather warps take turns on the
+// blocks, a quarter of a block's rows each; all a warp needs to know about a block is one record (descriptor + 64
+// resolved row numbers) that a bulk copy brought to shared memory kAhead blocks before its weights.  Each lane hands its
+// copies to the stage's mbarrier with cp.async.mbarrier.arrive, so a stage is released to the MMA warp the moment its
+// bytes have landed.  Accumulators live in TMEM, double buffered: the epilogue of one work unit overlaps the main loop
+// of the next.  Eight epilogue warps (two per TMEM lane quarter; each half of them takes every other 64-column group of
+// the unit) convert their 32 rows of a group to 16 bit in a 128-byte-swizzled 4 KiB staging buffer per warp.  When the
+// tile's kept columns are consecutive rows of Ct (no column pruning) a warp's rows leave with one TMA store; otherwise
+// with 16-byte coalesced stores through the kept-column list.
 //
-// Warp roles (448 threads): warp 0 = weight TMA, warp 1 = TMEM allocation + MMA issue,
-// warps 2-5 = activation gather, warps 6-13 = epilogue.  (Eight gather warps were measured: 18 warps
-// leave 96 registers per thread, the kernel spills, and every workload got slower.)
+// Warp roles (576 threads): warp 0 = weights by TMA and block records, warp 1 = TMEM allocation + MMA issue, warps
+// 2-9 = activation gather, warps 10-17 = epilogue.  18 warps leave 96 registers per thread, which the epilogue keeps to
+// by holding 32 accumulators at a time.
 #include <cstddef>
 #include <type_traits>
 
@@ -704,9 +703,9 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
 // is channel c of the copy of the padded input shifted by j pixels, read r image rows further down:
 // segment ((j * cin + c) * plane_ld + r * Wp) / 8.  The kept row number itself comes from the tile's
 // list, or list position + offset for lists in the reference's relative form.
-// Lists that the caller hands over per call (reference-signature entry point): `lists` carries their
-// addresses, the descriptors hold the tile's number and the byte offset inside its list instead of an address
-// (see stream_list_code), and the work items get their column lists here.
+// Lists that the caller hands over per call (reference-signature entry point): `lists` carries their addresses, the
+// descriptors hold the tile's number (stream_list_code) plus the byte offset inside its list instead of an address, and
+// the work items get their column lists here.
 __device__ __forceinline__ void expand_record(const BlockDesc& d, const int* idx, int r, int* rec, const RowMap& map) {
   int v = 0;
   if (d.meta != kBlockEnd && r < static_cast<int>(d.meta & 0x7fu)) {

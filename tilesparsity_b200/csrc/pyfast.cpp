@@ -3,7 +3,7 @@
 // A masked GEMM of a small batch takes 4 us on a B200; through ctypes the same call spent 11 us in the
 // interpreter (attribute reads, argument checks, six argument conversions, a device guard and a stream
 // query in Python).  Here the checks read the tensors' C++ objects directly and the C ABI is called without
-// conversions: 1 us on top of the launch.  The functions mirror their Python callers in layer.py and conv.py,
+// conversions: 3 us a call with the launch.  The functions mirror their Python callers in layer.py and masks.py,
 // which keep the rarely used forms (peer buffers, the CUDA-core twin) for themselves.
 #include <Python.h>
 

@@ -16,14 +16,14 @@ namespace ts {
 // same schedule at K-block granularity: CTA b's 64-row blocks in processing order, one record of
 // kBlockMetaInts ints each, at block_meta[b*blk_stride*kBlockMetaInts ...], terminated (and padded
 // to blk_stride records) by end markers; expand_block_meta_launch writes it from the descriptors.
-// tmap_c != nullptr enables TMA stores (tensor map over Ct [N][ldc], box 64 x 128, 128-byte swizzle)
-// for the work items whose flags say their kept columns are consecutive rows of Ct.  early_start
+// tmap_c != nullptr enables TMA stores (tensor map over Ct [N][ldc], box 64 batch columns x 32 rows, 128-byte
+// swizzle) for the work items whose flags say their kept columns are consecutive rows of Ct.  early_start
 // lets the kernel read sched, block_meta and the packed weights before it waits for the kernel before it
 // in the stream (programmatic dependent launch), so it must be false when that kernel wrote them.
 // lean: every unit of the schedule has kItemDenseRows set (the kernel then takes its store-only variant
-// when beta is 0).  rows: tmap_c is a map over a row-major output C[M][N] (box 32 columns x 64 rows, no
-// swizzle) and every tile's first column is a multiple of 8; needs lean and beta == 0.
-// Where the result goes: Ct [N][ldc], a row-major C [M][ldc], or NHWC pixels [B][H][W][ldc].
+// when beta is 0).  form: where the result goes, Ct [N][ldc], a row-major C [M][ldc] (tmap_c is then a map over C
+// [M][N], box 32 columns x 64 rows, no swizzle) or NHWC pixels [B][H][W][ldc] (no map); the latter two need lean,
+// beta == 0 and tiles whose first columns are multiples of 8.
 enum OutForm { kOutColumns, kOutRows, kOutNhwc };
 cudaError_t masked_gemm_launch(int dtype, int unit_rows, const CUtensorMap& tmap_w, const CUtensorMap* tmap_c,
                                const WorkItem* sched, int rounds, int grid, const int* block_meta,
@@ -44,7 +44,7 @@ cudaError_t expand_block_meta_launch(const BlockDesc* blocks, long long n_blocks
                                      cudaStream_t stream);
 
 // The same for the reference-signature entry point, whose index lists arrive with the call: descriptors hold
-// stream_list_code(tile, position) in place of an address, and the work items' column lists are filled in.
+// stream_list_code(tile) + the position's byte offset in place of an address, and the work items' column lists are filled in.
 cudaError_t expand_stream_launch(const BlockDesc* blocks, int n_blocks, int* meta, WorkItem* items, int n_items,
                                  const RowMap& map, const StreamLists& lists, cudaStream_t stream);
 

@@ -182,8 +182,8 @@ int take_block(std::vector<DeviceBlock>* spare, size_t bytes, DeviceBlock* out) 
   *out = DeviceBlock{p, bytes};
   return TS_OK;
 }
-// Copies host arrays to their places in a device block, and waits until they have landed (a copy from pageable memory may
-// return before).  Small ones go through one buffer: a copy costs some 10 us to start.  Large ones go as they are:
+// Copies host arrays to their places in a device block, on the null stream (the caller waits for it: a copy from pageable
+// memory may return before it has landed).  Small ones go through one buffer: a copy costs some 10 us to start.  Large ones go as they are:
 // gathering the 8 MB plan of a 16384 x 16384 layer first took longer than the copies.
 struct Piece {
   size_t at;
@@ -204,8 +204,7 @@ cudaError_t upload_pieces(char* base, const Piece* pieces, int n, size_t total) 
       if (pieces[i].bytes > 0) e = cudaMemcpy(base + pieces[i].at, pieces[i].src, pieces[i].bytes, cudaMemcpyHostToDevice);
     }
   }
-  const cudaError_t done = cudaStreamSynchronize(nullptr);
-  return e == cudaSuccess ? done : e;
+  return e;
 }
 // What a layer holds back between its re-tilings: the latest blocks, at most this many and this much together (a plan of
 // an encoder layer takes 1.3 MB; one of tens of megabytes takes longer to make than to allocate).
@@ -1133,6 +1132,7 @@ int ts_layer_set_tiles(ts_layer_t* l, int n_tiles, const int32_t* tile_k_ptr,
                            {o_n, nn.data(), nn.size() * sizeof(int)},
                            {o_tiles, td.data(), td.size() * sizeof(ts::TileDesc)}};
   TS_CUDA(upload_pieces(base, pieces, 3, upload));
+  TS_CUDA(cudaStreamSynchronize(nullptr));
   int rc = make_weight_tmap(&l->tmap, l->dtype, base + o_wp, wp_rows, ldw);
   if (rc != TS_OK) return rc;
   l->d_kept_k = reinterpret_cast<int*>(base + o_k);

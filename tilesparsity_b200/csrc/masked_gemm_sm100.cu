@@ -488,10 +488,11 @@ masked_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w,
       // The CTA's last unit: every K block has been consumed, so the pipeline stages are free and
       // each group gets a staging buffer of its own there; none waits for a store before it.
       const bool last_unit = __shfl_sync(0xffffffffu, word_next, kItemWordTile) < 0;
-      const long long c_row = active ? c_row_of(w, j) : 0;
+      const int tile_row0 = w.c_row0 + ((tma_store && w.n_list) ? ld_coherent(w.n_list) : 0);
+      // (the store-only variants' tiles keep consecutive columns: no list to read, and nothing to wait for without a bias)
+      const long long c_row = !active ? 0 : (LEAN ? tile_row0 + j : c_row_of(w, j));
       const int c_row_or_none = active ? static_cast<int>(c_row) : -1;
       const float bias_j = (ep.bias != nullptr && active) ? ld_coherent(ep.bias + c_row) : 0.0f;
-      const int tile_row0 = w.c_row0 + ((tma_store && w.n_list) ? ld_coherent(w.n_list) : 0);
       if (!mbar_wait(smem_u32(&bars->acc_full[a]), aph, abort_flag)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + a * MT + (static_cast<uint32_t>(q * 32) << 16);

@@ -18,7 +18,7 @@
  *    and base pointers 16-byte aligned.
  *  - A layer may be used on several streams and by several host threads; calls that depend on one another are ordered
  *    by the caller, and so are the launches of CUDA graphs that hold the same layer.  Such a graph is good until the
- *    layer is re-tiled, given other unit sizes or destroyed.
+ *    layer is re-tiled, given other unit sizes or destroyed, and the layer keeps its plan until then.
  *  - There is no CPU fallback: without a CUDA device every compute call fails with TS_ERR_CUDA.
  */
 #ifndef TILESPARSE_H_
@@ -302,6 +302,10 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
                       void* C, int block_num, const int* N_cal, const int* K_cal,
                       int* const* mask_n, int* const* mask_k, const int* off_B, const int* off_C,
                       int dtype, void* stream);
+
+/* Frees the plans ts_stream_gemm_nn keeps on the current device: those of the latest sixteen shapes, and those of every
+ * call that was captured into a CUDA graph (which may not be launched any more).  Waits for the device. */
+int ts_stream_gemm_trim(void);
 
 /* ---------------------------------------------------------------------------------------------
  * Mask construction

@@ -108,6 +108,7 @@ SIGNATURES = {
                                           C.POINTER(C.c_double), _vp]),
     "ts_residual_gemm": (C.c_int, [C.c_int, C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, C.c_int64, _vp, C.c_int64,
                                    C.c_float, _vp]),
+    "ts_stream_gemm_trim": (C.c_int, []),
     "ts_transpose16": (C.c_int, [_vp, C.c_int64, _vp, C.c_int64, C.c_int, C.c_int, _vp]),
     "ts_shard_plan": (C.c_int, [C.c_int, _i64p, C.c_int, _i32p]),
 }

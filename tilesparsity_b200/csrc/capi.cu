@@ -3,7 +3,6 @@
 #include "../../include/tilesparse.h"
 
 #include <algorithm>
-#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cmath>
@@ -236,36 +235,19 @@ struct Scratch {
 };
 constexpr size_t kScratchStreams = 4;
 
-// How many live CUDA graphs hold the device addresses of a plan.  A captured call counts itself in and leaves an object
-// with the graph that counts it out when the graph and what was instantiated from it are gone (from whatever thread that
-// happens on; the plan itself may have gone before).
-typedef std::shared_ptr<std::atomic<int>> GraphUses;
-void CUDART_CB graph_is_gone(void* p) {
-  GraphUses* uses = static_cast<GraphUses*>(p);
-  --**uses;
-  delete uses;
-}
-int note_capture(cudaStream_t stream, const GraphUses& uses) {
+// Whether calls on `stream` are being captured.  A CUDA graph holds the device addresses of the plans its calls use, and
+// nothing says when it is gone (a user object left with the graph would, but any such object makes every launch of
+// the graph 3 us longer, as long as half a GEMM of the graphs that programs replay): such plans are kept until their
+// owner goes or asks for their memory.
+int is_capturing(cudaStream_t stream, bool* out) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  cudaGraph_t graph = nullptr;
-  TS_CUDA(cudaStreamGetCaptureInfo(stream, &status, nullptr, &graph, nullptr, nullptr));
-  if (status != cudaStreamCaptureStatusActive) return TS_OK;
-  GraphUses* held = new GraphUses(uses);
-  ++**held;
-  cudaUserObject_t object = nullptr;
-  cudaError_t e = cudaUserObjectCreate(&object, held, graph_is_gone, 1, cudaUserObjectNoDestructorSync);
-  if (e != cudaSuccess) {
-    graph_is_gone(held);
-  } else {
-    e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
-    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
-  }
-  TS_CUDA(e);
+  TS_CUDA(cudaStreamIsCapturing(stream, &status));
+  *out = status != cudaStreamCaptureStatusNone;
   return TS_OK;
 }
 
 struct Schedule {
-  GraphUses graphs = std::make_shared<std::atomic<int>>(0);
+  bool captured = false;       // a CUDA graph may hold its addresses
   DeviceBlock mem;             // holds everything below
   ts::WorkItem* d_units = nullptr;
   ts::BlockDesc* d_blocks = nullptr;
@@ -737,7 +719,7 @@ namespace {
 void drop_schedules(ts_layer* l, bool keep_captured = false) {
   for (auto it = l->schedules.begin(); it != l->schedules.end();) {
     Schedule& s = it->second;
-    if (keep_captured && *s.graphs > 0) {
+    if (keep_captured && s.captured) {
       ++it;
       continue;
     }
@@ -768,11 +750,9 @@ void drop_tiles(ts_layer* l) {
 }
 
 // The scratch memory a call on `stream` uses.
-int scratch_for(Schedule* s, cudaStream_t stream, Scratch** out) {
+int scratch_for(Schedule* s, cudaStream_t stream, bool capturing, Scratch** out) {
   ++s->tick;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  TS_CUDA(cudaStreamIsCapturing(stream, &capture));
-  if (capture != cudaStreamCaptureStatusNone) {
+  if (capturing) {
     Scratch* c = &s->scratch[0];
     for (Scratch& o : s->scratch) {
       if (o.captured) c = &o;
@@ -838,8 +818,8 @@ int get_schedule(ts_layer* l, int M, long long ld, int conv_wp, bool allow_split
     return TS_OK;
   }
   size_t droppable = 0;
-  for (const auto& kv : l->schedules) droppable += *kv.second.graphs == 0;
-  if (droppable >= 16) {  // bounded cache: drop everything that no captured graph refers to, rebuild on demand
+  for (const auto& kv : l->schedules) droppable += !kv.second.captured;
+  if (droppable >= 16) {  // bounded cache: drop everything that no graph may refer to, rebuild on demand
     TS_CUDA(cudaDeviceSynchronize());
     drop_schedules(l, /*keep_captured=*/true);
   }
@@ -1274,11 +1254,13 @@ int run_masked_gemm(ts_layer_t* l, int M, const void* At, int64_t lda, void* Ct,
   rc = get_schedule(l, M, lda, conv_wp, allow_split, &s);
   if (rc != TS_OK) return rc;
   if (s->n_units == 0) return TS_OK;
-  rc = note_capture(static_cast<cudaStream_t>(stream), s->graphs);
+  bool capturing = false;
+  rc = is_capturing(static_cast<cudaStream_t>(stream), &capturing);
   if (rc != TS_OK) return rc;
+  s->captured |= capturing;
   Scratch* scratch = nullptr;
   if (s->n_split > 0) {
-    rc = scratch_for(s, static_cast<cudaStream_t>(stream), &scratch);
+    rc = scratch_for(s, static_cast<cudaStream_t>(stream), capturing, &scratch);
     if (rc != TS_OK) return rc;
   }
   ep.scratch_map = scratch ? scratch->map : nullptr;
@@ -1690,7 +1672,7 @@ int ts_layer_schedule_stats(ts_layer_t* l, int M, int* n_ctas, float* cta_cost, 
 
 // Schedules of the reference-signature entry point, per device: one per shape (sizes, kept counts and
 // offsets; the lists' addresses and contents belong to the call), the latest kMaxShim of them and those a
-// live CUDA graph refers to, so that a program that alternates between layers neither rebuilds nor uploads
+// captured graph refers to (until ts_stream_gemm_trim), so that a program that alternates between layers neither rebuilds nor uploads
 // anything (calls on one device must be issued on one stream or externally ordered).
 namespace {
 struct ShimSchedule {
@@ -1703,7 +1685,7 @@ struct ShimSchedule {
   const void* B = nullptr;       // the weights `tmap` describes
   CUtensorMap tmap;
   unsigned long long used = 0;   // tick of the latest call
-  GraphUses graphs = std::make_shared<std::atomic<int>>(0);
+  bool captured = false;         // a CUDA graph may hold its addresses
 };
 constexpr size_t kMaxShim = 16;
 struct ShimDevice {
@@ -1721,6 +1703,18 @@ void free_shim(ShimSchedule& s) {
   cudaFree(s.d_meta);
 }
 }  // namespace
+
+int ts_stream_gemm_trim(void) {
+  int dev = 0;
+  TS_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(g_shim_mu);
+  auto it = g_shim.find(dev);
+  if (it == g_shim.end() || it->second.schedules.empty()) return TS_OK;
+  TS_CUDA(cudaDeviceSynchronize());
+  for (ShimSchedule& c : it->second.schedules) free_shim(c);
+  it->second.schedules.clear();
+  return TS_OK;
+}
 
 int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const void* B, float beta,
                       void* C, int block_num, const int* N_cal, const int* K_cal,
@@ -1802,15 +1796,14 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
     for (int t = 0; t < block_num; ++t) c.key.insert(c.key.end(), {N_cal[t], K_cal[t], off_B[t], off_C[t]});
     c.n_items = static_cast<int>(flat.size());
     c.n_blocks = static_cast<int>(blocks.size());
-    while (true) {      // (several go at once when graphs that held them are gone)
-      size_t n_free = 0;
-      auto oldest = sd.schedules.end();
-      for (auto it = sd.schedules.begin(); it != sd.schedules.end(); ++it) {
-        if (*it->graphs > 0) continue;
-        ++n_free;
-        if (oldest == sd.schedules.end() || it->used < oldest->used) oldest = it;
-      }
-      if (n_free < kMaxShim) break;
+    size_t n_free = 0;
+    auto oldest = sd.schedules.end();
+    for (auto it = sd.schedules.begin(); it != sd.schedules.end(); ++it) {
+      if (it->captured) continue;
+      ++n_free;
+      if (oldest == sd.schedules.end() || it->used < oldest->used) oldest = it;
+    }
+    if (n_free >= kMaxShim) {
       TS_CUDA(cudaDeviceSynchronize());
       free_shim(*oldest);
       sd.schedules.erase(oldest);
@@ -1829,8 +1822,10 @@ int ts_stream_gemm_nn(int M, int N, int K, float alpha, const void* A, const voi
     w = &sd.schedules.back();
   }
   w->used = ++sd.tick;
-  int rc = note_capture(s, w->graphs);
+  bool capturing = false;
+  int rc = is_capturing(s, &capturing);
   if (rc != TS_OK) return rc;
+  w->captured |= capturing;
   if (w->B != B) {
     w->B = nullptr;
     rc = make_weight_tmap(&w->tmap, dtype, B, N, K);

@@ -36,6 +36,12 @@ def mask_gen(rng: np.random.Generator, n: int, n_pruned: int) -> np.ndarray:
     return keep - np.arange(n_pruned, dtype=np.int32)
 
 
+def trim_plans() -> None:
+    """Frees the plans `stream_gemm_nn` keeps on the current device, those of captured calls (whose graphs may not be
+    launched any more) among them; waits for the device."""
+    check(lib.ts_stream_gemm_trim())
+
+
 def prepare_stream_gemm_nn(M: int, N: int, K: int, alpha: float, A: torch.Tensor, B: torch.Tensor, beta: float,
                            C_out: torch.Tensor, block_num: int, N_cal, K_cal, mask_n, mask_k, off_B, off_C):
     """Marshals the arguments of Stream_Gemm_NN once and returns a zero-argument callable that issues

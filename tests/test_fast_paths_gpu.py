@@ -309,7 +309,8 @@ def test_retiling_reuses_memory_soundly():
     ("tw1m", 4096, 128, 64, 1.0),       # long chains: split-K
     ("tw1m", 256, 8, 8, -2.0),          # one tile of eight columns
 ])
-def test_tew_keeps_non_finite_activations_to_the_columns_that_keep_their_rows(algo, K, N, M, alpha, dtype):
+@pytest.mark.parametrize("everywhere", [False, True])     # one feature infinite, one NaN in every batch row
+def test_tew_keeps_non_finite_activations_to_the_columns_that_keep_their_rows(algo, K, N, M, alpha, everywhere, dtype):
     """Infinities and NaN in the activations: every output is what the mask's own entries give (an infinity of that
     sign, NaN where they clash, a finite sum where the column keeps no such row)."""
     from tilesparsity_b200 import TEWLayer, build_mask
@@ -320,8 +321,13 @@ def test_tew_keeps_non_finite_activations_to_the_columns_that_keep_their_rows(al
     kept = res.masks[0] | res.residuals[0]
     x = torch.randn((K, M), device="cuda", generator=g).to(dtype)
     inf = float("inf")
-    for i, (k, m, v) in enumerate([(7, 3, inf), (100, 3, -inf), (101, 5, float("nan")), (K - 1, M - 1, -inf), (0, 0, inf), (3, 0, inf)]):
+    for k, m, v in [(7, 3, inf), (100, 3, -inf), (101, 5, float("nan")), (K - 1, M - 1, -inf), (0, 0, inf), (3, 0, inf)]:
         x[k, m] = v
+    if everywhere:                                       # (features that the fewest columns keep)
+        few = [k for k in torch.argsort(kept.sum(1)).tolist() if kept[k].any()]
+        x[few[0]], x[few[1]] = inf, float("nan")
+        if N == 8:
+            x[[0, 3, 7, 100, 101, K - 1]] = 0.5
     ref = torch.zeros((N, M), dtype=torch.float64, device="cuda")
     Wd, xd = W.to(dtype).double(), x.double()
     for n in range(N):

@@ -532,8 +532,7 @@ int group_stages(const std::vector<LayerIn>& L, int G, bool two_d, double q_col,
   // np.percentile of n values, n known on the host, into thr[slot] and thr_host[slot]
   auto percentile = [&](const float* vals, long long n, double q, int slot) {
     if (n <= kGroupSelect) {
-      ts::MaskGroup none;
-      memset(&none, 0, sizeof(none));
+      static const ts::MaskGroup none = {};
       TSM_CUDA(ts::group_percentile_launch(vals, n, n, none, q, wide ? 1 : 0, thr + slot, thr_host + slot, s));
       return TS_OK;
     }
